@@ -27,6 +27,7 @@
 #include "backend_impl.hpp"
 #include "fullmag_fdm.h"
 #include "fullmag_fdm_ext.h"
+#include "linefft.cuh"
 #include "newell_host.hpp"
 
 struct fullmag_fdm_backend {
@@ -355,13 +356,30 @@ bool create_impl(Backend &b, const fullmag_fdm_plan_desc *plan, const fullmag_fd
         fm::make_line_plan(b.Lx, b.px);
         fm::make_line_plan(b.Ly, b.py);
         fm::make_line_plan(b.Lz, b.pz);
+        // in-plane lengths of the line FFTs (line_length(2n)); the shared-memory FFT and
+        // the projection fallback, which has Nyquist entries of its own, keep 2n
+        const int PX = fm::line_length(b.Lx), PY = fm::line_length(b.Ly);
+        const bool repad = PX != b.Lx || PY != b.Ly;
+        if (repad && b.projection) b.force_stockham = true;
+        auto take_padded = [&] {
+            b.Lx = PX; b.Ly = PY;
+            b.nkx = PX / 2 + 1; b.KY = PY / 2 + 1;
+        };
         if (demag_src == FULLMAG_FDM_EXT_DEMAG_NEWELL) {
-            fm::newell_octant_spectra(b.nx, b.ny, b.nz, b.dx, b.dy, b.dz, b.thin, spec);
+            if (!b.force_stockham) take_padded();
+            fm::newell_octant_spectra_padded(b.nx, b.ny, b.nz, b.dx, b.dy, b.dz, b.thin, b.Lx, b.Ly, 2 * b.nz, spec);
         } else if (b.projection) {
             projection_octant(b, spec);
         } else {
             // a 3-D spectrum of an nz = 1 grid is constant along kz: its kz = 0 plane is the 2-D one
             if (!extract_octant(b, plan, b.thin && Lzs == 2 ? 2 : Lzs, spec)) return false;
+            if (repad && !b.force_stockham) {
+                double scale = 0.0;
+                for (int c = 0; c < 3; ++c)
+                    for (double v : spec[c]) scale = std::max(scale, std::fabs(v));
+                if (fm::octant_repad(b.KZ, b.nx, b.ny, PX, PY, b.thin, 1e-8 * scale, spec)) take_padded();
+                else b.force_stockham = true;
+            }
         }
     }
 

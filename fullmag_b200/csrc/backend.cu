@@ -23,6 +23,7 @@
 #include "backend_impl.hpp"
 #include "demag.cuh"
 #include "demag_reg.cuh"
+#include "linefft.cuh"
 #include "demag_yz.hpp"
 #include "demag_row.hpp"
 #include "stage_vec.hpp"
@@ -45,28 +46,6 @@ bool upload_tw64(Backend &b) {
     }
     return cuda_ok(b, cudaMemcpyToSymbol(c_tw64d, d, sizeof(d)), "twiddle64 d") &&
            cuda_ok(b, cudaMemcpyToSymbol(c_tw64f, f, sizeof(f)), "twiddle64 f");
-}
-
-template <int V> using IC = std::integral_constant<int, V>;
-
-// (L1, L2) split of a power-of-two line length, as fftreg.cuh's l2_for.
-template <class F>
-static bool with_split(int L, F &&f) {
-    switch (L) {
-        case 2: f(IC<2>{}, IC<1>{}); return true;
-        case 4: f(IC<4>{}, IC<1>{}); return true;
-        case 8: f(IC<8>{}, IC<1>{}); return true;
-        case 16: f(IC<16>{}, IC<1>{}); return true;
-        case 32: f(IC<32>{}, IC<1>{}); return true;
-        case 64: f(IC<8>{}, IC<8>{}); return true;
-        case 128: f(IC<16>{}, IC<8>{}); return true;
-        case 256: f(IC<16>{}, IC<16>{}); return true;
-        case 512: f(IC<32>{}, IC<16>{}); return true;
-        case 1024: f(IC<32>{}, IC<32>{}); return true;
-        case 2048: f(IC<64>{}, IC<32>{}); return true;
-        case 4096: f(IC<64>{}, IC<64>{}); return true;
-        default: return false;
-    }
 }
 
 static bool is_pow2(int L) { return L >= 2 && (L & (L - 1)) == 0; }
@@ -160,6 +139,7 @@ struct Impl {
         a.px = b.px; a.py = b.py; a.pz = b.pz;
         a.twx = (const C *)b.twx; a.twy = (const C *)b.twy; a.twz = (const C *)b.twz;
         a.twxT = (const C *)b.twxT; a.twyT = (const C *)b.twyT;
+        a.twx4 = (const C *)b.twx4; a.twy4 = (const C *)b.twy4;
         a.s1 = (C *)b.s1; a.s2 = (C *)b.s2;
         a.spec = (const T *)b.spec;
         a.m = (const T *)m;
@@ -190,95 +170,22 @@ struct Impl {
         }
     }
 
-    // Register-FFT path: power-of-two x/y lengths <= 1024 (FP64) or 4096 (FP32).
+    // Line-FFT path (demag_line.cuh): padded in-plane lengths are line_length(2n).
     // z: direct summation for nz <= 8 (any nz; FULLMAG_FDM_ZCONV=fft keeps the
-    // z FFT) and in FP32 for nz <= 16 (k_zdw), else the register z FFT, Lz a
-    // power of two <= 16 (FP64) or 32 (FP32) since a thread holds 3 z lines.
-    static bool configure_reg(Backend &b) {
+    // z FFT) and in FP32 for nz <= 16 (k_zdw), else the register z FFT, Lz a power
+    // of two <= 16 (FP64) or 32 (FP32) since a thread holds 3 z lines, else the
+    // shared-memory z FFT of demag.cuh (any 2,3,5,7-smooth Lz).
+    static bool configure_line(Backend &b) {
         const bool dbl = sizeof(T) == 8;
-        const int maxxy = dbl ? 1024 : 4096, maxz = dbl ? 16 : 32;
-        if (!is_pow2(b.Lx) || !is_pow2(b.Ly) || b.Lx > maxxy || b.Ly > maxxy) return false;
         const bool zdw = zdw_wanted(b, !dbl);
         b.use_zdw = false;
         b.zdirect = zdw || (!b.thin && b.nz <= 8 && !b.want_yz && !env_is("FULLMAG_FDM_ZCONV", "fft"));
-        if (!b.thin && !b.zdirect && (!is_pow2(b.Lz) || b.Lz > maxz)) return false;
-        const size_t sz = sizeof(C), maxs = 200 * 1024;
-        const int target = 128;  // x passes: small blocks, several per SM
+        b.zreg = !b.thin && !b.zdirect && is_pow2(b.Lz) && b.Lz <= (dbl ? 16 : 32);
+        if (!cuda_ok(b, line_setup<T>(b.line, b.Lx, b.Ly, b.thin, b.ny, b.nz, b.nkx), "line FFT setup")) return false;
+        b.use_yz = false;
+        if (!b.thin && b.want_yz && b.zreg && is_pow2(b.Lx) && is_pow2(b.Ly) && !yz_configure<T>(b)) return false;
         bool ok = true;
-        // x passes: lines_x complex lines (row pairs) of L2 threads
-        with_split(b.Lx, [&](auto l1, auto l2) {
-            constexpr int L1 = decltype(l1)::value, L2 = decltype(l2)::value;
-            if constexpr (sizeof(T) == 8 && L1 > 32) { ok = false; } else {
-                constexpr int TE = line_region<L1, L2>();
-                const int unit = L2 >= 32 ? 1 : 32 / L2;    // lines per warp multiple
-                int lp = std::max(1, target / L2);
-                lp = std::min(lp, std::max(unit, ((b.ny + 1) / 2 + unit - 1) / unit * unit));
-                while (lp > unit && (size_t)(lp * TE) * sz > maxs) lp -= unit;
-                b.lines_x = lp;
-                b.thr_x = lp * L2;
-                b.rsm_x = (size_t)(lp * TE) * sz;
-                ok &= cuda_ok(b, cudaFuncSetAttribute(k_xf_r<T, L1, L2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.rsm_x), "attr xf_r");
-                // even ny: the pair gather (both rows of a line pair per load)
-                b.xi_pair = b.ny % 2 == 0;
-                b.rsm_xi = (size_t)lp * (b.xi_pair ? xi_stride<T, L1, L2, true>() : xi_stride<T, L1, L2, false>()) * sz +
-                           (size_t)L1 * L2 * sz;  // line regions + the twiddle table
-                ok &= cuda_ok(b, cudaFuncSetAttribute(b.xi_pair ? k_xi_r<T, L1, L2, xi_gather_pair<T>(), true>
-                                                                : k_xi_r<T, L1, L2, xi_gather<T>(), false>,
-                                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.rsm_xi), "attr xi_r");
-                // pipelined x forward for a uniform material with 16-byte rows
-                b.use_xpipe = false;
-                if (ok && !b.has_mask && !b.has_ms_map && !b.boundary_tier && (b.nx * sizeof(T)) % 16 == 0) {
-                    const int RB = 2 * lp;
-                    const size_t smem = xpipe_region_bytes<L1, L2, T>(lp) + (size_t)2 * RB * b.nx * sizeof(T) +
-                                        (size_t)L1 * L2 * sizeof(C);
-                    int occ = 0, sms = 148;
-                    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b.device);
-                    if (smem <= 200 * 1024 &&
-                        cudaFuncSetAttribute(k_xf_pipe<T, L1, L2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
-                        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_xf_pipe<T, L1, L2>, b.thr_x, smem) == cudaSuccess &&
-                        occ > 0 && !env_is("FULLMAG_FDM_XPIPE", "off")) {
-                        b.groups_x = 3 * b.nz * ((b.ny + RB - 1) / RB);
-                        b.grid_xpipe = std::min(b.groups_x, occ * sms);
-                        b.rsm_xpipe = smem;
-                        b.use_xpipe = true;
-                    }
-                    cudaGetLastError();
-                }
-            }
-        });
-        if (!ok) return false;
-        with_split(b.Ly, [&](auto l1, auto l2) {
-            constexpr int L1 = decltype(l1)::value, L2 = decltype(l2)::value;
-            if constexpr (sizeof(T) == 8 && L1 > 32) { ok = false; } else {
-                if (b.thin) {
-                    constexpr int TE = line_region<L1, L2>();
-                    const int unit = L2 >= 32 ? 1 : 32 / L2;  // kb multiple so 3*kb*L2 % 32 == 0
-                    int kb = std::max(unit, (256 / (3 * L2)) / unit * unit);
-                    kb = std::min(kb, std::max(unit, (b.nkx + unit - 1) / unit * unit));
-                    while (kb > unit && (size_t)(3 * kb * TE) * sz > maxs) kb -= unit;
-                    b.kb_y = kb;
-                    b.thr_yc = 3 * kb * L2;
-                    b.rsm_yc = (size_t)(3 * kb * TE) * sz;
-                    ok &= b.rsm_yc <= 227 * 1024 && b.thr_yc <= 256;
-                    ok &= cuda_ok(b, cudaFuncSetAttribute(k_yc_r<T, L1, L2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.rsm_yc), "attr yc_r");
-                } else {
-                    constexpr int TE = tile_elems(L1, L2);
-                    // lines per block: for 32-thread lines 6 (FP32) or 4 (FP64) lines,
-                    // measured at Ly = 1024 against 8 (FP32 -2 us per pass; FP64 8 lines
-                    // leave one 135 KB block per SM: 86.5 -> 74.5 us forward); at most
-                    // 68 KB of tiles per block otherwise
-                    int lpb = L2 == 32 ? (sizeof(T) == 8 ? 4 : 6) : std::max(1, 256 / L2);
-                    while (lpb > 1 && (size_t)(lpb * TE) * sz > 68 * 1024) lpb /= 2;
-                    b.lines_y = lpb;
-                    b.thr_y = lpb * L2;
-                    b.rsm_y = (size_t)(lpb * TE) * sz;
-                    ok &= cuda_ok(b, cudaFuncSetAttribute(k_yf_r<T, L1, L2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.rsm_y), "attr yf_r");
-                    ok &= cuda_ok(b, cudaFuncSetAttribute(k_yi_r<T, L1, L2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.rsm_y), "attr yi_r");
-                }
-            }
-        });
-        if (ok && !b.thin && b.want_yz && !yz_configure<T>(b)) return false;
-        if (ok && b.zdirect) {
+        if (b.zdirect) {
             with_nz(b.nz, [&](auto nzc) {
                 constexpr int NZ = decltype(nzc)::value;
                 const size_t smem = (size_t)zd_threads<T>() * zd_smem_per_thread<T, NZ>();
@@ -290,11 +197,13 @@ struct Impl {
                 b.grid_zd = (int)std::max<long long>(1, std::min<long long>((cols + zd_threads<T>() - 1) / zd_threads<T>(), (long long)std::max(occ, 1) * sms));
                 b.rsm_zd = smem;
             });
+        } else if (!b.thin && !b.zreg) {
+            ok &= configure_z_smem(b);
         }
         b.use_yzy = false;
         if (ok && zdw) {
             ok &= zdw_configure(b);
-            if (ok && !b.use_zdw) return false;  // no resident block: the generic path
+            if (ok && !b.use_zdw) { b.last_error = "direct z convolution: no resident block"; return false; }
         }
         if (ok && b.zdirect && !b.use_zdw) ok &= yzy_configure<T>(b);
         return ok;
@@ -305,35 +214,20 @@ struct Impl {
         x_fwd_reg(b, a);
         if (!mid_reg(b, a)) return false;
         x_inv_reg(b, a);
-        return check_launch(b, "demag (register FFT)");
+        return check_launch(b, "demag (line FFT)");
     }
 
     // x forward: Ms m -> S1
     static void x_fwd_reg(Backend &b, const DemagArgs<T> &a) {
-        const int RB = 2 * b.lines_x;
-        dim3 gx((b.ny + RB - 1) / RB, b.nz, 3);
-        with_split(b.Lx, [&](auto l1, auto l2) {
-            constexpr int L1 = decltype(l1)::value, L2 = decltype(l2)::value;
-            if constexpr (!(sizeof(T) == 8 && L1 > 32)) {
-                ProfScope p(b, "demag_x_fwd");
-                if (b.use_xpipe)
-                    k_xf_pipe<T, L1, L2><<<b.grid_xpipe, b.thr_x, b.rsm_xpipe, b.stream>>>(a, b.groups_x);
-                else
-                    k_xf_r<T, L1, L2><<<gx, b.thr_x, b.rsm_x, b.stream>>>(a);
-            }
-        });
+        ProfScope p(b, "demag_x_fwd");
+        line_x_fwd<T>(b.line, a, b.stream);
     }
 
     // the y (thin film) or y / z passes: S1 -> S1
     static bool mid_reg(Backend &b, const DemagArgs<T> &a) {
         if (b.thin) {
-            with_split(b.Ly, [&](auto l1, auto l2) {
-                constexpr int L1 = decltype(l1)::value, L2 = decltype(l2)::value;
-                if constexpr (!(sizeof(T) == 8 && L1 > 32)) {
-                    ProfScope p(b, "demag_y_conv");
-                    k_yc_r<T, L1, L2><<<(b.nkx + b.kb_y - 1) / b.kb_y, b.thr_yc, b.rsm_yc, b.stream>>>(a);
-                }
-            });
+            ProfScope p(b, "demag_y_conv");
+            line_y_conv<T>(b.line, a, b.stream);
         } else if (b.use_yz) {
             ProfScope p(b, "demag_yz");
             if (!yz_launch(b, a)) return false;
@@ -341,15 +235,10 @@ struct Impl {
             ProfScope p(b, "demag_yzy");
             if (!yzy_launch(b, a)) return false;
         } else {
-            const long long lines = 3LL * b.nz * b.nkx;
-            const unsigned gy = (unsigned)((lines + b.lines_y - 1) / b.lines_y);
-            with_split(b.Ly, [&](auto l1, auto l2) {
-                constexpr int L1 = decltype(l1)::value, L2 = decltype(l2)::value;
-                if constexpr (!(sizeof(T) == 8 && L1 > 32)) {
-                    ProfScope p(b, "demag_y_fwd");
-                    k_yf_r<T, L1, L2><<<gy, b.thr_y, b.rsm_y, b.stream>>>(a);
-                }
-            });
+            {
+                ProfScope p(b, "demag_y_fwd");
+                line_y_fwd<T>(b.line, a, b.stream);
+            }
             if (b.use_zdw) {
                 ProfScope p(b, "demag_z_direct");
                 if constexpr (sizeof(T) == 4) zdw_launch(b, a);
@@ -359,7 +248,7 @@ struct Impl {
                     constexpr int NZ = decltype(nzc)::value;
                     k_zd<T, NZ><<<b.grid_zd, zd_threads<T>(), b.rsm_zd, b.stream>>>(a);
                 });
-            } else {
+            } else if (b.zreg) {
                 ProfScope p(b, "demag_z_conv");
                 const long long cols = (long long)b.nkx * b.Ly;
                 // one thread per column up to 3 x 8 z points, a thread pair (split by
@@ -374,32 +263,37 @@ struct Impl {
                     case 322: if constexpr (sizeof(T) == 4) k_zc_r<T, 32, 2><<<gz2, 128, 0, b.stream>>>(a); break;
                     default: break;
                 }
+            } else {
+                ProfScope p(b, "demag_z_conv");
+                launch_z_smem(b, a);
             }
-            with_split(b.Ly, [&](auto l1, auto l2) {
-                constexpr int L1 = decltype(l1)::value, L2 = decltype(l2)::value;
-                if constexpr (!(sizeof(T) == 8 && L1 > 32)) {
-                    ProfScope p(b, "demag_y_inv");
-                    k_yi_r<T, L1, L2><<<gy, b.thr_y, b.rsm_y, b.stream>>>(a);
-                }
-            });
+            ProfScope p(b, "demag_y_inv");
+            line_y_inv<T>(b.line, a, b.stream);
         }
         return true;
     }
 
     // x inverse: S1 -> H_d
     static void x_inv_reg(Backend &b, const DemagArgs<T> &a) {
-        const int RB = 2 * b.lines_x;
-        dim3 gx((b.ny + RB - 1) / RB, b.nz, 3);
-        with_split(b.Lx, [&](auto l1, auto l2) {
-            constexpr int L1 = decltype(l1)::value, L2 = decltype(l2)::value;
-            if constexpr (!(sizeof(T) == 8 && L1 > 32)) {
-                ProfScope p(b, "demag_x_inv");
-                if (b.xi_pair)
-                    k_xi_r<T, L1, L2, xi_gather_pair<T>(), true><<<gx, b.thr_x, b.rsm_xi, b.stream>>>(a);
-                else
-                    k_xi_r<T, L1, L2, xi_gather<T>(), false><<<gx, b.thr_x, b.rsm_xi, b.stream>>>(a);
-            }
-        });
+        ProfScope p(b, "demag_x_inv");
+        line_x_inv<T>(b.line, a, b.stream);
+    }
+
+    // the shared-memory z FFT: ky tile and shared memory
+    static bool configure_z_smem(Backend &b) {
+        const int budget = 100 * 1024, sz = (int)sizeof(C), ld = b.Lz + 1;
+        b.kt_z = std::min(std::max(1, std::min(32, (budget - b.Lz * sz) / (2 * ld * sz * 3))), b.Ly);
+        b.smem_z = (size_t)sz * (b.Lz + 2 * 3 * (size_t)b.kt_z * (b.Lz + 1));
+        if (b.smem_z > 227 * 1024) {
+            b.last_error = "padded FFT length too large for the shared-memory FFT (max 4096 per axis)";
+            return false;
+        }
+        return cuda_ok(b, cudaFuncSetAttribute(k_z_conv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.smem_z), "attr z_conv");
+    }
+
+    static void launch_z_smem(Backend &b, const DemagArgs<T> &a) {
+        const dim3 gz((b.Ly + b.kt_z - 1) / b.kt_z, b.nkx);
+        k_z_conv<T><<<gz, 256, b.smem_z, b.stream>>>(a);
     }
 
     // the ring-fed stage kernels' shared memory (above 48 KB for FP64)
@@ -432,15 +326,14 @@ struct Impl {
 
     static bool configure(Backend &b) {
         if (!upload_tw64(b)) return false;
-        if (!b.force_stockham && configure_reg(b)) {
+        if (!b.force_stockham) {
             b.use_reg = true;
-            return row_configure<T>(b);
+            return configure_line(b) && row_configure<T>(b);
         }
         b.use_reg = false;
         b.zdirect = false;
         b.use_yzy = false;
         b.use_zdw = false;
-        if (!b.last_error.empty()) return false;
         const int budget = 100 * 1024;
         const int sz = (int)sizeof(C);
         auto lines_for = [&](int ld, int L, int per_line_mult, int maxl) {
@@ -457,12 +350,10 @@ struct Impl {
         } else {
             b.lines_y = lines_for(b.Ly + 1, b.Ly, 1, 16);
             b.smem_yf = (size_t)sz * (b.Ly + 2 * (size_t)b.lines_y * (b.Ly + 1));
-            b.kt_z = lines_for(b.Lz + 1, b.Lz, 3, 32);
-            b.kt_z = std::min(b.kt_z, b.Ly);
-            b.smem_z = (size_t)sz * (b.Lz + 2 * 3 * (size_t)b.kt_z * (b.Lz + 1));
+            if (!configure_z_smem(b)) return false;
         }
         const size_t maxs = 227 * 1024;
-        if (b.smem_xf > maxs || b.smem_yf > maxs || b.smem_z > maxs || b.smem_yc > maxs) {
+        if (b.smem_xf > maxs || b.smem_yf > maxs || b.smem_yc > maxs) {
             b.last_error = "padded FFT length too large for the shared-memory FFT (max 4096 per axis)";
             return false;
         }
@@ -474,7 +365,6 @@ struct Impl {
         } else {
             ok &= cuda_ok(b, cudaFuncSetAttribute(k_y_fwd<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.smem_yf), "attr y_fwd");
             ok &= cuda_ok(b, cudaFuncSetAttribute(k_y_inv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.smem_yf), "attr y_inv");
-            ok &= cuda_ok(b, cudaFuncSetAttribute(k_z_conv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.smem_z), "attr z_conv");
         }
         return ok;
     }
@@ -518,8 +408,7 @@ struct Impl {
             }
             {
                 ProfScope p(b, "demag_z_conv");
-                dim3 gz((b.Ly + b.kt_z - 1) / b.kt_z, b.nkx);
-                k_z_conv<T><<<gz, 256, b.smem_z, b.stream>>>(a);
+                launch_z_smem(b, a);
             }
             {
                 ProfScope p(b, "demag_y_inv");
@@ -1270,10 +1159,14 @@ bool backend_alloc(Backend &b) {
         items.push_back({&b.twy, (size_t)b.Ly * cs});
         items.push_back({&b.twxT, (size_t)b.Lx * cs});
         items.push_back({&b.twyT, (size_t)b.Ly * cs});
+        items.push_back({&b.twx4, (size_t)(dbl ? line_twiddle_count<double>(b.Lx) : line_twiddle_count<float>(b.Lx)) * cs});
+        items.push_back({&b.twy4, (size_t)(dbl ? line_twiddle_count<double>(b.Ly) : line_twiddle_count<float>(b.Ly)) * cs});
         items.push_back({&b.twz, (size_t)b.Lz * cs});
         items.push_back({&b.s1, (size_t)3 * b.nz * b.nkx * b.ny * cs});
         if (!b.thin) items.push_back({&b.s2, (size_t)3 * b.nz * b.nkx * b.Ly * cs});
-        items.push_back({&b.spec, (size_t)6 * b.KZ * b.nkx * b.KY * b.scalar});
+        // the octant, or a direct z table: nz planes of KY values, or of the fused pass's row
+        items.push_back({&b.spec, 6 * b.nkx * b.scalar *
+                                      std::max((size_t)b.KZ * b.KY, b.thin ? 0 : (size_t)b.nz * (dbl ? yzy_table_values_f64(b.Ly) : yzy_table_values_f32(b.Ly)))});
     }
     items.push_back({&b.staging, (size_t)3 * b.n * sizeof(double)});
     if (b.has_mask) items.push_back({(void **)&b.d_mask, (size_t)b.n});
@@ -1342,11 +1235,16 @@ static bool upload_tables(Backend &b, const std::vector<double> (&spec)[6]) {
     };
     if (!tw(b.Lx, b.twx) || !tw(b.Ly, b.twy) || !tw(b.Lz, b.twz)) return false;
     auto tw4 = [&](int L, void *dst) {
-        if (L < 2 || (L & (L - 1))) return true;  // register FFT only (powers of two)
+        if (L < 2 || (L & (L - 1))) return true;  // the opt-in fused passes' 4-step FFT (powers of two)
         const std::vector<cx<T>> t = host_tw4<T>(L);
         return cuda_ok(b, cudaMemcpy(dst, t.data(), L * sizeof(cx<T>), cudaMemcpyHostToDevice), "twiddles (4-step)");
     };
     if (!tw4(b.Lx, b.twxT) || !tw4(b.Ly, b.twyT)) return false;
+    auto twl = [&](int L, void *dst) {
+        const std::vector<cx<T>> t = line_twiddles<T>(L);
+        return t.empty() || cuda_ok(b, cudaMemcpy(dst, t.data(), t.size() * sizeof(cx<T>), cudaMemcpyHostToDevice), "twiddles (line)");
+    };
+    if (!twl(b.Lx, b.twx4) || !twl(b.Ly, b.twy4)) return false;
     // the octant, or for the direct z convolution its z-inverse table (nz planes)
     std::vector<double> zt[6];
     if (b.zdirect) octant_to_z_direct(b.nkx, b.KY, b.nz, spec, zt);
@@ -1360,6 +1258,16 @@ static bool upload_tables(Backend &b, const std::vector<double> (&spec)[6]) {
         for (int c = 0; c < 6; ++c)
             for (size_t r = 0; r < rows; ++r)
                 for (int ky = 0; ky < b.KY; ++ky) host[(c * rows + r) * kyp + ky] = (T)src[c][r * b.KY + ky];
+    } else if (b.use_yzy) {
+        const size_t row = (size_t)(sizeof(T) == 4 ? yzy_table_values_f32(b.Ly) : yzy_table_values_f64(b.Ly)), rows = (size_t)b.nz * b.nkx;
+        host.assign(6 * rows * row, T(0));
+        for (int c = 0; c < 6; ++c)
+            for (size_t r = 0; r < rows; ++r) {
+                const double *from = &src[c][r * b.KY], sign = (c == 3 || c == 5) ? -1.0 : 1.0;  // xy, yz odd in y
+                T *to = &host[(c * rows + r) * row];
+                if constexpr (sizeof(T) == 4) yzy_table_row_f32(b.Ly, from, sign, to);
+                else yzy_table_row_f64(b.Ly, from, sign, to);
+            }
     } else {
         host.resize(6 * plane);
         for (int c = 0; c < 6; ++c)

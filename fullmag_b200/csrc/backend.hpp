@@ -9,6 +9,7 @@
 
 #include "fullmag_fdm.h"
 #include "fullmag_fdm_ext.h"
+#include "demag_line.hpp"
 #include "fft.cuh"
 
 namespace fm {
@@ -86,16 +87,13 @@ struct Backend {
     LinePlan px{}, py{}, pz{};
     void *twx = nullptr, *twy = nullptr, *twz = nullptr;
     void *twxT = nullptr, *twyT = nullptr;  // 4-step twiddle tables (fftreg.cuh fill_tw4 order)
+    void *twx4 = nullptr, *twy4 = nullptr;  // line-FFT twiddle tables (linefft.cuh line_twiddles)
     void *s1 = nullptr, *s2 = nullptr, *spec = nullptr;
     int lines_x = 1, lines_y = 1, kt_z = 1, kb_y = 1;
     size_t smem_xf = 0, smem_yf = 0, smem_z = 0, smem_yc = 0;
-    // register-FFT path (power-of-two lengths): block sizes and shared memory
-    bool use_reg = false;
-    bool force_stockham = false;  // FULLMAG_FDM_FFT=stockham selects the shared-memory FFT
-    int thr_x = 0, thr_y = 0, thr_yc = 0;
-    bool use_xpipe = false;       // uniform material: cp.async-pipelined x forward
-    size_t rsm_xpipe = 0;
-    int grid_xpipe = 0, groups_x = 0;
+    bool use_reg = false;         // line-FFT passes (demag_line.cuh)
+    LineCfg line;                 // ... and their block shapes
+    bool force_stockham = false;  // FULLMAG_FDM_FFT=stockham selects the shared-memory FFT at the lengths 2n
     bool stage_plain = false;     // uniform material: z-marching stage kernel
     bool stage_ring = false;      // ... fed by the cp.async plane ring (FULLMAG_FDM_STAGE=plain: register prefetch)
     bool stage_vec = false;       // stage kernels on 16-byte cell groups (stage_vec.cuh; FULLMAG_FDM_STAGE=ring/plain/cell: off)
@@ -106,9 +104,7 @@ struct Backend {
     int yz_P = 0, thr_yz = 0;     // cluster size (ky residues per kx), threads
     int yz_min_P = 1;             // FULLMAG_FDM_YZ_P: smallest cluster size tried
     size_t rsm_yz = 0;
-    size_t rsm_x = 0, rsm_y = 0, rsm_yc = 0;
-    size_t rsm_xi = 0;            // x inverse: line regions + twiddle table
-    bool xi_pair = false;         // x inverse gathers row pairs (ny even)
+    bool zreg = false;            // z FFT in registers (k_zc_r), else in shared memory (k_z_conv)
     bool zdirect = false;         // 3-D, nz <= 8 (FP32: nz <= 16): z convolution by direct summation (k_zd, k_zdw)
     bool use_yzy = false;         // y forward + direct z + y inverse fused per kx plane (k_yzy)
     int yzy_P = 0;                // its cluster size (CTAs per plane)

@@ -35,6 +35,7 @@ struct DemagArgs {
     // register-FFT inter-level twiddles in the order fft4step reads them
     // (twT[k1 L2 + t] = W_L^{k1 t}, fill_tw4's layout), read from global memory
     const cx<T> *twxT, *twyT;
+    const cx<T> *twx4, *twy4;  // twiddles of the line FFTs (linefft.cuh line_twiddles)
     cx<T> *s1, *s2;
     const T *spec;          // octant, 6 components
     const T *m;             // SoA magnetisation, component stride n
@@ -46,6 +47,7 @@ struct DemagArgs {
     T *hd;                  // SoA demag field out
     double norm;            // 1 / (Lx Ly Lz)
     int lines_x;            // complex lines (= 2 rows) per x-pass block
+    int te_x;               // line stride of the x passes' shared memory (line FFTs)
     int lines_y;            // lines per y-pass block
     int kt_z;               // ky tile of the z pass
     int kb_y;               // kx per block of the 2-D y_conv pass

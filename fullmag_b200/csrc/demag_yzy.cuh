@@ -6,25 +6,32 @@
 // by the y inverse pass).  Here the 3 nz lines (c, z) of plane kx stay in the
 // shared memory of one thread-block cluster from the y forward FFT to the y
 // inverse FFT.  CTA h of the cluster owns lines [h NLH, (h + 1) NLH):
-//   1. one group of L2 threads per owned line: forward y (fft4step, the
-//      zero-padded half of the input pruned) from S1 into the line's row;
+//   1. one group of threads per owned line: forward y (line_fwd, the zero-padded
+//      half of the input pruned) from S1 into the line's row, left in slot order;
 //   2. cluster barrier; CTA h sums the direct z convolution of the ky columns
 //      [h Ly/P, (h + 1) Ly/P), reading each column's 3 nz values from the
 //      owners' rows (distributed shared memory for the other CTAs' lines) and
 //      writing the results back there (k_zd's loop, all three components at once;
 //      one component at a time measured 104.6 against 99.4 us at 512 x 512 x 8);
-//   3. cluster barrier; inverse y (fft4step) from the owned rows back into S1,
+//   3. cluster barrier; inverse y (line_inv) from the owned rows back into S1,
 //      keeping y < ny.
 // The sums are those of k_zd, in the same order per output, and the FFTs are
-// those of k_yf_r and k_yi_r, so the result is bitwise the split path's.
-// Shared memory per CTA: NLH rows of tile_elems(L1, L2) complex (a row is also
-// its line's 4-step tile), then the Ly twiddles.  P = 1 is one CTA per plane.
-// No TMA; the remote rows are read and written with plain loads and stores.
+// those of k_ly_fwd and k_ly_inv, so the result is bitwise the split path's.
+// Shared memory per CTA: NLH rows of a line's tile, then the twiddles.  P = 1 is one
+// CTA per plane.  No TMA; the remote rows are read and written with plain loads and
+// stores.
 //
-// Measured at 512 x 512 x 8 (FP32, P = 1): 112 us with scalar complex adds,
-// 117 us with the packed FP32 pair, so the units that include this header
-// define FM_SCALAR_COMPLEX_ADD first.  One unit per precision
-// (demag_yzy_f32.cu, demag_yzy_f64.cu), so that they compile in parallel.
+// The spectrum stays in the slots the transforms leave it in (linefft.cuh), and the z
+// table is uploaded in the same order (yzy_table), so the lanes of the z sum read
+// neighbouring slots of every row and neighbouring table values.
+//
+// Measured at 512 x 512 x 8 (FP32, P = 2, one half plane's CTA): 12.4 kcycles
+// forward, 16.8 the z sum, 8 inverse; the z sum is bound by its 576 packed
+// multiply-adds per column (2.05 cycles each per scheduler, the FP32 peak).
+// 106 us with 3-pass lines of 64 threads and named barriers, 100 us with the
+// two-pass lines of one warp each; P = 1 (384 threads) 114 us.
+// One unit per precision (demag_yzy_f32.cu, demag_yzy_f64.cu), so that they
+// compile in parallel.
 #pragma once
 #include <cooperative_groups.h>
 
@@ -36,43 +43,58 @@
 #include "backend_impl.hpp"
 #include "demag.cuh"
 #include "demag_reg.cuh"
+#include "linefft.cuh"
 #include "demag_yzy.hpp"
 
 namespace cg = cooperative_groups;
 
 namespace fm {
 
+// table values per (component, offset, kx): tile rows k0 <= R0 / 2
+template <typename T, int L> __host__ __device__ constexpr int yzy_row() { return (Lf<T, L>::R0 / 2 + 1) * (L / Lf<T, L>::R0); }
 // lines owned by one CTA of a P-CTA cluster
 template <int NZ, int P> __host__ __device__ constexpr int yzy_nlh() { return (3 * NZ + P - 1) / P; }
-// lines per FFT pass: FP32 CTAs of at most 192 threads (168 registers each, so
-// that two CTAs of 107 KB fit per SM), FP64 at most 384
+// lines per FFT pass: at most 384 threads in FP32 for a whole plane, 192 for a cluster's
+// share of one (168 registers each, the z sum's need, so that two CTAs of 107 KB fit per
+// SM), 384 in FP64
 template <typename T, int L2, int NZ, int P> __host__ __device__ constexpr int yzy_lpp() {
-    return yzy_nlh<NZ, P>() * L2 <= (sizeof(T) == 4 ? 192 : 384) ? yzy_nlh<NZ, P>() : (sizeof(T) == 4 ? 192 : 384) / L2;
+    constexpr int most = sizeof(T) == 4 && P > 1 ? 192 : 384;
+    constexpr int cap = L2 > 32 ? (most / L2 < 15 ? most / L2 : 15) : most / L2;  // named barriers
+    constexpr int l = yzy_nlh<NZ, P>() < cap ? yzy_nlh<NZ, P>() : cap;
+    constexpr int unit = L2 < 32 ? 32 / L2 : 1;  // whole warps
+    return (l + unit - 1) / unit * unit;
 }
 // rows: the owned lines rounded up to whole passes (the idle line groups of a
 // last, partial pass use their own rows as 4-step scratch)
 template <typename T, int L2, int NZ, int P> __host__ __device__ constexpr int yzy_rows() {
     return (yzy_nlh<NZ, P>() + yzy_lpp<T, L2, NZ, P>() - 1) / yzy_lpp<T, L2, NZ, P>() * yzy_lpp<T, L2, NZ, P>();
 }
-template <typename T, int L1, int L2, int NZ, int P>
+template <typename T, int L, int NZ, int P>
 __host__ __device__ constexpr size_t yzy_smem() {
-    return ((size_t)yzy_rows<T, L2, NZ, P>() * tile_elems(L1, L2) + (size_t)L1 * L2) * sizeof(cx<T>);
+    return ((size_t)yzy_rows<T, Lf<T, L>::G, NZ, P>() * Lf<T, L>::TILE + (size_t)Lf<T, L>::TW) * sizeof(cx<T>);
 }
 constexpr size_t kYzySmemMax = 227 * 1024;
-template <typename T, int L1, int L2, int NZ, int P>
+template <typename T, int L, int NZ, int P>
 __host__ __device__ constexpr bool yzy_fits() {
-    return yzy_smem<T, L1, L2, NZ, P>() <= kYzySmemMax &&
-           (sizeof(T) == 4 || L1 <= 32);  // FP64 4-step lines: 32 values per thread at most
+    return yzy_smem<T, L, NZ, P>() <= kYzySmemMax;
 }
-template <typename T, int L2, int NZ, int P> __host__ __device__ constexpr int yzy_threads() {
-    return yzy_lpp<T, L2, NZ, P>() * L2;
+template <typename T, int L, int NZ, int P> __host__ __device__ constexpr int yzy_threads() {
+    return yzy_lpp<T, Lf<T, L>::G, NZ, P>() * Lf<T, L>::G;
 }
 
-template <typename T, int L1, int L2, int NZ, int P>
-__global__ void __launch_bounds__(yzy_threads<T, L2, NZ, P>()) k_yzy(DemagArgs<T> a) {
+// CTAs per SM: as many as fit the shared memory, registers cut to match
+template <typename T, int L, int NZ, int P> __host__ __device__ constexpr int yzy_min_blocks() {
+    constexpr int by_smem = (int)(kYzySmemMax / (yzy_smem<T, L, NZ, P>() + 1024));
+    constexpr int by_thr = 65536 / (yzy_threads<T, L, NZ, P>() * 168);
+    constexpr int m = by_smem < by_thr ? by_smem : by_thr;
+    return m < 1 ? 1 : m;
+}
+
+template <typename T, int L, int NZ, int P>
+__global__ void __launch_bounds__((yzy_threads<T, L, NZ, P>()), (yzy_min_blocks<T, L, NZ, P>())) k_yzy(DemagArgs<T> a) {
     using C = cx<T>;
-    constexpr int L = L1 * L2, TE = tile_elems(L1, L2), NL = 3 * NZ, NLH = yzy_nlh<NZ, P>();
-    constexpr int LPP = yzy_lpp<T, L2, NZ, P>(), ROWS = yzy_rows<T, L2, NZ, P>(), BT = LPP * L2;
+    constexpr int G = Lf<T, L>::G, TE = Lf<T, L>::TILE, NL = 3 * NZ, NLH = yzy_nlh<NZ, P>();
+    constexpr int LPP = yzy_lpp<T, G, NZ, P>(), ROWS = yzy_rows<T, G, NZ, P>(), BT = LPP * G;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C *S = reinterpret_cast<C *>(smem_raw);
     C *tws = S + ROWS * TE;
@@ -81,18 +103,17 @@ __global__ void __launch_bounds__(yzy_threads<T, L2, NZ, P>()) k_yzy(DemagArgs<T
         if constexpr (P > 1) cg::this_cluster().sync();
         else __syncthreads();
     };
-    for (int k = threadIdx.x; k < L; k += BT) tws[k] = a.twyT[k];
-    __syncthreads();  // fft4step reads twiddles before its first barrier
+    for (int k = threadIdx.x; k < Lf<T, L>::TW; k += BT) tws[k] = a.twy4[k];
+    __syncthreads();  // the transforms have no block barrier
     const int kx = blockIdx.x / P, nkx = a.nkx, ny = a.ny;
-    const int qg = threadIdx.x / L2, t = threadIdx.x - qg * L2;
-    {   // only the z sum reads the plane's table (6 NZ rows of KY values): bring it
-        // into L2 while the y forward FFTs run, the rows split over the cluster's CTAs
-        constexpr int LN = 128 / (int)sizeof(T);  // values per 128-byte line
-        const int KY = a.KY, nln = (KY + LN - 1) / LN;
-        const T *t0 = a.spec + (long long)kx * KY;
-        for (int i = h * BT + threadIdx.x; i < 6 * NZ * nln; i += P * BT) {
-            const int r = i / nln, j = i - r * nln;
-            const T *p = t0 + (long long)r * nkx * KY + min(j * LN, KY - 1);
+    const int qg = threadIdx.x / G, t = threadIdx.x % G;
+    {   // only the z sum reads the plane's table (6 NZ rows of yzy_row<T, L>() values): bring
+        // it into L2 while the y forward FFTs run, the rows split over the cluster's CTAs
+        constexpr int LN = 128 / (int)sizeof(T), ROW = yzy_row<T, L>(), NLN = (ROW + LN - 1) / LN;
+        const T *t0 = a.spec + (long long)kx * ROW;
+        for (int i = h * BT + threadIdx.x; i < 6 * NZ * NLN; i += P * BT) {
+            const int r = i / NLN, j = i - r * NLN;
+            const T *p = t0 + (long long)r * nkx * ROW + min(j * LN, ROW - 1);
             asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
         }
     }
@@ -104,9 +125,9 @@ __global__ void __launch_bounds__(yzy_threads<T, L2, NZ, P>()) k_yzy(DemagArgs<T
         const bool valid = lr < NLH && q < NL;     // spare rows are scratch
         const C *line1 = a.s1 + ((long long)(valid ? q : 0) * nkx + kx) * ny;  // S1 [c][z][kx][y]
         C *row = S + lr * TE;
-        auto in1 = [&](int j) -> C { return valid ? line1[j] : mk<T>(0, 0); };
-        auto out1 = [&](int k, C v) { row[k] = v; };
-        fft4step<L1, L2, false, false, true, true>(t, tws, row, in1, out1);
+        auto in1 = [&](int j) -> C { return j < ny ? line1[j] : mk<T>(0, 0); };
+        auto out1 = [&](int k, C v) { row[line_slot<T, L>(k)] = v; };
+        line_fwd<L, true>(t, qg, tws, row, in1, out1);
     }
     cluster_sync();
     // 2. direct z convolution of this CTA's ky columns (table and signs as in k_zd)
@@ -117,20 +138,35 @@ __global__ void __launch_bounds__(yzy_threads<T, L2, NZ, P>()) k_yzy(DemagArgs<T
             if constexpr (P > 1) own[r] = cg::this_cluster().map_shared_rank(S, r);
             else own[r] = S;
         }
-        auto cell = [&](int line, int ky) -> C & { return own[line / NLH][(line % NLH) * TE + ky]; };
-        const int KY = a.KY, dstr = nkx * KY, tstr = NZ * dstr;
+        auto cell = [&](int line, int s) -> C & { return own[line / NLH][(line % NLH) * TE + s]; };
+        // column i of the plane in slot order: tile row k0 = i / M0, place i % M0.  The
+        // table (yzy_table) holds the rows k0 <= R0 / 2 in the same order; a row above is
+        // the mirror ky -> L - ky of row R0 - k0, read backwards, with the components odd
+        // in y negated.  So neighbouring lanes read neighbouring table values and
+        // neighbouring slots of every line.
+        constexpr int R0 = Lf<T, L>::R0, M0 = L / R0, LD = Lf<T, L>::LD, ROW = yzy_row<T, L>();
+        const int dstr = nkx * ROW, tstr = NZ * dstr;
         constexpr int KC = L / P;  // columns per CTA
         for (int kk = threadIdx.x; kk < KC; kk += BT) {
-            const int ky = h * KC + kk;
-            const bool ymir = ky > L / 2;
-            const T sy = ymir ? T(-1) : T(1);
-            const T *tp = a.spec + (kx * KY + (ymir ? L - ky : ky));
+            const int i = h * KC + kk, k0 = i / M0, idx = i % M0, sl = Lf<T, L>::NP == 1 ? i : k0 * LD + idx;
+            const bool mir = 2 * k0 > R0;
+            const T sy = mir ? T(-1) : T(1);
+            const T *tp = a.spec + ((long long)kx * ROW + (mir ? (R0 - k0) * M0 + (M0 - 1 - idx) : i));
+            // the table entries of offset d, loaded two offsets ahead of their use
+            T nx_[2][6];
+            auto fetch = [&](int d, T (&c)[6]) {
+                const T *qd = tp + d * dstr;
+#pragma unroll
+                for (int e = 0; e < 6; ++e) c[e] = (e < 4 || d > 0) ? __ldg(qd + e * tstr) : T(0);
+            };
+            fetch(0, nx_[0]);
+            if (NZ > 1) fetch(1, nx_[1]);
             C mx[NZ], my[NZ], mz[NZ];
 #pragma unroll
             for (int z = 0; z < NZ; ++z) {
-                mx[z] = cell(z, ky);
-                my[z] = cell(NZ + z, ky);
-                const C v = cell(2 * NZ + z, ky);
+                mx[z] = cell(z, sl);
+                my[z] = cell(NZ + z, sl);
+                const C v = cell(2 * NZ + z, sl);
                 mz[z] = mk<T>(v.y, -v.x);  // -i Mz
             }
             C hx[NZ], hy[NZ], hz[NZ];
@@ -139,9 +175,9 @@ __global__ void __launch_bounds__(yzy_threads<T, L2, NZ, P>()) k_yzy(DemagArgs<T
             // the loop of k_zd: per output, offsets d ascending, +d then -d
 #pragma unroll
             for (int d = 0; d < NZ; ++d) {
-                const T *qd = tp + d * dstr;
-                const T cxx = qd[0], cyy = qd[tstr], czz = qd[2 * tstr], cxy = qd[3 * tstr] * sy;
-                const T cxz = d > 0 ? qd[4 * tstr] : T(0), cyz = d > 0 ? qd[5 * tstr] * sy : T(0);
+                const T cxx = nx_[d & 1][0], cyy = nx_[d & 1][1], czz = nx_[d & 1][2], cxy = nx_[d & 1][3] * sy;
+                const T cxz = nx_[d & 1][4], cyz = nx_[d & 1][5] * sy;
+                if (d + 2 < NZ) fetch(d + 2, nx_[d & 1]);
 #pragma unroll
                 for (int z = 0; z + d < NZ; ++z) {
                     {   // output z + d from input z (offset +d)
@@ -151,18 +187,18 @@ __global__ void __launch_bounds__(yzy_threads<T, L2, NZ, P>()) k_yzy(DemagArgs<T
                         zd_fma(hz[o], -cxz, mx[z]); zd_fma(hz[o], -cyz, my[z]); zd_fma(hz[o], czz, mz[z]);
                     }
                     if (d > 0) {  // output z from input z + d (offset -d: odd-in-z entries flip)
-                        const int i = z + d;
-                        zd_fma(hx[z], cxx, mx[i]); zd_fma(hx[z], cxy, my[i]); zd_fma(hx[z], -cxz, mz[i]);
-                        zd_fma(hy[z], cxy, mx[i]); zd_fma(hy[z], cyy, my[i]); zd_fma(hy[z], -cyz, mz[i]);
-                        zd_fma(hz[z], cxz, mx[i]); zd_fma(hz[z], cyz, my[i]); zd_fma(hz[z], czz, mz[i]);
+                        const int j = z + d;
+                        zd_fma(hx[z], cxx, mx[j]); zd_fma(hx[z], cxy, my[j]); zd_fma(hx[z], -cxz, mz[j]);
+                        zd_fma(hy[z], cxy, mx[j]); zd_fma(hy[z], cyy, my[j]); zd_fma(hy[z], -cyz, mz[j]);
+                        zd_fma(hz[z], cxz, mx[j]); zd_fma(hz[z], cyz, my[j]); zd_fma(hz[z], czz, mz[j]);
                     }
                 }
             }
 #pragma unroll
             for (int z = 0; z < NZ; ++z) {
-                cell(z, ky) = hx[z];
-                cell(NZ + z, ky) = hy[z];
-                cell(2 * NZ + z, ky) = mk<T>(-hz[z].y, hz[z].x);  // Hz = i Hz'
+                cell(z, sl) = hx[z];
+                cell(NZ + z, sl) = hy[z];
+                cell(2 * NZ + z, sl) = mk<T>(-hz[z].y, hz[z].x);  // Hz = i Hz'
             }
         }
     }
@@ -174,34 +210,34 @@ __global__ void __launch_bounds__(yzy_threads<T, L2, NZ, P>()) k_yzy(DemagArgs<T
         const bool valid = lr < NLH && q < NL;
         C *line1 = a.s1 + ((long long)(valid ? q : 0) * nkx + kx) * ny;
         C *row = S + lr * TE;
-        auto in3 = [&](int j) -> C { return row[j]; };
-        auto out3 = [&](int k, C v) { if (valid && k < ny) line1[k] = v; };
-        fft4step<L1, L2, true, true, false>(t, tws, row, in3, out3);
+        auto in3 = [&](int k) -> C { return row[line_slot<T, L>(k)]; };
+        auto out3 = [&](int n, C v) { if (valid && n < ny) line1[n] = v; };
+        line_inv<L, true>(t, qg, tws, row, in3, out3);
     }
 }
 
 template <int N> using YzyIC = std::integral_constant<int, N>;
 
-// (L1, L2) of Ly in 256..1024 and NZ of nz as compile-time values
+// Ly in 256..1024 and NZ of nz as compile-time values
 template <class F>
 void yzy_dispatch(int Ly, int nz, F &&f) {
-    auto nzs = [&](auto l1, auto l2) {
+    auto nzs = [&](auto l) {
         switch (nz) {
-            case 1: f(l1, l2, YzyIC<1>{}); break;
-            case 2: f(l1, l2, YzyIC<2>{}); break;
-            case 3: f(l1, l2, YzyIC<3>{}); break;
-            case 4: f(l1, l2, YzyIC<4>{}); break;
-            case 5: f(l1, l2, YzyIC<5>{}); break;
-            case 6: f(l1, l2, YzyIC<6>{}); break;
-            case 7: f(l1, l2, YzyIC<7>{}); break;
-            case 8: f(l1, l2, YzyIC<8>{}); break;
+            case 1: f(l, YzyIC<1>{}); break;
+            case 2: f(l, YzyIC<2>{}); break;
+            case 3: f(l, YzyIC<3>{}); break;
+            case 4: f(l, YzyIC<4>{}); break;
+            case 5: f(l, YzyIC<5>{}); break;
+            case 6: f(l, YzyIC<6>{}); break;
+            case 7: f(l, YzyIC<7>{}); break;
+            case 8: f(l, YzyIC<8>{}); break;
             default: break;
         }
     };
     switch (Ly) {
-        case 256: nzs(YzyIC<16>{}, YzyIC<16>{}); break;
-        case 512: nzs(YzyIC<32>{}, YzyIC<16>{}); break;
-        case 1024: nzs(YzyIC<32>{}, YzyIC<32>{}); break;
+        case 256: nzs(YzyIC<256>{}); break;
+        case 512: nzs(YzyIC<512>{}); break;
+        case 1024: nzs(YzyIC<1024>{}); break;
         default: break;  // other lengths: the split kernels
     }
 }
@@ -217,21 +253,7 @@ void yzy_with_p(int P, F &&f) {
     }
 }
 
-// static: every unit that includes this header has its own copy of the
-// constant twiddle table (fftreg.cuh) and must fill that one
-static bool yzy_upload_tw64(Backend &b) {
-    double2 d[64];
-    float2 f[64];
-    for (int k = 0; k < 64; ++k) {
-        const double ang = 2.0 * 3.14159265358979323846 * (double)k / 64.0;
-        d[k] = make_double2(std::cos(ang), -std::sin(ang));
-        f[k] = make_float2((float)d[k].x, (float)d[k].y);
-    }
-    return cuda_ok(b, cudaMemcpyToSymbol(c_tw64d, d, sizeof(d)), "twiddle64 d (yzy)") &&
-           cuda_ok(b, cudaMemcpyToSymbol(c_tw64f, f, sizeof(f)), "twiddle64 f (yzy)");
-}
-
-template <typename T, int L1, int L2, int NZ, int P>
+template <typename T, int L, int NZ, int P>
 cudaLaunchConfig_t yzy_config(const Backend &b, cudaLaunchAttribute *attr) {
     cudaLaunchConfig_t cfg = {};
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -239,8 +261,8 @@ cudaLaunchConfig_t yzy_config(const Backend &b, cudaLaunchAttribute *attr) {
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.gridDim = dim3((unsigned)(b.nkx * P));
-    cfg.blockDim = dim3((unsigned)yzy_threads<T, L2, NZ, P>());
-    cfg.dynamicSmemBytes = yzy_smem<T, L1, L2, NZ, P>();
+    cfg.blockDim = dim3((unsigned)yzy_threads<T, L, NZ, P>());
+    cfg.dynamicSmemBytes = yzy_smem<T, L, NZ, P>();
     cfg.stream = b.stream;
     cfg.attrs = attr;
     cfg.numAttrs = P > 1 ? 1 : 0;
@@ -252,24 +274,23 @@ bool yzy_configure_t(Backend &b) {
     b.use_yzy = false;
     b.yzy_P = 0;
     const char *off = std::getenv("FULLMAG_FDM_YZY");
-    if (b.thin || !b.zdirect || b.Ly != 2 * b.ny || (off && std::strcmp(off, "off") == 0)) return true;
+    if (b.thin || !b.zdirect || (off && std::strcmp(off, "off") == 0)) return true;
     // cluster size: FULLMAG_FDM_YZY_P, else the smallest P whose CTA fits twice per SM
     int want = 0;
     if (const char *p = std::getenv("FULLMAG_FDM_YZY_P")) want = std::atoi(p);
     // FP64 only on request: at 512 x 512 x 8 its 8-CTA clusters ran 320 us against
     // 244 us for the three split kernels
     if (sizeof(T) == 8 && !want) return true;
-    if (!yzy_upload_tw64(b)) return false;
-    yzy_dispatch(b.Ly, b.nz, [&](auto l1, auto l2, auto nzc) {
-        constexpr int L1 = decltype(l1)::value, L2 = decltype(l2)::value, NZ = decltype(nzc)::value;
+    yzy_dispatch(b.Ly, b.nz, [&](auto l, auto nzc) {
+        constexpr int L = decltype(l)::value, NZ = decltype(nzc)::value;
         for (int P : {1, 2, 4, 8}) {
             if (b.use_yzy || (want && P != want)) continue;
             yzy_with_p(P, [&](auto pc) {
                 constexpr int PP = decltype(pc)::value;
-                if constexpr (yzy_fits<T, L1, L2, NZ, PP>()) {
-                    constexpr size_t smem = yzy_smem<T, L1, L2, NZ, PP>();
+                if constexpr (yzy_fits<T, L, NZ, PP>()) {
+                    constexpr size_t smem = yzy_smem<T, L, NZ, PP>();
                     if (!want && PP < 8 && smem > kYzySmemMax / 2) return;  // one CTA per SM: try a larger cluster
-                    auto kern = k_yzy<T, L1, L2, NZ, PP>;
+                    auto kern = k_yzy<T, L, NZ, PP>;
                     // the largest shared-memory carveout, so that two CTAs fit per SM
                     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
                         cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
@@ -279,7 +300,7 @@ bool yzy_configure_t(Backend &b) {
                     }
                     if constexpr (PP > 1) {
                         cudaLaunchAttribute attr[1];
-                        cudaLaunchConfig_t cfg = yzy_config<T, L1, L2, NZ, PP>(b, attr);
+                        cudaLaunchConfig_t cfg = yzy_config<T, L, NZ, PP>(b, attr);
                         int nclusters = 0;
                         if (cudaOccupancyMaxActiveClusters(&nclusters, kern, &cfg) != cudaSuccess || nclusters < 1) {
                             cudaGetLastError();
@@ -297,18 +318,41 @@ bool yzy_configure_t(Backend &b) {
 
 template <typename T>
 bool yzy_launch_t(Backend &b, const DemagArgs<T> &a) {
-    yzy_dispatch(b.Ly, b.nz, [&](auto l1, auto l2, auto nzc) {
-        constexpr int L1 = decltype(l1)::value, L2 = decltype(l2)::value, NZ = decltype(nzc)::value;
+    yzy_dispatch(b.Ly, b.nz, [&](auto l, auto nzc) {
+        constexpr int L = decltype(l)::value, NZ = decltype(nzc)::value;
         yzy_with_p(b.yzy_P, [&](auto pc) {
             constexpr int PP = decltype(pc)::value;
-            if constexpr (yzy_fits<T, L1, L2, NZ, PP>()) {
+            if constexpr (yzy_fits<T, L, NZ, PP>()) {
                 cudaLaunchAttribute attr[1];
-                cudaLaunchConfig_t cfg = yzy_config<T, L1, L2, NZ, PP>(b, attr);
-                cudaLaunchKernelEx(&cfg, k_yzy<T, L1, L2, NZ, PP>, a);
+                cudaLaunchConfig_t cfg = yzy_config<T, L, NZ, PP>(b, attr);
+                cudaLaunchKernelEx(&cfg, k_yzy<T, L, NZ, PP>, a);
             }
         });
     });
     return true;
+}
+
+// Values per row of the fused pass's z table for length Ly (0: other lengths).
+template <typename T> inline int yzy_table_row(int Ly) {
+    int r = 0;
+    yzy_dispatch(Ly, 1, [&](auto l, auto) { r = yzy_row<T, decltype(l)::value>(); });
+    return r;
+}
+
+// One row of the direct z table (ky = 0..Ly/2) in the order k_yzy reads it: place
+// i = k0 M0 + idx of tile row k0 <= R0 / 2 holds the frequency in that slot, those
+// above Ly / 2 by the ky mirror with `sign` (-1 for components odd in y).
+template <typename T>
+inline void yzy_table(int Ly, const double *src, double sign, T *dst) {
+    yzy_dispatch(Ly, 1, [&](auto l, auto) {
+        constexpr int L = decltype(l)::value, R0 = Lf<T, L>::R0, M0 = L / R0, M1 = Lf<T, L>::NP == 3 ? Lf<T, L>::M1 : 1;
+        constexpr int R1 = M0 / M1;
+        for (int k0 = 0; k0 <= R0 / 2; ++k0)
+            for (int idx = 0; idx < M0; ++idx) {
+                const int ky = k0 + R0 * (idx / M1 + R1 * (idx % M1));
+                dst[k0 * M0 + idx] = (T)(ky > L / 2 ? sign * src[L - ky] : src[ky]);
+            }
+    });
 }
 
 }  // namespace fm
