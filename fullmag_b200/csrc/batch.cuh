@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(256) k_batch_y(const DemagArgs<T> *__restrict_
 }
 
 // Direct z sum of one column (col = kx Ly + ky) with the table of
-// octant_to_z_direct: the arithmetic of k_zd in the same order per output,
+// octant_to_z_direct: the arithmetic of k_zd (zsum.cuh),
 // inputs and table entries read straight from global memory.
 template <typename T, int NZ>
 __device__ __forceinline__ void zd_col(const DemagArgs<T> &a, int col) {
@@ -93,41 +93,26 @@ __device__ __forceinline__ void zd_col(const DemagArgs<T> &a, int col) {
     const T sy = ymir ? T(-1) : T(1);
     const T *tp = a.spec + (kx * KY + (ymir ? Ly - ky : ky));
     C *base = a.s2 + col;
-    C mx[NZ], my[NZ], mz[NZ], hx[NZ], hy[NZ], hz[NZ];
+    C mx[NZ], my[NZ], mz[NZ];
 #pragma unroll
     for (int z = 0; z < NZ; ++z) {
         mx[z] = base[z * cols];
         my[z] = base[cs + z * cols];
+        my[z].x *= sy; my[z].y *= sy;  // xy and yz change sign with ky: so do My and Hy
         const C v = base[2 * cs + z * cols];
         mz[z] = mk<T>(v.y, -v.x);  // -i Mz
-        hx[z] = mk<T>(0, 0); hy[z] = mk<T>(0, 0); hz[z] = mk<T>(0, 0);
     }
+    T tab[6][NZ];
 #pragma unroll
-    for (int d = 0; d < NZ; ++d) {
-        const T *qd = tp + d * dstr;
-        const T cxx = qd[0], cyy = qd[tstr], czz = qd[2 * tstr], cxy = qd[3 * tstr] * sy;
-        const T cxz = d > 0 ? qd[4 * tstr] : T(0), cyz = d > 0 ? qd[5 * tstr] * sy : T(0);
+    for (int e = 0; e < 6; ++e)
 #pragma unroll
-        for (int z = 0; z + d < NZ; ++z) {
-            {   // output z + d from input z (offset +d)
-                const int o = z + d;
-                zd_fma(hx[o], cxx, mx[z]); zd_fma(hx[o], cxy, my[z]); zd_fma(hx[o], cxz, mz[z]);
-                zd_fma(hy[o], cxy, mx[z]); zd_fma(hy[o], cyy, my[z]); zd_fma(hy[o], cyz, mz[z]);
-                zd_fma(hz[o], -cxz, mx[z]); zd_fma(hz[o], -cyz, my[z]); zd_fma(hz[o], czz, mz[z]);
-            }
-            if (d > 0) {  // output z from input z + d (offset -d: odd-in-z entries flip)
-                const int i = z + d;
-                zd_fma(hx[z], cxx, mx[i]); zd_fma(hx[z], cxy, my[i]); zd_fma(hx[z], -cxz, mz[i]);
-                zd_fma(hy[z], cxy, mx[i]); zd_fma(hy[z], cyy, my[i]); zd_fma(hy[z], -cyz, mz[i]);
-                zd_fma(hz[z], cxz, mx[i]); zd_fma(hz[z], cyz, my[i]); zd_fma(hz[z], czz, mz[i]);
-            }
-        }
-    }
+        for (int d = 0; d < NZ; ++d) tab[e][d] = e < 4 || d > 0 ? tp[e * tstr + d * dstr] : T(0);
+    zsum_column<NZ, T>(mx, my, mz, [&](int e, int d) { return tab[e][d]; });
 #pragma unroll
     for (int z = 0; z < NZ; ++z) {
-        base[z * cols] = hx[z];
-        base[cs + z * cols] = hy[z];
-        base[2 * cs + z * cols] = mk<T>(-hz[z].y, hz[z].x);  // Hz = i Hz'
+        base[z * cols] = mx[z];
+        base[cs + z * cols] = mk<T>(my[z].x * sy, my[z].y * sy);
+        base[2 * cs + z * cols] = mk<T>(-mz[z].y, mz[z].x);  // Hz = i Hz'
     }
 }
 

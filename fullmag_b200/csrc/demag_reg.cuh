@@ -11,6 +11,7 @@
 #include "cpasync.cuh"
 #include "demag.cuh"
 #include "fftreg.cuh"
+#include "zsum.cuh"
 
 namespace fm {
 
@@ -583,26 +584,18 @@ __global__ void __launch_bounds__(128) k_zc_r(DemagArgs<T> a) {
 // FFT pass computes, per (kx, ky) column, the linear convolution
 //   H(z) = -sum_{z' < nz} n(z - z') M(z'),   n(d) = sum_kz N(kx, ky, kz) W_Lz^{-kz d},
 // and only offsets |d| < nz reach a kept output, so the same sum is taken here
-// directly: nz^2 3x3 tensor products per column instead of the two z FFTs,
-// no twiddles and no padded points.  The table (built on the host from the
+// directly (zsum.cuh): nz^2 / 2 3x3 tensor products per column instead of the two
+// z FFTs, no twiddles and no padded points.  The table (built on the host from the
 // octant, newell_host.hpp octant_to_z_direct) holds n(d) for d in [0, nz):
 // components even in z are real; xz and yz are i tau(d) with tau real and odd
 // in d.  With Mz' = -i Mz and Hz' = -i Hz the product is a real matrix on
 // complex vectors,
 //   (Hx, Hy, Hz') = [[-nxx, -nxy, tau_xz], [-nxy, -nyy, tau_yz],
 //                    [-tau_xz, -tau_yz, -nzz]] (Mx, My, Mz'),
-// stored as tab[c][d][kx][ky'] = (-nxx, -nyy, -nzz, -nxy, tau_xz, tau_yz) for
+// stored as tab[c][d][kx][ky'] = (-nxx, -nyy, -nzz, -nxy, tau_xz, tau_yz) / 2 for
 // ky' <= Ly/2.  ky > Ly/2 reads the mirror with the sign of the components odd
 // in y (xy, yz); d < 0 flips the components odd in z (xz, yz).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void zd_fma(float2 &h, float c, float2 m) {
-    h = __ffma2_rn(make_float2(c, c), m, h);  // packed: one instruction for both parts
-}
-__device__ __forceinline__ void zd_fma(double2 &h, double c, double2 m) {
-    h.x = fma(c, m.x, h.x);
-    h.y = fma(c, m.y, h.y);
-}
-
 // Persistent threads, one column per thread per iteration; the
 // next column's inputs and table entries are copied into the thread's own
 // shared-memory slots (cp.async, double buffer) while the current one is
@@ -655,42 +648,22 @@ __global__ void __launch_bounds__(zd_threads<T>()) k_zd(DemagArgs<T> a) {
         const T *st = tb0 + buf * NT * BT + tid;
         const int kx = col / Ly, ky = col - kx * Ly;
         const T sy = ky > Ly / 2 ? T(-1) : T(1);
-        C mx[NZ], my[NZ], mz[NZ], hx[NZ], hy[NZ], hz[NZ];
+        C mx[NZ], my[NZ], mz[NZ];
 #pragma unroll
         for (int z = 0; z < NZ; ++z) {
             mx[z] = sm[z * BT];
             my[z] = sm[(NZ + z) * BT];
+            my[z].x *= sy; my[z].y *= sy;  // xy and yz change sign with ky: so do My and Hy
             const C v = sm[(2 * NZ + z) * BT];
             mz[z] = mk<T>(v.y, -v.x);  // -i Mz
-            hx[z] = mk<T>(0, 0); hy[z] = mk<T>(0, 0); hz[z] = mk<T>(0, 0);
         }
-#pragma unroll
-        for (int d = 0; d < NZ; ++d) {
-            const T cxx = st[d * BT], cyy = st[(NZ + d) * BT], czz = st[(2 * NZ + d) * BT];
-            const T cxy = st[(3 * NZ + d) * BT] * sy;
-            const T cxz = d > 0 ? st[(4 * NZ + d) * BT] : T(0), cyz = d > 0 ? st[(5 * NZ + d) * BT] * sy : T(0);
-#pragma unroll
-            for (int z = 0; z + d < NZ; ++z) {
-                {   // output z + d from input z (offset +d)
-                    const int o = z + d;
-                    zd_fma(hx[o], cxx, mx[z]); zd_fma(hx[o], cxy, my[z]); zd_fma(hx[o], cxz, mz[z]);
-                    zd_fma(hy[o], cxy, mx[z]); zd_fma(hy[o], cyy, my[z]); zd_fma(hy[o], cyz, mz[z]);
-                    zd_fma(hz[o], -cxz, mx[z]); zd_fma(hz[o], -cyz, my[z]); zd_fma(hz[o], czz, mz[z]);
-                }
-                if (d > 0) {  // output z from input z + d (offset -d: odd-in-z entries flip)
-                    const int i = z + d;
-                    zd_fma(hx[z], cxx, mx[i]); zd_fma(hx[z], cxy, my[i]); zd_fma(hx[z], -cxz, mz[i]);
-                    zd_fma(hy[z], cxy, mx[i]); zd_fma(hy[z], cyy, my[i]); zd_fma(hy[z], -cyz, mz[i]);
-                    zd_fma(hz[z], cxz, mx[i]); zd_fma(hz[z], cyz, my[i]); zd_fma(hz[z], czz, mz[i]);
-                }
-            }
-        }
+        zsum_column<NZ, T>(mx, my, mz, [&](int e, int d) { return st[(e * NZ + d) * BT]; });
         C *base = a.s2 + col;
 #pragma unroll
         for (int z = 0; z < NZ; ++z) {
-            base[z * cols] = hx[z];
-            base[cs + z * cols] = hy[z];
-            base[2 * cs + z * cols] = mk<T>(-hz[z].y, hz[z].x);  // Hz = i Hz'
+            base[z * cols] = mx[z];
+            base[cs + z * cols] = mk<T>(my[z].x * sy, my[z].y * sy);
+            base[2 * cs + z * cols] = mk<T>(-mz[z].y, mz[z].x);  // Hz = i Hz'
         }
     }
     cp_async_wait_all();

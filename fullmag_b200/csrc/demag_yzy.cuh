@@ -30,8 +30,8 @@
 // multiply-adds per column (2.05 cycles each per scheduler, the FP32 peak).
 // 106 us with 3-pass lines of 64 threads and named barriers, 100 us with the
 // two-pass lines of one warp each; P = 1 (384 threads) 114 us.
-// One unit per precision (demag_yzy_f32.cu, demag_yzy_f64.cu), so that they
-// compile in parallel.
+// Two units per precision (demag_yzy_f32.cu, demag_yzy_f32b.cu, ..: nz <= 4 and
+// above), so that they compile in parallel.
 #pragma once
 #include <cooperative_groups.h>
 
@@ -152,53 +152,26 @@ __global__ void __launch_bounds__((yzy_threads<T, L, NZ, P>()), (yzy_min_blocks<
             const bool mir = 2 * k0 > R0;
             const T sy = mir ? T(-1) : T(1);
             const T *tp = a.spec + ((long long)kx * ROW + (mir ? (R0 - k0) * M0 + (M0 - 1 - idx) : i));
-            // the table entries of offset d, loaded two offsets ahead of their use
-            T nx_[2][6];
-            auto fetch = [&](int d, T (&c)[6]) {
-                const T *qd = tp + d * dstr;
+            T tab[6][NZ];  // the column's table entries, all in flight at once
 #pragma unroll
-                for (int e = 0; e < 6; ++e) c[e] = (e < 4 || d > 0) ? __ldg(qd + e * tstr) : T(0);
-            };
-            fetch(0, nx_[0]);
-            if (NZ > 1) fetch(1, nx_[1]);
+            for (int e = 0; e < 6; ++e)
+#pragma unroll
+                for (int d = 0; d < NZ; ++d) tab[e][d] = e < 4 || d > 0 ? __ldg(tp + e * tstr + d * dstr) : T(0);
             C mx[NZ], my[NZ], mz[NZ];
 #pragma unroll
             for (int z = 0; z < NZ; ++z) {
                 mx[z] = cell(z, sl);
                 my[z] = cell(NZ + z, sl);
+                my[z].x *= sy; my[z].y *= sy;  // xy and yz change sign with ky: so do My and Hy
                 const C v = cell(2 * NZ + z, sl);
                 mz[z] = mk<T>(v.y, -v.x);  // -i Mz
             }
-            C hx[NZ], hy[NZ], hz[NZ];
-#pragma unroll
-            for (int z = 0; z < NZ; ++z) { hx[z] = mk<T>(0, 0); hy[z] = mk<T>(0, 0); hz[z] = mk<T>(0, 0); }
-            // the loop of k_zd: per output, offsets d ascending, +d then -d
-#pragma unroll
-            for (int d = 0; d < NZ; ++d) {
-                const T cxx = nx_[d & 1][0], cyy = nx_[d & 1][1], czz = nx_[d & 1][2], cxy = nx_[d & 1][3] * sy;
-                const T cxz = nx_[d & 1][4], cyz = nx_[d & 1][5] * sy;
-                if (d + 2 < NZ) fetch(d + 2, nx_[d & 1]);
-#pragma unroll
-                for (int z = 0; z + d < NZ; ++z) {
-                    {   // output z + d from input z (offset +d)
-                        const int o = z + d;
-                        zd_fma(hx[o], cxx, mx[z]); zd_fma(hx[o], cxy, my[z]); zd_fma(hx[o], cxz, mz[z]);
-                        zd_fma(hy[o], cxy, mx[z]); zd_fma(hy[o], cyy, my[z]); zd_fma(hy[o], cyz, mz[z]);
-                        zd_fma(hz[o], -cxz, mx[z]); zd_fma(hz[o], -cyz, my[z]); zd_fma(hz[o], czz, mz[z]);
-                    }
-                    if (d > 0) {  // output z from input z + d (offset -d: odd-in-z entries flip)
-                        const int j = z + d;
-                        zd_fma(hx[z], cxx, mx[j]); zd_fma(hx[z], cxy, my[j]); zd_fma(hx[z], -cxz, mz[j]);
-                        zd_fma(hy[z], cxy, mx[j]); zd_fma(hy[z], cyy, my[j]); zd_fma(hy[z], -cyz, mz[j]);
-                        zd_fma(hz[z], cxz, mx[j]); zd_fma(hz[z], cyz, my[j]); zd_fma(hz[z], czz, mz[j]);
-                    }
-                }
-            }
+            zsum_column<NZ, T>(mx, my, mz, [&](int e, int d) { return tab[e][d]; });
 #pragma unroll
             for (int z = 0; z < NZ; ++z) {
-                cell(z, sl) = hx[z];
-                cell(NZ + z, sl) = hy[z];
-                cell(2 * NZ + z, sl) = mk<T>(-hz[z].y, hz[z].x);  // Hz = i Hz'
+                cell(z, sl) = mx[z];
+                cell(NZ + z, sl) = mk<T>(my[z].x * sy, my[z].y * sy);
+                cell(2 * NZ + z, sl) = mk<T>(-mz[z].y, mz[z].x);  // Hz = i Hz'
             }
         }
     }
@@ -218,19 +191,24 @@ __global__ void __launch_bounds__((yzy_threads<T, L, NZ, P>()), (yzy_min_blocks<
 
 template <int N> using YzyIC = std::integral_constant<int, N>;
 
-// Ly in 256..1024 and NZ of nz as compile-time values
+// Ly in 256..1024 and NZ of nz as compile-time values: nz <= 4 in the units with
+// YZY_HALF 0, above in those with 1
+// static: the two halves have different bodies
 template <class F>
-void yzy_dispatch(int Ly, int nz, F &&f) {
+static void yzy_dispatch(int Ly, int nz, F &&f) {
     auto nzs = [&](auto l) {
         switch (nz) {
+#if YZY_HALF == 0
             case 1: f(l, YzyIC<1>{}); break;
             case 2: f(l, YzyIC<2>{}); break;
             case 3: f(l, YzyIC<3>{}); break;
             case 4: f(l, YzyIC<4>{}); break;
+#else
             case 5: f(l, YzyIC<5>{}); break;
             case 6: f(l, YzyIC<6>{}); break;
             case 7: f(l, YzyIC<7>{}); break;
             case 8: f(l, YzyIC<8>{}); break;
+#endif
             default: break;
         }
     };
@@ -270,7 +248,7 @@ cudaLaunchConfig_t yzy_config(const Backend &b, cudaLaunchAttribute *attr) {
 }
 
 template <typename T>
-bool yzy_configure_t(Backend &b) {
+static bool yzy_configure_t(Backend &b) {
     b.use_yzy = false;
     b.yzy_P = 0;
     const char *off = std::getenv("FULLMAG_FDM_YZY");
@@ -317,7 +295,7 @@ bool yzy_configure_t(Backend &b) {
 }
 
 template <typename T>
-bool yzy_launch_t(Backend &b, const DemagArgs<T> &a) {
+static bool yzy_launch_t(Backend &b, const DemagArgs<T> &a) {
     yzy_dispatch(b.Ly, b.nz, [&](auto l, auto nzc) {
         constexpr int L = decltype(l)::value, NZ = decltype(nzc)::value;
         yzy_with_p(b.yzy_P, [&](auto pc) {
@@ -333,7 +311,7 @@ bool yzy_launch_t(Backend &b, const DemagArgs<T> &a) {
 }
 
 // Values per row of the fused pass's z table for length Ly (0: other lengths).
-template <typename T> inline int yzy_table_row(int Ly) {
+template <typename T> static int yzy_table_row(int Ly) {
     int r = 0;
     yzy_dispatch(Ly, 1, [&](auto l, auto) { r = yzy_row<T, decltype(l)::value>(); });
     return r;
@@ -343,7 +321,7 @@ template <typename T> inline int yzy_table_row(int Ly) {
 // i = k0 M0 + idx of tile row k0 <= R0 / 2 holds the frequency in that slot, those
 // above Ly / 2 by the ky mirror with `sign` (-1 for components odd in y).
 template <typename T>
-inline void yzy_table(int Ly, const double *src, double sign, T *dst) {
+static void yzy_table(int Ly, const double *src, double sign, T *dst) {
     yzy_dispatch(Ly, 1, [&](auto l, auto) {
         constexpr int L = decltype(l)::value, R0 = Lf<T, L>::R0, M0 = L / R0, M1 = Lf<T, L>::NP == 3 ? Lf<T, L>::M1 : 1;
         constexpr int R1 = M0 / M1;

@@ -1,23 +1,17 @@
 // demag_zdw.cuh — direct z convolution for 8 < nz <= 16 in FP32 (the split
 // y / z / y path of 3-D grids whose z lines are too long for one thread).
 //
-// k_zd (demag_reg.cuh) sums the whole column in one thread: 3 nz inputs and
-// 3 nz outputs in registers, which for nz = 16 would be 192 FP32 registers of
-// data alone.  Here a column is split by output half over two warps of the
-// block, so each thread holds the column's 3 nz inputs and 3 ceil(nz/2)
-// accumulators (96 + 48 registers at nz = 16):
+// k_zd (demag_reg.cuh) sums the whole column in one thread, which for nz = 16
+// would be 192 FP32 registers of inputs and outputs alone.  Here the two sets of
+// zsum.cuh go to two warps of the block, each with 3 nz/2 inputs and as many sums:
 //   - a block of 4 warps takes 64 consecutive columns (col = kx Ly + ky) per
-//     iteration of its persistent loop; warps 0-1 sum outputs z < H = ceil(nz/2)
-//     of columns [c0, c0 + 64), warps 2-3 outputs z >= H of the same columns
-//     (in the z-reversed frame, with the same code);
+//     iteration of its persistent loop; warps 0-1 sum set S of columns
+//     [c0, c0 + 64), warps 2-3 set A of the same columns;
 //   - the 64 columns' inputs (3 nz complex) and table entries (6 nz reals) are
 //     copied into shared memory with cp.async by all 128 threads, double
 //     buffered: the next batch's copies run while this batch is summed, and
-//     both halves read one copy.
-// Per output the sum runs over offsets d ascending with the table of k_zd
-// (tab[c][d][kx][ky'], newell_host.hpp octant_to_z_direct) and the same packed
-// FMAs; the lower half's outputs are bitwise k_zd's, the upper half's sum each
-// pair of +d / -d terms in the other order.
+//     both sets read one copy; the sums are exchanged in the input slots.
+// The sums and their order are k_zd's, so the outputs are bitwise its own.
 // Shared memory: 2 buffers x 64 columns x (3 nz complex + 6 nz reals),
 // 96 KiB at nz = 16 (99 KiB in the window form below): two blocks per SM.
 // No TMA; plain cp.async copies.
@@ -54,65 +48,67 @@ template <int NZ, bool WIN> __host__ __device__ constexpr size_t zdw_buf_bytes()
 }
 template <int NZ, bool WIN> __host__ __device__ constexpr size_t zdw_smem() { return 2 * zdw_buf_bytes<NZ, WIN>(); }
 
-// Outputs of one column: z < H = ceil(nz / 2) (rev = false), or z >= H summed
-// in the z-reversed frame (rev = true).  Reversing z (z' = nz - 1 - z) maps
-// offset d to -d, which flips the components odd in z (xz, yz), so the upper
-// half runs the lower half's code on the inputs read in reverse order with
-// those two entries negated, and stores its outputs in reverse order: one code
-// path for both warps of a column (the fully unrolled sum is long enough that
-// two paths compete for the instruction cache).  Per output the sum runs over
-// offsets d ascending, the inputs below the output first.  si / st: the
-// column's inputs and table entries in the batch buffer (slot strides
-// kZdwCols and TS).
-template <int NZ, int TS>
-__device__ __forceinline__ void zdw_col(const float2 *si, const float *st, bool ymir, bool rev, float2 *base,
-                                        int cols, bool store) {
-    constexpr int H = (NZ + 1) / 2, CS = kZdwCols;
-    float2 mx[NZ], my[NZ], mz[NZ];
+// One set (zsum.cuh) of one column: the thread of set S or A reads the column's
+// inputs and table entries from the batch buffer (si, st: slot strides kZdwCols and
+// TS), the two exchange their sums through the column's input slots, and S stores
+// the outputs z < H (and the middle one's x and y for odd nz), A those above (and the
+// middle z).  bar: the named barrier of the 64 threads that share 32 columns.
+template <int NZ, int TS, bool SETA>
+__device__ __forceinline__ void zdw_col(float2 *si, const float *st, float sy, float2 *base, int cols, bool store,
+                                        int bar) {
+    constexpr int H = NZ / 2, CS = kZdwCols;
+    auto group_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(bar) : "memory"); };
+    float2 x[H + 1], y[H + 1], z[H + 1], mid[3];
 #pragma unroll
-    for (int z = 0; z < NZ; ++z) {
-        const int zz = rev ? NZ - 1 - z : z;
-        mx[z] = si[zz * CS];
-        my[z] = si[(NZ + zz) * CS];
-        const float2 v = si[(2 * NZ + zz) * CS];
-        mz[z] = make_float2(v.y, -v.x);  // -i Mz
+    for (int j = 0; j < H; ++j) {
+        const float2 xa = si[j * CS], xb = si[(NZ - 1 - j) * CS];
+        float2 ya = si[(NZ + j) * CS], yb = si[(2 * NZ - 1 - j) * CS];
+        const float2 va = si[(2 * NZ + j) * CS], vb = si[(3 * NZ - 1 - j) * CS];
+        ya.x *= sy; ya.y *= sy; yb.x *= sy; yb.y *= sy;  // xy and yz change sign with ky: so do My and Hy
+        const float2 za = make_float2(va.y, -va.x), zb = make_float2(vb.y, -vb.x);  // -i Mz
+        x[j] = SETA ? zs_sub(xa, xb) : zs_add(xa, xb);
+        y[j] = SETA ? zs_sub(ya, yb) : zs_add(ya, yb);
+        z[j] = SETA ? zs_neg(zs_add(za, zb)) : zs_sub(za, zb);
     }
-    float2 hx[H], hy[H], hz[H];
-#pragma unroll
-    for (int j = 0; j < H; ++j) { hx[j] = make_float2(0.f, 0.f); hy[j] = hx[j]; hz[j] = hx[j]; }
-    const float sy = ymir ? -1.f : 1.f, sz = rev ? -1.f : 1.f;
-#pragma unroll
-    for (int d = 0; d < NZ; ++d) {
-        const float cxx = st[d * TS], cyy = st[(NZ + d) * TS], czz = st[(2 * NZ + d) * TS];
-        const float cxy = st[(3 * NZ + d) * TS] * sy;
-        const float cxz = d > 0 ? st[(4 * NZ + d) * TS] * sz : 0.f;
-        const float cyz = d > 0 ? st[(5 * NZ + d) * TS] * (sy * sz) : 0.f;
-#pragma unroll
-        for (int o = 0; o < H; ++o) {
-            if (o - d >= 0) {  // output o from input o - d (offset +d)
-                const int z = o - d;
-                zd_fma(hx[o], cxx, mx[z]); zd_fma(hx[o], cxy, my[z]); zd_fma(hx[o], cxz, mz[z]);
-                zd_fma(hy[o], cxy, mx[z]); zd_fma(hy[o], cyy, my[z]); zd_fma(hy[o], cyz, mz[z]);
-                zd_fma(hz[o], -cxz, mx[z]); zd_fma(hz[o], -cyz, my[z]); zd_fma(hz[o], czz, mz[z]);
-            }
-            if (d > 0 && o + d < NZ) {  // output o from input o + d (offset -d: odd-in-z entries flip)
-                const int i = o + d;
-                zd_fma(hx[o], cxx, mx[i]); zd_fma(hx[o], cxy, my[i]); zd_fma(hx[o], -cxz, mz[i]);
-                zd_fma(hy[o], cxy, mx[i]); zd_fma(hy[o], cyy, my[i]); zd_fma(hy[o], -cyz, mz[i]);
-                zd_fma(hz[o], cxz, mx[i]); zd_fma(hz[o], cyz, my[i]); zd_fma(hz[o], czz, mz[i]);
-            }
-        }
+    if (NZ & 1) {
+        mid[0] = si[H * CS];
+        mid[1] = si[(NZ + H) * CS];
+        mid[1].x *= sy; mid[1].y *= sy;
+        const float2 v = si[(2 * NZ + H) * CS];
+        mid[2] = make_float2(v.y, -v.x);
     }
+    float2 X[H + 1], Y[H + 1], Z[H + 1];
+    zsum_set<SETA, NZ, float>(x, y, z, X, Y, Z, mid, [&](int e, int d) { return st[(e * NZ + d) * TS]; });
+    group_sync();  // both sets have read the inputs: their slots carry the sums
+    float2 *mine = si + (SETA ? 3 * H * CS : 0), *other = si + (SETA ? 0 : 3 * H * CS);
+#pragma unroll
+    for (int i = 0; i < H; ++i) {
+        mine[i * CS] = X[i];
+        mine[(H + i) * CS] = Y[i];
+        mine[(2 * H + i) * CS] = Z[i];
+    }
+    group_sync();
     if (!store) return;
     const int cs = NZ * cols;
 #pragma unroll
-    for (int j = 0; j < H; ++j) {
-        // odd nz: the reversed frame's last output is the lower half's
-        if ((NZ & 1) && rev && j == H - 1) continue;
-        const int o = rev ? NZ - 1 - j : j;
-        base[o * cols] = hx[j];
-        base[cs + o * cols] = hy[j];
-        base[2 * cs + o * cols] = make_float2(-hz[j].y, hz[j].x);  // Hz = i Hz'
+    for (int i = 0; i < H; ++i) {
+        const float2 ox = other[i * CS], oy = other[(H + i) * CS], oz = other[(2 * H + i) * CS];
+        // S: (S_x + A_x, S_y + A_y, A_z + S_z) at i; A: (S_x - A_x, S_y - A_y, S_z - A_z) at nz - 1 - i; Z of A = -S_z
+        const float2 hx = SETA ? zs_sub(ox, X[i]) : zs_add(X[i], ox);
+        const float2 hy = SETA ? zs_sub(oy, Y[i]) : zs_add(Y[i], oy);
+        const float2 hz = SETA ? zs_neg(zs_add(Z[i], oz)) : zs_sub(Z[i], oz);
+        const int o = SETA ? NZ - 1 - i : i;
+        base[o * cols] = hx;
+        base[cs + o * cols] = make_float2(hy.x * sy, hy.y * sy);
+        base[2 * cs + o * cols] = make_float2(-hz.y, hz.x);  // Hz = i Hz'
+    }
+    if (NZ & 1) {
+        if (SETA) {
+            base[2 * cs + H * cols] = make_float2(-mid[2].y, mid[2].x);
+        } else {
+            base[H * cols] = mid[0];
+            base[cs + H * cols] = make_float2(mid[1].x * sy, mid[1].y * sy);
+        }
     }
 }
 
@@ -184,10 +180,11 @@ __global__ void __launch_bounds__(kZdwThreads, 2) k_zdw(DemagArgs<float> a, int 
         // the column's table entries: its own slot position, or in the window
         // form ky' - wstart (64 - cl for a mirrored batch)
         const int ti = WIN ? ((ky - cl) >= Ly / 2 ? CS - cl : cl) : cl;
-        const float2 *si = in_buf(buf) + cl;
+        float2 *si = in_buf(buf) + cl;
         const float *st = tab_buf(buf) + ti;
         float2 *base = a.s2 + (ok ? col : 0);
-        zdw_col<NZ, TS>(si, st, ky > Ly / 2, half != 0, base, cols, ok);
+        if (half == 0) zdw_col<NZ, TS, false>(si, st, ky > Ly / 2 ? -1.f : 1.f, base, cols, ok, 1 + (warp & 1));
+        else zdw_col<NZ, TS, true>(si, st, ky > Ly / 2 ? -1.f : 1.f, base, cols, ok, 1 + (warp & 1));
         __syncthreads();  // this buffer is refilled by the next iteration's copies
     }
     cp_async_wait_all();

@@ -139,7 +139,11 @@ struct HostFft {
         if (len == 1) { out[0] = in[0]; return; }
         const size_t p = fac[fi], m = len / p;
         for (size_t r = 0; r < p; ++r) rec(in + r * stride, out + r * m, m, stride * p, fi + 1);
-        std::vector<std::complex<double>> t(p), o(p);
+        // small factors (all of a 2,3,5,7-smooth length) combine in a fixed buffer: an
+        // allocation per recursion was most of a short transform's time
+        std::complex<double> tb[8], ob[8];
+        std::vector<std::complex<double>> big(p > 8 ? 2 * p : 0);
+        std::complex<double> *t = p > 8 ? big.data() : tb, *o = p > 8 ? big.data() + p : ob;
         for (size_t k = 0; k < m; ++k) {
             for (size_t r = 0; r < p; ++r)
                 t[r] = out[r * m + k] * tw[((r * k) % len) * (n / len)];
@@ -285,7 +289,7 @@ void octant_to_z_direct(int nkx, int KY, int nz, const std::vector<double> (&spe
         out[c].assign((size_t)nz * plane, 0.0);
         const double *S = spec[c].data();
         double *O = out[c].data();
-        const double sign = oddz[c] ? 1.0 : -1.0;
+        const double half = oddz[c] ? 0.5 : -0.5;
         parallel_for(plane, [&](size_t o) {
             for (int d = 0; d < nz; ++d) {
                 double acc = 0.0;
@@ -293,7 +297,7 @@ void octant_to_z_direct(int nkx, int KY, int nz, const std::vector<double> (&spe
                     acc += S[(size_t)k * plane + o] * (oddz[c] ? sn[(size_t)d * h + k] : cs[(size_t)d * h + k]);
                 acc *= 2.0;
                 if (!oddz[c]) acc += S[o] + ((d & 1) ? -1.0 : 1.0) * S[(size_t)h * plane + o];
-                O[(size_t)d * plane + o] = sign * acc;
+                O[(size_t)d * plane + o] = half * acc;
             }
         });
     }

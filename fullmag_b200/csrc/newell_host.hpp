@@ -29,7 +29,7 @@ void newell_octant_spectra_padded(int nx, int ny, int nz, double dx, double dy, 
 //   odd in z (xz, yz):          i tau(d), tau(d) = 2 sum_{0<k<h} S(k) sin(pi k d / h)
 // (the kz = 0 and kz = h entries of an odd component are zero up to rounding
 // and are left out).  Output layout [c][d][kx][ky], entries
-// (-n_xx, -n_yy, -n_zz, -n_xy, tau_xz, tau_yz): the real matrix of H = -N M on
+// (-n_xx, -n_yy, -n_zz, -n_xy, tau_xz, tau_yz) / 2 (zsum.cuh): half the real matrix of H = -N M on
 // (Mx, My, -i Mz) -> (Hx, Hy, -i Hz).  With zero padding, offsets |d| < nz
 // never wrap for any Lz >= 2 nz - 1, so the sum over z' < nz of n(z - z') M(z')
 // is the padded z convolution kept at z < nz.
