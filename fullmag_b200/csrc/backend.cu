@@ -48,6 +48,10 @@ bool upload_tw64(Backend &b) {
            cuda_ok(b, cudaMemcpyToSymbol(c_tw64f, f, sizeof(f)), "twiddle64 f");
 }
 
+// dynamic shared-memory limit of the kernels whose need varies with the grid: one value
+// per kernel and device, so never less than another handle may ask
+constexpr int kSmemMost = 227 * 1024;
+
 static bool is_pow2(int L) { return L >= 2 && (L & (L - 1)) == 0; }
 
 static bool env_is(const char *name, const char *value) {
@@ -288,7 +292,7 @@ struct Impl {
             b.last_error = "padded FFT length too large for the shared-memory FFT (max 4096 per axis)";
             return false;
         }
-        return cuda_ok(b, cudaFuncSetAttribute(k_z_conv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.smem_z), "attr z_conv");
+        return cuda_ok(b, cudaFuncSetAttribute(k_z_conv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost), "attr z_conv");
     }
 
     static void launch_z_smem(Backend &b, const DemagArgs<T> &a) {
@@ -358,13 +362,13 @@ struct Impl {
             return false;
         }
         bool ok = true;
-        ok &= cuda_ok(b, cudaFuncSetAttribute(k_x_fwd<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.smem_xf), "attr x_fwd");
-        ok &= cuda_ok(b, cudaFuncSetAttribute(k_x_inv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.smem_xf), "attr x_inv");
+        ok &= cuda_ok(b, cudaFuncSetAttribute(k_x_fwd<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost), "attr x_fwd");
+        ok &= cuda_ok(b, cudaFuncSetAttribute(k_x_inv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost), "attr x_inv");
         if (b.thin) {
-            ok &= cuda_ok(b, cudaFuncSetAttribute(k_y_conv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.smem_yc), "attr y_conv");
+            ok &= cuda_ok(b, cudaFuncSetAttribute(k_y_conv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost), "attr y_conv");
         } else {
-            ok &= cuda_ok(b, cudaFuncSetAttribute(k_y_fwd<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.smem_yf), "attr y_fwd");
-            ok &= cuda_ok(b, cudaFuncSetAttribute(k_y_inv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.smem_yf), "attr y_inv");
+            ok &= cuda_ok(b, cudaFuncSetAttribute(k_y_fwd<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost), "attr y_fwd");
+            ok &= cuda_ok(b, cudaFuncSetAttribute(k_y_inv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost), "attr y_inv");
         }
         return ok;
     }

@@ -3,7 +3,7 @@
 // launch per stage for the whole batch (batch.cuh), one CUDA graph per step.
 // No counterpart in the reference; exported through include/fullmag_fdm_ext.h.
 //
-// Per problem: padded lengths are the powers of two >= 2n per axis (any such
+// Per problem: padded in-plane lengths are line-FFT lengths >= 2n (any such
 // length gives the reference's field, see newell_octant_spectra_padded); a
 // film (nz = 1) takes the 3-D pipeline with Lz = 2, the CPU engine's form.
 // The autotuner times each stage kernel at persistent grid sizes of 1..16
@@ -49,23 +49,30 @@ int pow2_at_least(int v) {
     return p;
 }
 
-// Padded in-plane length >= v, at least 16: in FP32 the smallest power of two
-// or 3 * 2^k in 96..768 (lengths fft4step takes with a radix-3 first level), in
-// FP64 a power of two (its batched FFT kernels already use all 255 registers; a
-// radix-3 level would spill more).  FULLMAG_FDM_BATCH_PAD=pow2 keeps powers of
-// two in FP32 too.  Measured on the 256-problem C4 draw (FP32, one process):
-// 4.98 ms per step with powers of two, 4.44 ms with 3 * 2^k from 192 and 4.08 ms
-// (another run) from 96.
-int batch_length(int v, bool dbl) {
-    int L = std::max(16, pow2_at_least(v));
+// Padded in-plane length >= v, at least 16: the line-FFT lengths (linefft.cuh), powers
+// of two and 3 * 2^k.  FULLMAG_FDM_BATCH_PAD=pow2 keeps powers of two.
+int batch_length(int v) {
     const char *e = std::getenv("FULLMAG_FDM_BATCH_PAD");
-    if (dbl || (e && std::strcmp(e, "pow2") == 0)) return L;
-    for (int c : {96, 192, 384, 768})
-        if (c >= v && c < L) L = c;
-    return L;
+    if (e && std::strcmp(e, "pow2") == 0) return std::max(16, pow2_at_least(v));
+    return line_length(std::max(16, v));
 }
 
-constexpr int l2_of(int L) { return l2_for(L); }
+// threads per line of length L, tile elements, and the x passes' line stride
+template <typename T> int line_group(int L) {
+    int g = 1;
+    with_line(L, [&](auto l) { g = Lf<T, decltype(l)::value>::G; });
+    return g;
+}
+template <typename T> int line_tile(int L) {
+    int n = 0;
+    with_line(L, [&](auto l) { n = Lf<T, decltype(l)::value>::TILE; });
+    return n;
+}
+template <typename T> int line_te(int L, int lp) {
+    int n = 0;
+    with_line(L, [&](auto l) { n = line_stride<T, decltype(l)::value>(lp); });
+    return n;
+}
 
 // kernel kinds tuned and launched per step
 enum { KX_FWD = 0, KY_FWD, KZ, KY_INV, KX_INV, KSTAGE, KCOMB, NKINDS };
@@ -81,8 +88,7 @@ struct BatchImpl {
     };
     std::vector<Prob> probs;
     void *arena = nullptr;
-    std::vector<std::pair<int, size_t>> tw_off;   // (L, offset) of shared twiddle tables
-    std::vector<std::pair<int, size_t>> tw4_off;  // (L, offset) of the 4-step tables (host_tw4)
+    std::vector<std::pair<int, size_t>> tw_off;   // (L, offset) of the line-FFT twiddle tables
     // device argument tables and work lists
     DemagArgs<T> *dA_m = nullptr, *dA_s = nullptr;  // demag of m / of m_stage
     StageArgs<T> *dS_eval = nullptr, *dS_corr = nullptr;
@@ -90,9 +96,10 @@ struct BatchImpl {
     int *d_zb = nullptr;
     int4 *dW[NKINDS] = {};
     int nW[NKINDS] = {};
-    size_t smem_x = 0, smem_y = 0;   // for 256-thread x / y blocks (the larger tile)
+    size_t smem_x[2] = {0, 0}, smem_y[2] = {0, 0};  // for 128- and 256-thread x / y blocks
+    bool long_lines = false;         // a line over 512 points: the LONG forms of the x / y kernels
     // tile shape of the x and y passes, chosen by the autotuner: threads per block
-    // (128 or 256), so a block holds tpb / L2 lines of each problem
+    // (128 or 256), so a block holds tpb / G lines of each problem
     int tpb_x = 256, tpb_y = 256;
     int capW[NKINDS] = {};           // work-list capacity (the 128-thread lists are the longest)
     int grid[NKINDS] = {};
@@ -142,10 +149,10 @@ struct BatchImpl {
             p.n = (long long)d.nx * d.ny * d.nz;
             zmax = std::max(zmax, (int)d.nz);
             // in-plane lengths of at least 16 (the smallest the batched x / y kernels take)
-            p.Lx = batch_length(2 * (int)d.nx, sizeof(T) == 8);
-            p.Ly = batch_length(2 * (int)d.ny, sizeof(T) == 8);
+            p.Lx = batch_length(2 * (int)d.nx);
+            p.Ly = batch_length(2 * (int)d.ny);
             p.Lz = pow2_at_least(2 * (int)d.nz);
-            if (p.Lx > 1024 || p.Ly > 1024 || p.Lz > 16) {
+            if (p.Lx == 0 || p.Ly == 0 || p.Lx > 1024 || p.Ly > 1024 || p.Lz > 16) {
                 B.last_error = "problem " + std::to_string(i) + ": grid too large for the batch (nx, ny <= 512, nz <= 8)";
                 return false;
             }
@@ -160,14 +167,12 @@ struct BatchImpl {
             p.off_s1 = take((size_t)3 * d.nz * p.nkx * d.ny * cs);
             p.off_s2 = take((size_t)3 * d.nz * p.nkx * p.Ly * cs);
             p.off_spec = take((size_t)6 * p.KZ * p.nkx * p.KY * s);
-            const int Ls[3] = {p.Lx, p.Ly, p.Lz};
+            const int Ls[2] = {p.Lx, p.Ly};
             for (int L : Ls) {
+                long_lines = long_lines || L > 512;
                 bool have = false;
                 for (auto &t : tw_off) have = have || t.first == L;
-                if (!have) {
-                    tw_off.push_back({L, take((size_t)L * cs)});
-                    tw4_off.push_back({L, take((size_t)L * cs)});
-                }
+                if (!have) tw_off.push_back({L, take((size_t)line_twiddle_count<T>(L) * cs)});
             }
         }
         // FP64 sums of nz > 4 hold more registers than a thread has: z FFTs there
@@ -210,19 +215,9 @@ struct BatchImpl {
             if (nW[k] && !batch_ok(B, cudaMemcpy(dW[k], W[k].data(), W[k].size() * sizeof(int4), cudaMemcpyHostToDevice), "upload work list"))
                 return false;
         }
-        // twiddles exp(-2 pi i k / L), computed in FP64
         for (auto &t : tw_off) {
-            std::vector<C> tw(t.first);
-            for (int k = 0; k < t.first; ++k) {
-                const double a = 2.0 * kPi * (double)k / (double)t.first;
-                tw[k] = mk<T>((T)std::cos(a), (T)(-std::sin(a)));
-            }
+            const std::vector<C> tw = line_twiddles<T>(t.first);
             if (!batch_ok(B, cudaMemcpy(base() + t.second, tw.data(), tw.size() * sizeof(C), cudaMemcpyHostToDevice), "upload twiddles"))
-                return false;
-        }
-        for (auto &t : tw4_off) {
-            const std::vector<C> tw = host_tw4<T>(t.first);
-            if (!batch_ok(B, cudaMemcpy(base() + t.second, tw.data(), tw.size() * sizeof(C), cudaMemcpyHostToDevice), "upload 4-step twiddles"))
                 return false;
         }
         // per problem: octant spectra, m0, shared-memory needs
@@ -248,37 +243,41 @@ struct BatchImpl {
             if (!batch_ok(B, cudaMemcpy(base() + p.off_m, m.data(), m.size() * sizeof(T), cudaMemcpyHostToDevice), "upload m0"))
                 return false;
             zb[i] = (int)d.nz;
-            const int lx2 = l2_of(p.Lx), ly2 = l2_of(p.Ly);
-            const size_t TEx = (size_t)std::max(lx2 == 1 ? 0 : (p.Lx / lx2) * (lx2 + 1), p.Lx) + 1;
-            smem_x = std::max(smem_x, ((size_t)(256 / lx2) * TEx) * cs);
-            const size_t TEy = ly2 == 1 ? 0 : (size_t)(p.Ly / ly2) * (ly2 + 1);
-            smem_y = std::max(smem_y, ((size_t)(256 / ly2) * TEy) * cs);
+            for (int i = 0; i < 2; ++i) {
+                const int t = 128 << i;
+                const int lx = std::max(1, t / line_group<T>(p.Lx)), ly = std::max(1, t / line_group<T>(p.Ly));
+                smem_x[i] = std::max(smem_x[i], (size_t)lx * line_te<T>(p.Lx, lx) * cs);
+                smem_y[i] = std::max(smem_y[i], (size_t)ly * line_tile<T>(p.Ly) * cs);
+            }
         }
         if (!batch_ok(B, cudaMemcpy(d_zb, zb.data(), count * sizeof(int), cudaMemcpyHostToDevice), "upload zb")) return false;
-        if (smem_x > 227 * 1024 || smem_y > 227 * 1024) { B.last_error = "batch FFT tiles exceed shared memory"; return false; }
-        bool ok = batch_ok(B, cudaFuncSetAttribute(k_batch_x<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_x), "attr x") &&
-                  batch_ok(B, cudaFuncSetAttribute(k_batch_x<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_x), "attr x") &&
-                  batch_ok(B, cudaFuncSetAttribute(k_batch_y<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_y), "attr y") &&
-                  batch_ok(B, cudaFuncSetAttribute(k_batch_y<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_y), "attr y");
+        if (smem_x[1] > 227 * 1024 || smem_y[1] > 227 * 1024) { B.last_error = "batch FFT tiles exceed shared memory"; return false; }
+        // one limit per kernel and device: never less than another batch may ask
+        constexpr int most = 227 * 1024;
+        auto limit = [&](auto kern) { return batch_ok(B, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most), "attr x / y"); };
+        const bool ok = long_lines ? limit(k_batch_x<T, false, true>) && limit(k_batch_x<T, true, true>) &&
+                                         limit(k_batch_y<T, false, true>) && limit(k_batch_y<T, true, true>)
+                                   : limit(k_batch_x<T, false, false>) && limit(k_batch_x<T, true, false>) &&
+                                         limit(k_batch_y<T, false, false>) && limit(k_batch_y<T, true, false>);
         if (!ok) return false;
         return set_tiles(B, 256, 256) && upload_args(B, 1e-13);
     }
 
     // x / y work lists for tx- and ty-thread blocks: x item (problem, row block of
-    // 2 tx / L2 rows, z, component), y item (problem, block of ty / L2 lines)
+    // 2 tx / G rows, z, component), y item (problem, block of ty / G lines)
     void xy_lists(int tx, int ty, std::vector<int4> (&W)[NKINDS]) const {
         for (int k : {KX_FWD, KX_INV, KY_FWD, KY_INV}) W[k].clear();
         for (size_t i = 0; i < probs.size(); ++i) {
             const Prob &p = probs[i];
             const int ny = p.d.ny, nz = p.d.nz;
-            const int RB = 2 * std::max(1, tx / l2_of(p.Lx));
+            const int RB = 2 * std::max(1, tx / line_group<T>(p.Lx));
             for (int c = 0; c < 3; ++c)
                 for (int z = 0; z < nz; ++z)
                     for (int bx = 0; bx < (ny + RB - 1) / RB; ++bx) {
                         W[KX_FWD].push_back(make_int4((int)i, bx, z, c));
                         W[KX_INV].push_back(make_int4((int)i, bx, z, c));
                     }
-            const int ly = std::max(1, ty / l2_of(p.Ly));
+            const int ly = std::max(1, ty / line_group<T>(p.Ly));
             const long long lines = 3LL * nz * p.nkx;
             for (long long bx = 0; bx < (lines + ly - 1) / ly; ++bx) {
                 W[KY_FWD].push_back(make_int4((int)i, (int)bx, 0, 0));
@@ -309,12 +308,6 @@ struct BatchImpl {
         return nullptr;
     }
 
-    const C *tw4(int L) {
-        for (auto &t : tw4_off)
-            if (t.first == L) return (const C *)(base() + t.second);
-        return nullptr;
-    }
-
     // argument tables for step size dt (the predictor and corrector use it)
     bool upload_args(fullmag_fdm_batch &B, double dt) {
         const size_t P = probs.size();
@@ -331,16 +324,16 @@ struct BatchImpl {
             DemagArgs<T> a{};
             a.nx = d.nx; a.ny = d.ny; a.nz = d.nz; a.n = p.n;
             a.Lx = p.Lx; a.Ly = p.Ly; a.Lz = p.Lz; a.nkx = p.nkx; a.KZ = p.KZ; a.KY = p.KY;
-            a.twx = tw(p.Lx); a.twy = tw(p.Ly); a.twz = tw(p.Lz);
-            a.twxT = tw4(p.Lx); a.twyT = tw4(p.Ly);
+            a.twx4 = tw(p.Lx); a.twy4 = tw(p.Ly);
             a.s1 = (C *)(base() + p.off_s1);
             a.s2 = (C *)(base() + p.off_s2);
             a.spec = (const T *)(base() + p.off_spec);
             a.ms = d.saturation_magnetisation;
             a.hd = hd;
             a.norm = 1.0 / ((double)p.Lx * (double)p.Ly * (double)p.Lz);
-            a.lines_x = std::max(1, tpb_x / l2_of(p.Lx));
-            a.lines_y = std::max(1, tpb_y / l2_of(p.Ly));
+            a.lines_x = std::max(1, tpb_x / line_group<T>(p.Lx));
+            a.te_x = line_te<T>(p.Lx, a.lines_x);
+            a.lines_y = std::max(1, tpb_y / line_group<T>(p.Ly));
             a.m = m;
             hA_m[i] = a;
             a.m = ms;
@@ -387,16 +380,28 @@ struct BatchImpl {
     void launch(cudaStream_t st, int kind, bool staged, int G) {
         const DemagArgs<T> *A = staged ? dA_s : dA_m;
         switch (kind) {
-            case KX_FWD: k_batch_x<T, false><<<g(kind, G), tpb_x, smem_x * tpb_x / 256, st>>>(A, dW[kind], nW[kind]); break;
-            case KY_FWD: k_batch_y<T, false><<<g(kind, G), tpb_y, smem_y * tpb_y / 256, st>>>(A, dW[kind], nW[kind]); break;
+            case KX_FWD:
+                if (long_lines) k_batch_x<T, false, true><<<g(kind, G), tpb_x, smem_x[tpb_x / 256], st>>>(A, dW[kind], nW[kind]);
+                else k_batch_x<T, false, false><<<g(kind, G), tpb_x, smem_x[tpb_x / 256], st>>>(A, dW[kind], nW[kind]);
+                break;
+            case KY_FWD:
+                if (long_lines) k_batch_y<T, false, true><<<g(kind, G), tpb_y, smem_y[tpb_y / 256], st>>>(A, dW[kind], nW[kind]);
+                else k_batch_y<T, false, false><<<g(kind, G), tpb_y, smem_y[tpb_y / 256], st>>>(A, dW[kind], nW[kind]);
+                break;
             case KZ:
                 if (zdirect && zmax <= 4) k_batch_z<T, true, 4><<<g(kind, G), 128, 0, st>>>(A, dW[kind], nW[kind]);
                 else if (zdirect) {
                     if constexpr (sizeof(T) == 4) k_batch_z<T, true, 8><<<g(kind, G), 128, 0, st>>>(A, dW[kind], nW[kind]);
                 } else k_batch_z<T, false><<<g(kind, G), 128, 0, st>>>(A, dW[kind], nW[kind]);
                 break;
-            case KY_INV: k_batch_y<T, true><<<g(kind, G), tpb_y, smem_y * tpb_y / 256, st>>>(A, dW[kind], nW[kind]); break;
-            case KX_INV: k_batch_x<T, true><<<g(kind, G), tpb_x, smem_x * tpb_x / 256, st>>>(A, dW[kind], nW[kind]); break;
+            case KY_INV:
+                if (long_lines) k_batch_y<T, true, true><<<g(kind, G), tpb_y, smem_y[tpb_y / 256], st>>>(A, dW[kind], nW[kind]);
+                else k_batch_y<T, true, false><<<g(kind, G), tpb_y, smem_y[tpb_y / 256], st>>>(A, dW[kind], nW[kind]);
+                break;
+            case KX_INV:
+                if (long_lines) k_batch_x<T, true, true><<<g(kind, G), tpb_x, smem_x[tpb_x / 256], st>>>(A, dW[kind], nW[kind]);
+                else k_batch_x<T, true, false><<<g(kind, G), tpb_x, smem_x[tpb_x / 256], st>>>(A, dW[kind], nW[kind]);
+                break;
             case KSTAGE:
                 if (staged)
                     k_batch_stage<T, MODE_HEUN_CORR><<<g(kind, G), dim3(32, kStagePlainBY), 0, st>>>(dS_corr, d_zb, dW[kind], nW[kind]);
@@ -413,7 +418,7 @@ struct BatchImpl {
     }
 
     // Autotuner: for the x and y passes the tile shape (128- or 256-thread blocks,
-    // so tpb / L2 lines of a problem per block) together with the persistent grid
+    // so tpb / G lines of a problem per block) together with the persistent grid
     // size; for the other kernels the grid size; grid sizes from {1, 2, 4, 8, 16}
     // blocks per SM; by CUDA-event time of two launches each (after one warm-up).
     // The stage kernel is tuned in its RHS form, which writes only k1.
@@ -567,15 +572,10 @@ bool batch_upload_tw64(fullmag_fdm_batch &B) {
         d[k] = make_double2(std::cos(a), -std::sin(a));
         f[k] = make_float2((float)d[k].x, (float)d[k].y);
     }
-    double2 d3[192];
-    float2 f3[192];
-    host_tw192(d3, f3);
     // legacy-stream uploads from pageable memory, then a device synchronisation:
     // the batch's stream is non-blocking
     return batch_ok(B, cudaMemcpyToSymbol(c_tw64d, d, sizeof(d)), "twiddle64 d (batch)") &&
            batch_ok(B, cudaMemcpyToSymbol(c_tw64f, f, sizeof(f)), "twiddle64 f (batch)") &&
-           batch_ok(B, cudaMemcpyToSymbol(c_tw192d, d3, sizeof(d3)), "twiddle192 d (batch)") &&
-           batch_ok(B, cudaMemcpyToSymbol(c_tw192f, f3, sizeof(f3)), "twiddle192 f (batch)") &&
            batch_ok(B, cudaDeviceSynchronize(), "twiddle (batch) sync");
 }
 

@@ -3,116 +3,82 @@
 //
 // Every stage of a step is one launch for the whole batch: the blocks walk a
 // work list of (problem, block coordinates) items in grid-stride order and
-// run the same block bodies as the single-problem kernels (demag_reg.cuh,
+// run the same block bodies as the single-problem kernels (demag_line.cuh,
 // stages.cuh) on that problem's arguments.  The padded FFT lengths differ per
 // problem, so each item dispatches on its problem's length; the switch is
 // uniform across the block.  Work lists, per-problem arguments and the grid
 // sizes (chosen by the batch autotuner) are set up by batch.cu.
 #pragma once
 
+#include "demag_line.cuh"
 #include "demag_reg.cuh"
 #include "stages.cuh"
 
 namespace fm {
 
-// x passes: item (p, bx, z, c); 256 threads, lines_x = 256 / L2 per problem;
-// Lx a power of two in 16..1024, or in FP32 3 * 2^k in 96..768 (batch.cu pads
-// every in-plane axis to at least 16)
-template <typename T, bool INV>
-__global__ void __launch_bounds__(256) k_batch_x(const DemagArgs<T> *__restrict__ A, const int4 *__restrict__ work,
-                                                 int nwork) {
+// Blocks of 256 threads per SM the x / y kernels' registers are cut for.  A kernel holds
+// the registers of its longest line, so batches without lines over 512 points take
+// the form without them (LONG = false: FP32 80 registers, 24 warps per SM).
+template <typename T, bool LONG> __host__ __device__ constexpr int batch_min_blocks() {
+    return sizeof(T) == 4 ? (LONG ? 2 : 3) : 1;
+}
+
+// x passes: item (p, bx, z, c); lines_x = threads / G lines per block for each problem;
+// Lx one of the line-FFT lengths 16..1024 (batch.cu pads every in-plane axis to them)
+template <typename T, bool INV, bool LONG>
+__global__ void __launch_bounds__(256, (batch_min_blocks<T, LONG>())) k_batch_x(const DemagArgs<T> *__restrict__ A,
+                                                                                 const int4 *__restrict__ work, int nwork) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
         const int4 it = work[w];
         const DemagArgs<T> &a = A[it.x];
         switch (a.Lx) {
-#define FM_X(L1, L2)                                                             \
-    if (INV) xi_body<T, L1, L2>(a, it.y, it.z, it.w, smem_raw);                  \
-    else xf_body<T, L1, L2, true>(a, it.y, it.z, it.w, smem_raw);                \
-    break;
-            case 16: FM_X(16, 1)
-            case 32: FM_X(32, 1)
-            case 64: FM_X(8, 8)
-            case 96: if constexpr (sizeof(T) == 4) { FM_X(24, 4) } break;
-            case 128: FM_X(16, 8)
-            case 192: if constexpr (sizeof(T) == 4) { FM_X(24, 8) } break;
-            case 256: FM_X(16, 16)
-            case 384: if constexpr (sizeof(T) == 4) { FM_X(48, 8) } break;
-            case 512: FM_X(32, 16)
-            case 768: if constexpr (sizeof(T) == 4) { FM_X(48, 16) } break;
-            case 1024: FM_X(32, 32)
-#undef FM_X
-            default: break;
+#define FM_B(L)                                                                  \
+    case L:                                                                      \
+        if (INV) lx_inv_body<T, L, true>(a, it.y, it.z, it.w, smem_raw);  \
+        else lx_fwd_body<T, L, true>(a, it.y, it.z, it.w, smem_raw);      \
+        break;
+            FM_B(16) FM_B(32) FM_B(64) FM_B(96) FM_B(128) FM_B(192) FM_B(256) FM_B(384) FM_B(512)
+            default:
+                if constexpr (LONG) {
+                    switch (a.Lx) {
+                        FM_B(768) FM_B(1024)
+                        default: break;
+                    }
+                }
+                break;
+#undef FM_B
         }
-        __syncthreads();  // the next item refills the shared tables
+        __syncthreads();  // the next item reuses the line tiles
     }
 }
 
-// y passes: item (p, bx); 256 threads, lines_y = 256 / L2 per problem
-template <typename T, bool INV>
-__global__ void __launch_bounds__(256) k_batch_y(const DemagArgs<T> *__restrict__ A, const int4 *__restrict__ work,
-                                                 int nwork) {
+// y passes: item (p, bx); lines_y = threads / G lines per block
+template <typename T, bool INV, bool LONG>
+__global__ void __launch_bounds__(256, (batch_min_blocks<T, LONG>())) k_batch_y(const DemagArgs<T> *__restrict__ A,
+                                                                                 const int4 *__restrict__ work, int nwork) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
         const int4 it = work[w];
         const DemagArgs<T> &a = A[it.x];
         switch (a.Ly) {
-#define FM_Y(L1, L2)                                                             \
-    if (INV) yi_body<T, L1, L2>(a, it.y, smem_raw);                              \
-    else yf_body<T, L1, L2, true>(a, it.y, smem_raw);                            \
-    break;
-            case 16: FM_Y(16, 1)
-            case 32: FM_Y(32, 1)
-            case 64: FM_Y(8, 8)
-            case 96: if constexpr (sizeof(T) == 4) { FM_Y(24, 4) } break;
-            case 128: FM_Y(16, 8)
-            case 192: if constexpr (sizeof(T) == 4) { FM_Y(24, 8) } break;
-            case 256: FM_Y(16, 16)
-            case 384: if constexpr (sizeof(T) == 4) { FM_Y(48, 8) } break;
-            case 512: FM_Y(32, 16)
-            case 768: if constexpr (sizeof(T) == 4) { FM_Y(48, 16) } break;
-            case 1024: FM_Y(32, 32)
-#undef FM_Y
-            default: break;
+#define FM_B(L)                                                                  \
+    case L:                                                                      \
+        if (INV) ly_inv_body<T, L>(a, it.y, smem_raw);  \
+        else ly_fwd_body<T, L>(a, it.y, smem_raw);      \
+        break;
+            FM_B(16) FM_B(32) FM_B(64) FM_B(96) FM_B(128) FM_B(192) FM_B(256) FM_B(384) FM_B(512)
+            default:
+                if constexpr (LONG) {
+                    switch (a.Ly) {
+                        FM_B(768) FM_B(1024)
+                        default: break;
+                    }
+                }
+                break;
+#undef FM_B
         }
-        __syncthreads();
-    }
-}
-
-// Direct z sum of one column (col = kx Ly + ky) with the table of
-// octant_to_z_direct: the arithmetic of k_zd (zsum.cuh),
-// inputs and table entries read straight from global memory.
-template <typename T, int NZ>
-__device__ __forceinline__ void zd_col(const DemagArgs<T> &a, int col) {
-    using C = cx<T>;
-    const int Ly = a.Ly, KY = a.KY, cols = a.nkx * Ly;
-    if (col >= cols) return;
-    const int cs = NZ * cols, dstr = a.nkx * KY, tstr = NZ * dstr;
-    const int kx = col / Ly, ky = col - kx * Ly;
-    const bool ymir = ky > Ly / 2;
-    const T sy = ymir ? T(-1) : T(1);
-    const T *tp = a.spec + (kx * KY + (ymir ? Ly - ky : ky));
-    C *base = a.s2 + col;
-    C mx[NZ], my[NZ], mz[NZ];
-#pragma unroll
-    for (int z = 0; z < NZ; ++z) {
-        mx[z] = base[z * cols];
-        my[z] = base[cs + z * cols];
-        my[z].x *= sy; my[z].y *= sy;  // xy and yz change sign with ky: so do My and Hy
-        const C v = base[2 * cs + z * cols];
-        mz[z] = mk<T>(v.y, -v.x);  // -i Mz
-    }
-    T tab[6][NZ];
-#pragma unroll
-    for (int e = 0; e < 6; ++e)
-#pragma unroll
-        for (int d = 0; d < NZ; ++d) tab[e][d] = e < 4 || d > 0 ? tp[e * tstr + d * dstr] : T(0);
-    zsum_column<NZ, T>(mx, my, mz, [&](int e, int d) { return tab[e][d]; });
-#pragma unroll
-    for (int z = 0; z < NZ; ++z) {
-        base[z * cols] = mx[z];
-        base[cs + z * cols] = mk<T>(my[z].x * sy, my[z].y * sy);
-        base[2 * cs + z * cols] = mk<T>(-mz[z].y, mz[z].x);  // Hz = i Hz'
+        __syncthreads();  // the next item reuses the line tiles
     }
 }
 

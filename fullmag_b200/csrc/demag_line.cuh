@@ -8,6 +8,7 @@
 #include "demag.cuh"
 #include "demag_line.hpp"
 #include "linefft.cuh"
+#include "zsum.cuh"
 
 namespace fm {
 
@@ -25,14 +26,15 @@ template <typename T, int L> __host__ __device__ constexpr int line_min_blocks()
 // x forward: two rows of Ms m per complex line, R2C, transposed store.
 // grid (ceil(ny / 2 lines_x), nz, 3), lines_x groups of G threads.
 // ---------------------------------------------------------------------------
-template <typename T, int L>
-__global__ void __launch_bounds__((line_max_threads<T, L>()), (line_min_blocks<T, L>())) k_lx_fwd(DemagArgs<T> a) {
+// Block body (row block bx, plane z, component c); UNI: no mask, Ms map, volume
+// fraction or unit source (the batched kernels, batch.cuh).
+template <typename T, int L, bool UNI = false>
+__device__ __forceinline__ void lx_fwd_body(const DemagArgs<T> &a, int bx, int z, int c, unsigned char *smem_raw) {
     using C = cx<T>;
     constexpr int G = Lf<T, L>::G;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
     C *region = reinterpret_cast<C *>(smem_raw);
-    const int LP = a.lines_x, TE = a.te_x, RB = 2 * LP, z = blockIdx.y, c = blockIdx.z;
-    const int y0 = blockIdx.x * RB, nx = a.nx, ny = a.ny;
+    const int LP = a.lines_x, TE = a.te_x, RB = 2 * LP;
+    const int y0 = bx * RB, nx = a.nx, ny = a.ny;
     const int q = threadIdx.x / G, t = threadIdx.x % G;
     const int ya = y0 + 2 * q, yb = ya + 1;
     // rows past the grid read row ny - 1 and are zeroed
@@ -40,7 +42,7 @@ __global__ void __launch_bounds__((line_max_threads<T, L>()), (line_min_blocks<T
     const T *ma = a.m + (long long)c * a.n + rowa, *mb = a.m + (long long)c * a.n + rowb;
     C *line = region + q * TE;
     auto out = [&](int k, C v) { line[line_slot<T, L>(k)] = v; };
-    if (!a.mask && !a.ms_map && !a.vf) {
+    if (UNI || (!a.mask && !a.ms_map && !a.vf)) {
         // M = Ms m in the storage precision
         const T msT = a.unit_source ? T(1) : (T)a.ms;
         const T sa = ya < ny ? msT : T(0), sb = yb < ny ? msT : T(0);
@@ -93,18 +95,23 @@ __global__ void __launch_bounds__((line_max_threads<T, L>()), (line_min_blocks<T
     }
 }
 
+template <typename T, int L>
+__global__ void __launch_bounds__((line_max_threads<T, L>()), (line_min_blocks<T, L>())) k_lx_fwd(DemagArgs<T> a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    lx_fwd_body<T, L>(a, blockIdx.x, blockIdx.y, blockIdx.z, smem_raw);
+}
+
 // ---------------------------------------------------------------------------
 // x inverse: gather the half spectra of the line's two rows, Z = A + iB on the
 // full circle (DC and Nyquist taken as real), C2R, crop, 1/P, mask.
 // ---------------------------------------------------------------------------
-template <typename T, int L>
-__global__ void __launch_bounds__((line_max_threads<T, L>()), (line_min_blocks<T, L>())) k_lx_inv(DemagArgs<T> a) {
+template <typename T, int L, bool UNI = false>
+__device__ __forceinline__ void lx_inv_body(const DemagArgs<T> &a, int bx, int z, int c, unsigned char *smem_raw) {
     using C = cx<T>;
     constexpr int G = Lf<T, L>::G, U = sizeof(T) == 4 ? 8 : 4;  // loads in flight per thread
-    extern __shared__ __align__(16) unsigned char smem_raw[];
     C *region = reinterpret_cast<C *>(smem_raw);
-    const int LP = a.lines_x, TE = a.te_x, RB = 2 * LP, z = blockIdx.y, c = blockIdx.z;
-    const int y0 = blockIdx.x * RB, nx = a.nx, ny = a.ny, nkx = a.nkx;
+    const int LP = a.lines_x, TE = a.te_x, RB = 2 * LP;
+    const int y0 = bx * RB, nx = a.nx, ny = a.ny, nkx = a.nkx;
     {
         const C *s1row = a.s1 + ((long long)c * a.nz + z) * nkx * ny;
         const int qq = threadIdx.x % LP, kstep = blockDim.x / LP, k0 = threadIdx.x / LP, y = y0 + 2 * qq;
@@ -153,7 +160,7 @@ __global__ void __launch_bounds__((line_max_threads<T, L>()), (line_min_blocks<T
     const long long rowa = ((long long)z * ny + ya) * nx, rowb = rowa + nx;
     T *ha = a.hd + (long long)c * a.n + rowa, *hb = ha + nx;
     auto in = [&](int k) -> C { return line[line_slot<T, L>(k)]; };
-    if (!a.mask && !a.ms_map) {
+    if (UNI || (!a.mask && !a.ms_map)) {
         const T sc = a.ms > 0.0 ? nrm : T(0);  // no mask, no Ms map: every cell active when Ms > 0
         auto out = [&](int n, C v) {
             if (n >= nx) return;
@@ -172,17 +179,22 @@ __global__ void __launch_bounds__((line_max_threads<T, L>()), (line_min_blocks<T
     }
 }
 
+template <typename T, int L>
+__global__ void __launch_bounds__((line_max_threads<T, L>()), (line_min_blocks<T, L>())) k_lx_inv(DemagArgs<T> a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    lx_inv_body<T, L>(a, blockIdx.x, blockIdx.y, blockIdx.z, smem_raw);
+}
+
 // ---------------------------------------------------------------------------
 // y forward S1 -> S2 and inverse S2 -> S1 (3-D): line g = (c, z, kx),
 // lines_y groups of G threads per block; no block barrier
 // ---------------------------------------------------------------------------
 template <typename T, int L>
-__global__ void __launch_bounds__((line_max_threads<T, L>()), (line_min_blocks<T, L>())) k_ly_fwd(DemagArgs<T> a) {
+__device__ __forceinline__ void ly_fwd_body(const DemagArgs<T> &a, int bx, unsigned char *smem_raw) {
     using C = cx<T>;
     constexpr int G = Lf<T, L>::G, TE = Lf<T, L>::TILE;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
     const int q = threadIdx.x / G, t = threadIdx.x % G, ny = a.ny;
-    const long long total = 3LL * a.nz * a.nkx, g = (long long)blockIdx.x * a.lines_y + q;
+    const long long total = 3LL * a.nz * a.nkx, g = (long long)bx * a.lines_y + q;
     const bool valid = g < total;
     const C *src = a.s1 + (valid ? g : 0) * ny;
     C *dst = a.s2 + g * L;
@@ -192,12 +204,17 @@ __global__ void __launch_bounds__((line_max_threads<T, L>()), (line_min_blocks<T
 }
 
 template <typename T, int L>
-__global__ void __launch_bounds__((line_max_threads<T, L>()), (line_min_blocks<T, L>())) k_ly_inv(DemagArgs<T> a) {
+__global__ void __launch_bounds__((line_max_threads<T, L>()), (line_min_blocks<T, L>())) k_ly_fwd(DemagArgs<T> a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    ly_fwd_body<T, L>(a, blockIdx.x, smem_raw);
+}
+
+template <typename T, int L>
+__device__ __forceinline__ void ly_inv_body(const DemagArgs<T> &a, int bx, unsigned char *smem_raw) {
     using C = cx<T>;
     constexpr int G = Lf<T, L>::G, TE = Lf<T, L>::TILE;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
     const int q = threadIdx.x / G, t = threadIdx.x % G, ny = a.ny;
-    const long long total = 3LL * a.nz * a.nkx, g = (long long)blockIdx.x * a.lines_y + q;
+    const long long total = 3LL * a.nz * a.nkx, g = (long long)bx * a.lines_y + q;
     const bool valid = g < total;
     const C *src = a.s2 + (valid ? g : 0) * L;
     C *dst = a.s1 + g * ny;
@@ -206,20 +223,25 @@ __global__ void __launch_bounds__((line_max_threads<T, L>()), (line_min_blocks<T
     line_inv<L, true>(t, q, a.twy4, reinterpret_cast<C *>(smem_raw) + q * TE, in, out);
 }
 
+template <typename T, int L>
+__global__ void __launch_bounds__((line_max_threads<T, L>()), (line_min_blocks<T, L>())) k_ly_inv(DemagArgs<T> a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    ly_inv_body<T, L>(a, blockIdx.x, smem_raw);
+}
+
 // ---------------------------------------------------------------------------
 // y convolution (2-D thin film): kb_y kx columns x 3 components per block;
 // forward y, product with N(kx, ky, 0) where the spectrum lies, inverse y
 // ---------------------------------------------------------------------------
 template <typename T, int L>
-__global__ void __launch_bounds__((line_max_threads<T, L>() * 3 / 2)) k_ly_conv(DemagArgs<T> a) {
+__device__ __forceinline__ void ly_conv_body(const DemagArgs<T> &a, int bx, unsigned char *smem_raw) {
     using C = cx<T>;
     constexpr int G = Lf<T, L>::G, TE = Lf<T, L>::TILE;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
     C *region = reinterpret_cast<C *>(smem_raw);
     const int KB = a.kb_y, ny = a.ny, nkx = a.nkx;
     const int q = threadIdx.x / G, t = threadIdx.x % G;
     const int comp = q / KB, kxl = q - comp * KB;
-    const int kx0 = blockIdx.x * KB, kx = kx0 + kxl;
+    const int kx0 = bx * KB, kx = kx0 + kxl;
     const bool valid = kx < nkx;
     C *line = region + q * TE;
     C *g = a.s1 + ((long long)comp * nkx + (valid ? kx : 0)) * ny;
@@ -241,12 +263,78 @@ __global__ void __launch_bounds__((line_max_threads<T, L>() * 3 / 2)) k_ly_conv(
     line_inv<L, true>(t, q, a.twy4, line, in_s, out_g);
 }
 
+template <typename T, int L>
+__global__ void __launch_bounds__((line_max_threads<T, L>() * 3 / 2)) k_ly_conv(DemagArgs<T> a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    ly_conv_body<T, L>(a, blockIdx.x, smem_raw);
+}
+
+// ---------------------------------------------------------------------------
+// Direct z sum of one column (col = kx Ly + ky; the batched kernels) with the table of
+// octant_to_z_direct: the arithmetic of k_zd (zsum.cuh),
+// inputs and table entries read straight from global memory.
+template <typename T, int NZ>
+__device__ __forceinline__ void zd_col(const DemagArgs<T> &a, int col) {
+    using C = cx<T>;
+    const int Ly = a.Ly, KY = a.KY, cols = a.nkx * Ly;
+    if (col >= cols) return;
+    const int cs = NZ * cols, dstr = a.nkx * KY, tstr = NZ * dstr;
+    const int kx = col / Ly, ky = col - kx * Ly;
+    const bool ymir = ky > Ly / 2;
+    const T sy = ymir ? T(-1) : T(1);
+    const T *tp = a.spec + (kx * KY + (ymir ? Ly - ky : ky));
+    C *base = a.s2 + col;
+    C mx[NZ], my[NZ], mz[NZ];
+#pragma unroll
+    for (int z = 0; z < NZ; ++z) {
+        mx[z] = base[z * cols];
+        my[z] = base[cs + z * cols];
+        my[z].x *= sy; my[z].y *= sy;  // xy and yz change sign with ky: so do My and Hy
+        const C v = base[2 * cs + z * cols];
+        mz[z] = mk<T>(v.y, -v.x);  // -i Mz
+    }
+    T tab[6][NZ];
+#pragma unroll
+    for (int e = 0; e < 6; ++e)
+#pragma unroll
+        for (int d = 0; d < NZ; ++d) tab[e][d] = e < 4 || d > 0 ? tp[e * tstr + d * dstr] : T(0);
+    zsum_column<NZ, T>(mx, my, mz, [&](int e, int d) { return tab[e][d]; });
+#pragma unroll
+    for (int z = 0; z < NZ; ++z) {
+        base[z * cols] = mx[z];
+        base[cs + z * cols] = mk<T>(my[z].x * sy, my[z].y * sy);
+        base[2 * cs + z * cols] = mk<T>(-mz[z].y, mz[z].x);  // Hz = i Hz'
+    }
+}
+
 // ---------------------------------------------------------------------------
 // host
 // ---------------------------------------------------------------------------
+// The limit on a kernel's dynamic shared memory is one value per kernel and device, so
+// it is set to the most any grid asks of that kernel: a handle with smaller blocks,
+// created later, must not lower it for the others.
 template <typename K>
-cudaError_t line_smem(K kern, size_t bytes) {
-    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+cudaError_t line_smem(K kern, size_t most) {
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+// most lines per x or y block, and kx columns per thin-film block
+template <typename T, int L> constexpr int line_most() {
+    constexpr int G = Lf<T, L>::G, lp = line_max_threads<T, L>() / G;
+    return lp < 1 ? 1 : G > 32 && lp > 8 ? 8 : lp;
+}
+template <typename T, int L> constexpr int line_most_kb() {
+    constexpr int G = Lf<T, L>::G, least = G >= 32 ? 1 : 32 / G;  // whole warps
+    constexpr int kb = line_max_threads<T, L>() / (3 * G) / least * least;
+    return kb < least ? least : kb;
+}
+
+// Line stride of an x block of lp lines: they start 16 / lp (FP32; 8 / lp in FP64) banks
+// apart, so the threads that split or gather them at neighbouring kx do not collide.
+template <typename T, int L> int line_stride(int lp) {
+    const int banks = sizeof(T) == 4 ? 16 : 8, want = banks / std::min(lp, banks);
+    int te = Lf<T, L>::TILE;
+    while (te % banks != want % banks) ++te;
+    return te;
 }
 
 // Lines per block: 256 threads (4 lines of 1024 points: 64-byte segments of S1 per
@@ -263,20 +351,16 @@ cudaError_t line_setup(LineCfg &c, int Lx, int Ly, bool thin, int ny, int nz, in
     const bool okx = with_line(Lx, [&](auto l) {
         constexpr int L = decltype(l)::value, G = Lf<T, L>::G;
         const int pairs = (ny + 1) / 2, least = std::max(1, 32 / G);
-        int lp = std::max(1, line_max_threads<T, L>() / G);
-        if (G > 32) lp = std::min(lp, 8);
+        int lp = line_most<T, L>();
         while (lp > least && (pairs + lp - 1) / lp * nz * 3 < 2 * kSms) lp /= 2;
-        // the lines of a block start 16 / lp (FP32; 8 / lp in FP64) banks apart, so the
-        // threads that split or gather the lp lines at neighbouring kx do not collide
-        const int banks = sizeof(T) == 4 ? 16 : 8, want = banks / std::min(lp, banks);
-        int te = Lf<T, L>::TILE;
-        while (te % banks != want % banks) ++te;
+        const int te = line_stride<T, L>(lp);
         c.lines_x = lp;
         c.te_x = te;
         c.thr_x = lp * G;
         c.smem_x = (size_t)lp * te * sizeof(cx<T>);
-        err = line_smem(k_lx_fwd<T, L>, c.smem_x);
-        if (err == cudaSuccess) err = line_smem(k_lx_inv<T, L>, c.smem_x);
+        const size_t most = (size_t)line_most<T, L>() * (Lf<T, L>::TILE + 15) * sizeof(cx<T>);
+        err = line_smem(k_lx_fwd<T, L>, most);
+        if (err == cudaSuccess) err = line_smem(k_lx_inv<T, L>, most);
     });
     if (!okx || err != cudaSuccess) return err;
     err = cudaErrorInvalidValue;
@@ -285,23 +369,22 @@ cudaError_t line_setup(LineCfg &c, int Lx, int Ly, bool thin, int ny, int nz, in
         const size_t line = (size_t)Lf<T, L>::TILE * sizeof(cx<T>);
         if (thin) {
             const int least = G >= 32 ? 1 : 32 / G;  // whole warps
-            int kb = std::max(least, line_max_threads<T, L>() / (3 * G) / least * least);
+            int kb = line_most_kb<T, L>();
             while (kb > least && (nkx + kb - 1) / kb < kSms) kb = std::max(least, kb / 2 / least * least);
             c.kb_y = kb;
             c.thr_yc = 3 * kb * G;
             c.smem_yc = 3 * kb * line;
-            err = line_smem(k_ly_conv<T, L>, c.smem_yc);
+            err = line_smem(k_ly_conv<T, L>, 3 * line_most_kb<T, L>() * line);
         } else {
             const int least = std::max(1, 32 / G);
             const long long lines = 3LL * nz * nkx;
-            int lp = std::max(1, line_max_threads<T, L>() / G);
-            if (G > 32) lp = std::min(lp, 8);
+            int lp = line_most<T, L>();
             while (lp > least && (lines + lp - 1) / lp < 4 * kSms) lp /= 2;
             c.lines_y = lp;
             c.thr_y = lp * G;
             c.smem_y = lp * line;
-            err = line_smem(k_ly_fwd<T, L>, c.smem_y);
-            if (err == cudaSuccess) err = line_smem(k_ly_inv<T, L>, c.smem_y);
+            err = line_smem(k_ly_fwd<T, L>, line_most<T, L>() * line);
+            if (err == cudaSuccess) err = line_smem(k_ly_inv<T, L>, line_most<T, L>() * line);
         }
     });
     return err;
