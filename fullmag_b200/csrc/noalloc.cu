@@ -1,9 +1,9 @@
 // noalloc.cu — the demag field for callers that cannot allocate device memory.
 //
 // fullmag_fdm_demag_field_f64_noalloc computes H_demag = -IFFT(N(k) FFT(Ms m))
-// exactly like the stepper's FP64 demag passes (demag_reg.cuh), but it makes
-// no device allocation: the FFT work arrays (two half-spectrum buffers and the
-// twiddle tables) live in g_fft_scratch, a file-scope __device__ array of
+// exactly like the stepper's FP64 demag passes (demag_line.cuh), but it makes
+// no device allocation: the FFT work arrays (two half-spectrum buffers) live in
+// g_fft_scratch, a file-scope __device__ array of
 // kNoAllocScratchBytes (32 MiB).  Every GPU that loads this library holds that
 // array until the process exits.  The caller owns and passes the inputs (m,
 // the Newell octant) and the output (H); the library only launches kernels.
@@ -22,9 +22,11 @@
 #include <mutex>
 #include <type_traits>
 
+#include "demag_line.hpp"
 #include "demag_reg.cuh"
 #include "fullmag_fdm.h"
 #include "fullmag_fdm_ext.h"
+#include "linefft.cuh"
 
 namespace fm {
 namespace {
@@ -35,9 +37,26 @@ constexpr int kMaxDevices = 64;
 // FFT work arrays of the allocation-free entry point (shared by every call).
 static __device__ __align__(256) unsigned char g_fft_scratch[kNoAllocScratchBytes];
 
+// Line-FFT twiddles (linefft.cuh) of every in-plane length this entry point takes,
+// filled with the radix-64 constants when a device is set up: as constants they cost a
+// call nothing (five fill launches per call took 12 of the 62 us of a 128 x 128 x 8
+// field).
+constexpr int kTwLengths[] = {2, 4, 8, 16, 32, 64, 128, 256, 512, 1024};
+constexpr int kTwElems = 4096;  // >= the sum of their line_twiddle_count
+static __device__ double2 g_line_tw[kTwElems];
+int tw_offset(int L) {
+    int o = 0;
+    for (int l : kTwLengths) {
+        if (l == L) return o;
+        o += line_twiddle_count<double>(l);
+    }
+    return -1;
+}
+
 struct DeviceSlot {
     bool ready = false;
     unsigned char *scratch = nullptr;  // device address of g_fft_scratch on that device
+    double2 *tw = nullptr;             // ... and of g_line_tw
 };
 std::mutex g_mu;
 DeviceSlot g_slots[kMaxDevices];
@@ -56,18 +75,20 @@ void put_error(char *buf, uint64_t len, const char *msg) {
 // pageable memory, which may return before the data reach the device, and a
 // caller's non-blocking stream is not ordered after it: the device is
 // synchronised once here, before the first kernel can read the table.
-bool setup_device(int dev, unsigned char **out, char *err, uint64_t errlen) {
+bool setup_device(int dev, unsigned char **out, double2 **tw_out, char *err, uint64_t errlen) {
     std::lock_guard<std::mutex> lock(g_mu);
     DeviceSlot &s = g_slots[dev];
     void *p = nullptr;
+    void *ptw = nullptr;
     cudaError_t e = cudaGetSymbolAddress(&p, g_fft_scratch);
+    if (e == cudaSuccess) e = cudaGetSymbolAddress(&ptw, g_line_tw);
     if (e != cudaSuccess) {
         char m[256];
         std::snprintf(m, sizeof(m), "cudaGetSymbolAddress(g_fft_scratch): %s", cudaGetErrorString(e));
         put_error(err, errlen, m);
         return false;
     }
-    if (!s.ready || s.scratch != p) {
+    if (!s.ready || s.scratch != p || s.tw != ptw) {
         s.ready = false;
         double2 d[64];
         float2 f[64];
@@ -78,6 +99,11 @@ bool setup_device(int dev, unsigned char **out, char *err, uint64_t errlen) {
         }
         e = cudaMemcpyToSymbol(c_tw64d, d, sizeof(d));
         if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_tw64f, f, sizeof(f));
+        for (int L : kTwLengths) {
+            const std::vector<double2> t = line_twiddles<double>(L);
+            if (e == cudaSuccess)
+                e = cudaMemcpyToSymbol(g_line_tw, t.data(), t.size() * sizeof(double2), (size_t)tw_offset(L) * sizeof(double2));
+        }
         if (e == cudaSuccess) e = cudaDeviceSynchronize();
         if (e != cudaSuccess) {
             char m[256];
@@ -86,41 +112,12 @@ bool setup_device(int dev, unsigned char **out, char *err, uint64_t errlen) {
             return false;
         }
         s.scratch = static_cast<unsigned char *>(p);
+        s.tw = static_cast<double2 *>(ptw);
         s.ready = true;
     }
     *out = s.scratch;
+    *tw_out = s.tw;
     return true;
-}
-
-// tw[k] = exp(-2 pi i k / L), computed on the device (no host staging copy);
-// with L2 > 0 the 4-step table of fftreg.cuh (entry k1 L2 + t holds the value
-// of k = k1 t).
-__global__ void k_fill_twiddles(double2 *tw, int L, int L2) {
-    for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < L; idx += gridDim.x * blockDim.x) {
-        const int k = L2 > 0 ? (idx / L2) * (idx % L2) : idx;
-        double sn, cs;
-        sincospi(2.0 * (double)k / (double)L, &sn, &cs);
-        tw[idx] = make_double2(cs, -sn);
-    }
-}
-
-template <int V> using IC = std::integral_constant<int, V>;
-
-template <class F>
-bool split_for(int L, F &&f) {
-    switch (L) {
-        case 2: f(IC<2>{}, IC<1>{}); return true;
-        case 4: f(IC<4>{}, IC<1>{}); return true;
-        case 8: f(IC<8>{}, IC<1>{}); return true;
-        case 16: f(IC<16>{}, IC<1>{}); return true;
-        case 32: f(IC<32>{}, IC<1>{}); return true;
-        case 64: f(IC<8>{}, IC<8>{}); return true;
-        case 128: f(IC<16>{}, IC<8>{}); return true;
-        case 256: f(IC<16>{}, IC<16>{}); return true;
-        case 512: f(IC<32>{}, IC<16>{}); return true;
-        case 1024: f(IC<32>{}, IC<32>{}); return true;
-        default: return false;
-    }
 }
 
 bool pow2(int L) { return L >= 2 && (L & (L - 1)) == 0; }
@@ -153,7 +150,8 @@ extern "C" int fullmag_fdm_demag_field_f64_noalloc(uint32_t nx, uint32_t ny, uin
         return FULLMAG_FDM_ERR_INVALID;
     }
     const int nkx = (int)nx + 1;
-    // scratch layout (complex elements): twx | twy | twz | twxT | twyT | S1 | S2
+    // scratch layout (complex elements): S1 | S2.  The limit also counts 2 Lx + 2 Ly + Lz
+    // elements of tables, so that it does not depend on where those are kept
     const size_t s1 = (size_t)3 * nz * nkx * ny, s2 = thin ? 0 : (size_t)3 * nz * nkx * Ly;
     const size_t elems = (size_t)2 * Lx + 2 * Ly + Lz + s1 + s2 + 16;
     const size_t need = elems * sizeof(C);
@@ -172,22 +170,15 @@ extern "C" int fullmag_fdm_demag_field_f64_noalloc(uint32_t nx, uint32_t ny, uin
         return FULLMAG_FDM_ERR_CUDA;
     }
     unsigned char *base = nullptr;
-    if (!setup_device(dev, &base, error_out, error_out_len)) return FULLMAG_FDM_ERR_CUDA;
+    C *tw = nullptr;
+    if (!setup_device(dev, &base, &tw, error_out, error_out_len)) return FULLMAG_FDM_ERR_CUDA;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // a launch error left by earlier, unrelated work is not this call's: clear
     // it, so that the check after the launches reports only this call's own
     (void)cudaGetLastError();
 
-    C *p = reinterpret_cast<C *>(base);
-    C *twx = p, *twy = twx + Lx, *twz = twy + Ly;
-    C *twxT = twz + Lz, *twyT = twxT + Lx;
-    C *ps1 = twyT + Ly;
+    C *ps1 = reinterpret_cast<C *>(base);
     C *ps2 = ps1 + s1;
-    k_fill_twiddles<<<(Lx + 255) / 256, 256, 0, st>>>(twx, Lx, 0);
-    k_fill_twiddles<<<(Ly + 255) / 256, 256, 0, st>>>(twy, Ly, 0);
-    k_fill_twiddles<<<(Lz + 255) / 256, 256, 0, st>>>(twz, Lz, 0);
-    k_fill_twiddles<<<(Lx + 255) / 256, 256, 0, st>>>(twxT, Lx, l2_for(Lx));
-    k_fill_twiddles<<<(Ly + 255) / 256, 256, 0, st>>>(twyT, Ly, l2_for(Ly));
 
     DemagArgs<double> a{};
     a.nx = nx; a.ny = ny; a.nz = nz;
@@ -195,8 +186,8 @@ extern "C" int fullmag_fdm_demag_field_f64_noalloc(uint32_t nx, uint32_t ny, uin
     a.Lx = Lx; a.Ly = Ly; a.Lz = Lz; a.nkx = nkx;
     a.KZ = thin ? 1 : (int)nz + 1;
     a.KY = (int)ny + 1;
-    a.twx = twx; a.twy = twy; a.twz = twz;
-    a.twxT = twxT; a.twyT = twyT;
+    a.twx4 = tw + tw_offset(Lx);
+    a.twy4 = tw + tw_offset(Ly);
     a.s1 = ps1; a.s2 = thin ? nullptr : ps2;
     a.spec = octant;
     a.m = m;
@@ -206,69 +197,16 @@ extern "C" int fullmag_fdm_demag_field_f64_noalloc(uint32_t nx, uint32_t ny, uin
     a.hd = h;
     a.norm = 1.0 / ((double)Lx * (double)Ly * (double)Lz);
 
-    const size_t sz = sizeof(C);
-    bool ok = true;
-    // x passes: complex lines (row pairs) per block
-    int thr_x = 0;
-    size_t smx = 0, smxi = 0;
-    split_for(Lx, [&](auto l1, auto l2) {
-        constexpr int L1 = decltype(l1)::value, L2 = decltype(l2)::value;
-        constexpr int TE = line_region<L1, L2>();
-        const int unit = L2 >= 32 ? 1 : 32 / L2;
-        int lp = std::max(unit, (128 / L2) / unit * unit);
-        while (lp > unit && (size_t)(lp * TE) * sz > 200 * 1024) lp -= unit;
-        a.lines_x = lp;
-        thr_x = lp * L2;
-        smx = (size_t)(lp * TE) * sz;
-        smxi = smx + (size_t)L1 * L2 * sz;  // the x inverse also holds the twiddle table
-        ok &= cudaFuncSetAttribute(k_xf_r<double, L1, L2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smx) == cudaSuccess;
-        ok &= cudaFuncSetAttribute(k_xi_r<double, L1, L2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smxi) == cudaSuccess;
-    });
-    int thr_y = 0;
-    size_t smy = 0;
-    split_for(Ly, [&](auto l1, auto l2) {
-        constexpr int L1 = decltype(l1)::value, L2 = decltype(l2)::value;
-        if (thin) {
-            constexpr int TE = line_region<L1, L2>();
-            const int unit = L2 >= 32 ? 1 : 32 / L2;
-            int kb = std::max(unit, (192 / (3 * L2)) / unit * unit);
-            while (kb > unit && (size_t)(3 * kb * TE) * sz > 200 * 1024) kb -= unit;
-            a.kb_y = kb;
-            thr_y = 3 * kb * L2;
-            smy = (size_t)(3 * kb * TE) * sz;
-            ok &= cudaFuncSetAttribute(k_yc_r<double, L1, L2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smy) == cudaSuccess;
-        } else {
-            constexpr int TE = tile_elems(L1, L2);
-            const int lpb = std::max(1, 128 / L2);
-            a.lines_y = lpb;
-            thr_y = lpb * L2;
-            smy = (size_t)(lpb * TE) * sz;
-            ok &= cudaFuncSetAttribute(k_yf_r<double, L1, L2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smy) == cudaSuccess;
-            ok &= cudaFuncSetAttribute(k_yi_r<double, L1, L2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smy) == cudaSuccess;
-        }
-    });
-    if (!ok) {
+    LineCfg line;
+    if (line_setup<double>(line, Lx, Ly, thin, (int)ny, (int)nz, nkx) != cudaSuccess) {
         put_error(error_out, error_out_len, "cudaFuncSetAttribute failed");
         return FULLMAG_FDM_ERR_CUDA;
     }
-    const int RB = 2 * a.lines_x;
-    const dim3 gx((ny + RB - 1) / RB, nz, 3);
-    split_for(Lx, [&](auto l1, auto l2) {
-        constexpr int L1 = decltype(l1)::value, L2 = decltype(l2)::value;
-        k_xf_r<double, L1, L2><<<gx, thr_x, smx, st>>>(a);
-    });
+    line_x_fwd<double>(line, a, st);
     if (thin) {
-        split_for(Ly, [&](auto l1, auto l2) {
-            constexpr int L1 = decltype(l1)::value, L2 = decltype(l2)::value;
-            k_yc_r<double, L1, L2><<<(nkx + a.kb_y - 1) / a.kb_y, thr_y, smy, st>>>(a);
-        });
+        line_y_conv<double>(line, a, st);
     } else {
-        const long long lines = 3LL * nz * nkx;
-        const unsigned gy = (unsigned)((lines + a.lines_y - 1) / a.lines_y);
-        split_for(Ly, [&](auto l1, auto l2) {
-            constexpr int L1 = decltype(l1)::value, L2 = decltype(l2)::value;
-            k_yf_r<double, L1, L2><<<gy, thr_y, smy, st>>>(a);
-        });
+        line_y_fwd<double>(line, a, st);
         const int cols = nkx * Ly;
         const int P = Lz > 8 ? 2 : 1;
         const unsigned gz = (unsigned)std::min<long long>(((long long)cols * P + 127) / 128, 148LL * 64);
@@ -279,15 +217,9 @@ extern "C" int fullmag_fdm_demag_field_f64_noalloc(uint32_t nx, uint32_t ny, uin
             case 162: k_zc_r<double, 16, 2><<<gz, 128, 0, st>>>(a); break;
             default: break;
         }
-        split_for(Ly, [&](auto l1, auto l2) {
-            constexpr int L1 = decltype(l1)::value, L2 = decltype(l2)::value;
-            k_yi_r<double, L1, L2><<<gy, thr_y, smy, st>>>(a);
-        });
+        line_y_inv<double>(line, a, st);
     }
-    split_for(Lx, [&](auto l1, auto l2) {
-        constexpr int L1 = decltype(l1)::value, L2 = decltype(l2)::value;
-        k_xi_r<double, L1, L2><<<gx, thr_x, smxi, st>>>(a);
-    });
+    line_x_inv<double>(line, a, st);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         char msg[256];
