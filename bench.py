@@ -575,14 +575,13 @@ def _pow2_at_least(v):
     return p
 
 
-def _batch_length(v, dbl=False):
+def _batch_length(v):
     """The batch's padded in-plane length (batch.cu batch_length): at least 16,
-    the smallest power of two >= v, or in FP32 3 * 2^k in 96..768 when shorter."""
+    the smallest power of two or 3 * 2^k in 96..768 >= v."""
     L = max(16, _pow2_at_least(v))
-    if not dbl:
-        for c in (96, 192, 384, 768):
-            if v <= c < L:
-                L = c
+    for c in (96, 192, 384, 768):
+        if v <= c < L:
+            L = c
     return L
 
 
@@ -597,7 +596,7 @@ def batch_kind_bytes(probs, s=4, zdirect=True):
     for p in probs:
         nx, ny, nz = p["cells"]
         n = nx * ny * nz
-        Lx, Ly, Lz = _batch_length(2 * nx, s == 8), _batch_length(2 * ny, s == 8), _pow2_at_least(2 * nz)
+        Lx, Ly, Lz = _batch_length(2 * nx), _batch_length(2 * ny), _pow2_at_least(2 * nz)
         nkx = Lx // 2 + 1
         s1 = 3 * nz * nkx * ny * cs
         s2 = 3 * nz * nkx * Ly * cs

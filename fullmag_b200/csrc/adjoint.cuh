@@ -20,6 +20,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "pdl.cuh"
 
 namespace fm {
 
@@ -51,6 +52,7 @@ __device__ __forceinline__ void cross3(const double *a, const double *b, double 
 template <typename T>
 __global__ void __launch_bounds__(256) k_adj_start(AdjArgs a, const T *m, const T *k1, const T *k2,
                                                    const double *lam, double *acc, double *gk) {
+    pdl_wait();
     const long long n = a.n;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         double ms_i;
@@ -82,6 +84,7 @@ __global__ void __launch_bounds__(256) k_adj_start(AdjArgs a, const T *m, const 
 template <typename T>
 __global__ void __launch_bounds__(256) k_adj_vjp(AdjArgs a, const T *m, const T *H, const double *g,
                                                  T *lh, double *lloc) {
+    pdl_wait();
     const long long n = a.n;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         double ms_i;
@@ -120,6 +123,7 @@ __global__ void __launch_bounds__(256) k_adj_apply(AdjArgs a, const T *m, const 
                                                    const T *hex, const double *lloc, double *out,
                                                    double *g_ms, double *g_hext, double *g_hac,
                                                    double sin_t) {
+    pdl_wait();
     const long long n = a.n, sxy = (long long)a.nx * a.ny;
     const int nx = a.nx, ny = a.ny, nz = a.nz;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -165,6 +169,7 @@ __global__ void __launch_bounds__(256) k_adj_apply(AdjArgs a, const T *m, const 
 template <typename T>
 __global__ void __launch_bounds__(256) k_adj_pred(AdjArgs a, const T *m, const T *k1, const double *lmp,
                                                   double *acc, double *gk) {
+    pdl_wait();
     const long long n = a.n;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         double ms_i;
@@ -189,6 +194,7 @@ __global__ void __launch_bounds__(256) k_adj_pred(AdjArgs a, const T *m, const T
 // lambda_n = acc + the last stage's field pull-back.
 __global__ void __launch_bounds__(256) k_adj_finish(long long n3, const double *acc, const double *part,
                                                     double *lam) {
+    pdl_wait();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n3; i += (long long)gridDim.x * blockDim.x)
         lam[i] = acc[i] + part[i];
 }

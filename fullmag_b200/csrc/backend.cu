@@ -250,7 +250,7 @@ struct Impl {
                 ProfScope p(b, "demag_z_direct");
                 with_nz(b.nz, [&](auto nzc) {
                     constexpr int NZ = decltype(nzc)::value;
-                    k_zd<T, NZ><<<b.grid_zd, zd_threads<T>(), b.rsm_zd, b.stream>>>(a);
+                    pdl_launch(k_zd<T, NZ>, dim3((unsigned)b.grid_zd), dim3(zd_threads<T>()), b.rsm_zd, b.stream, a);
                 });
             } else if (b.zreg) {
                 ProfScope p(b, "demag_z_conv");
@@ -260,11 +260,11 @@ struct Impl {
                 const int P = (b.Lz > 8) ? 2 : 1;
                 const unsigned gz2 = (unsigned)std::min<long long>((cols * P + 127) / 128, 148LL * 64);
                 switch (b.Lz * 10 + P) {
-                    case 21: k_zc_r<T, 2, 1><<<gz2, 128, 0, b.stream>>>(a); break;
-                    case 41: k_zc_r<T, 4, 1><<<gz2, 128, 0, b.stream>>>(a); break;
-                    case 81: k_zc_r<T, 8, 1><<<gz2, 128, 0, b.stream>>>(a); break;
-                    case 162: k_zc_r<T, 16, 2><<<gz2, 128, 0, b.stream>>>(a); break;
-                    case 322: if constexpr (sizeof(T) == 4) k_zc_r<T, 32, 2><<<gz2, 128, 0, b.stream>>>(a); break;
+                    case 21: pdl_launch(k_zc_r<T, 2, 1>, dim3(gz2), dim3(128), 0, b.stream, a); break;
+                    case 41: pdl_launch(k_zc_r<T, 4, 1>, dim3(gz2), dim3(128), 0, b.stream, a); break;
+                    case 81: pdl_launch(k_zc_r<T, 8, 1>, dim3(gz2), dim3(128), 0, b.stream, a); break;
+                    case 162: pdl_launch(k_zc_r<T, 16, 2>, dim3(gz2), dim3(128), 0, b.stream, a); break;
+                    case 322: if constexpr (sizeof(T) == 4) pdl_launch(k_zc_r<T, 32, 2>, dim3(gz2), dim3(128), 0, b.stream, a); break;
                     default: break;
                 }
             } else {
@@ -314,6 +314,12 @@ struct Impl {
                           env_is("FULLMAG_FDM_STAGE", "cell");
         b.stage_vec = rows16 && simple && !keep && 3ULL * (unsigned long long)b.n < (1ULL << 32);
         b.stage_vec_mk = b.stage_vec && (b.has_mask || b.has_ms_map);
+        // RK stage kernels that also form the next stage state: always with the one-value
+        // kernels (512 x 512 x 8 FP64 RK4 1566 -> 1505 us per step, 256 x 256 x 4 217 -> 208);
+        // with the group kernels, whose registers then allow 16 warps per SM instead of 20,
+        // up to 2^18 cells (128 x 128 FP32 DP45 133 -> 124 us, 256 x 256 x 4 252 -> 249, but
+        // 300 x 180 x 5 masked 479 -> 486 and 1024 x 512 x 16 masked 242 -> 290 us per stage)
+        b.chain = !b.stage_vec || b.n <= (1LL << 18);
         if (!b.stage_plain) return true;
         b.stage_ring = !env_is("FULLMAG_FDM_STAGE", "plain");
         if (!b.stage_ring) return true;
@@ -321,6 +327,8 @@ struct Impl {
         bool ok = true;
         ok &= cuda_ok(b, cudaFuncSetAttribute(k_stage_ring<T, MODE_EVAL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               (int)ring_bytes<T, MODE_EVAL>(thr)), "attr stage ring");
+        ok &= cuda_ok(b, cudaFuncSetAttribute(k_stage_ring<T, MODE_EVAL_NEXT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)ring_bytes<T, MODE_EVAL_NEXT>(thr)), "attr stage ring");
         ok &= cuda_ok(b, cudaFuncSetAttribute(k_stage_ring<T, MODE_HEUN_CORR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               (int)ring_bytes<T, MODE_HEUN_CORR>(thr)), "attr stage ring");
         ok &= cuda_ok(b, cudaFuncSetAttribute(k_stage_ring<T, MODE_ERR_LAST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -482,13 +490,48 @@ struct Impl {
             const dim3 g((b.nx + 31) / 32, (b.ny + kStagePlainBY - 1) / kStagePlainBY,
                          (b.nz + b.stage_zb - 1) / b.stage_zb);
             if (b.stage_ring)
-                k_stage_ring<T, MODE><<<g, dim3(32, kStagePlainBY, 1), ring_bytes<T, MODE>(32 * kStagePlainBY),
-                                        b.stream>>>(s, b.stage_zb);
+                pdl_launch(k_stage_ring<T, MODE>, g, dim3(32, kStagePlainBY, 1), ring_bytes<T, MODE>(32 * kStagePlainBY),
+                           b.stream, s, b.stage_zb);
             else
-                k_stage_plain<T, MODE><<<g, dim3(32, kStagePlainBY, 1), 0, b.stream>>>(s, b.stage_zb);
+                pdl_launch(k_stage_plain<T, MODE>, g, dim3(32, kStagePlainBY, 1), 0, b.stream, s, b.stage_zb);
         } else {
-            k_stage<T, MODE><<<stage_grid(b), dim3(32, 4, 2), 0, b.stream>>>(s);
+            pdl_launch(k_stage<T, MODE>, stage_grid(b), dim3(32, 4, 2), 0, b.stream, s);
         }
+    }
+
+    // k = RHS(m, t) and from it the integrator's next stage state, in the same kernel:
+    // out = normalize(m0 + sum c_j k_j) (combine's form) with kout as the last slope;
+    // out is not m's buffer.  Saves combine's launch and its read of k.
+    static bool eval_combine(Backend &b, const void *m, double t, void *kout, int form, const void *m0,
+                             std::initializer_list<void *> earlier, std::initializer_list<double> cs, double dt,
+                             void *out) {
+        if (!b.chain) {
+            void *ks[5] = {kout, kout, kout, kout, kout};
+            int i = 0;
+            for (void *k : earlier) ks[i++] = k;
+            double c[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+            i = 0;
+            for (double v : cs) c[i++] = v;
+            return eval(b, m, t, kout, false, false) &&
+                   combine(b, form, m0, {ks[0], ks[1], ks[2], ks[3], ks[4]}, {c[0], c[1], c[2], c[3], c[4]}, dt, out);
+        }
+        StageArgs<T> s = stage_args(b, m, t);
+        s.kout = (T *)kout;
+        s.counter = b.counter;
+        s.out = b.d_out;
+        s.cb_m0 = (const T *)m0;
+        int i = 0;
+        for (void *k : earlier) s.cb_k[i++] = (const T *)k;
+        i = 0;
+        for (double c : cs) s.cb_c[i++] = c;
+        s.cb_dt = dt;
+        s.cb_form = form;
+        s.cb_out = (T *)out;
+        {
+            ProfScope p(b, "stage_eval");
+            launch_stage<MODE_EVAL_NEXT>(b, s);
+        }
+        return check_launch(b, "stage_eval");
     }
 
     // k = RHS(m, t); optional observables and diagnostics.
@@ -547,7 +590,7 @@ struct Impl {
                     done = true;
                 }
             }
-            if (!done) k_combine<T><<<grid_cells(b), 256, 0, b.stream>>>(a);
+            if (!done) pdl_launch(k_combine<T>, dim3(grid_cells(b)), dim3(256), 0, b.stream, a);
         }
         return check_launch(b, "combine");
     }
@@ -675,9 +718,10 @@ struct Impl {
             launch_stage<MODE_HEUN_CORR>(b, s);
         }
         if (!check_launch(b, "heun corrector")) return false;
-        // fields, RHS (next k1), the next predictor and diagnostics at the new state
+        // fields, RHS (next k1) and the next predictor at the new state; the diagnostics
+        // only where they are read back (512 x 512 x 8 FP32: 38 us against 47)
         if (!demag(b, b.m, b.hd)) return false;
-        if (!eval(b, b.m, b.time + dt, b.k[0], true, false, b.mstage, dt)) return false;
+        if (!eval(b, b.m, b.time + dt, b.k[0], readback, false, b.mstage, dt)) return false;
         b.pred_valid = true;
         b.pred_dt = dt;
         b.time += dt;
@@ -710,20 +754,23 @@ struct Impl {
         void **k = b.k;
         for (;;) {
             const double t = b.time;
-            if (!combine(b, 0, b.m, {k[0]}, {A21 * dt}, dt, b.mstage)) return false;
-            if (!demag(b, b.mstage, b.hd) || !eval(b, b.mstage, t + 0.2 * dt, k[1], false, false)) return false;
-            if (!combine(b, 1, b.m, {k[0], k[1]}, {A31, A32}, dt, b.mstage)) return false;
-            if (!demag(b, b.mstage, b.hd) || !eval(b, b.mstage, t + 0.3 * dt, k[2], false, false)) return false;
-            if (!combine(b, 2, b.m, {k[0], k[1], k[2]}, {A41, A42, A43}, dt, b.mstage)) return false;
-            if (!demag(b, b.mstage, b.hd) || !eval(b, b.mstage, t + 0.8 * dt, k[3], false, false)) return false;
-            if (!combine(b, 3, b.m, {k[0], k[1], k[2], k[3]}, {A51, A52, A53, A54}, dt, b.mstage)) return false;
-            if (!demag(b, b.mstage, b.hd) || !eval(b, b.mstage, t + 8.0 / 9.0 * dt, k[4], false, false)) return false;
-            if (!combine(b, 4, b.m, {k[0], k[1], k[2], k[3], k[4]}, {A61, A62, A63, A64, A65}, dt, b.mstage)) return false;
-            if (!demag(b, b.mstage, b.hd) || !eval(b, b.mstage, t + dt, k[5], false, false)) return false;
-            // 5th-order solution and k7 = RHS(y5) with the embedded error norm
-            if (!combine(b, 4, b.m, {k[0], k[2], k[3], k[4], k[5]}, {B1, B3, B4, B5, B6}, dt, b.mstage)) return false;
-            if (!demag(b, b.mstage, b.hd)) return false;
-            StageArgs<T> s = stage_args(b, b.mstage, t + dt);
+            // the stage states alternate between two buffers: a stage kernel writes the next
+            // one while its stencil reads its own
+            void *x = b.mstage, *y = b.mstage2;
+            if (!combine(b, 0, b.m, {k[0]}, {A21 * dt}, dt, x)) return false;
+            if (!demag(b, x, b.hd) || !eval_combine(b, x, t + 0.2 * dt, k[1], 1, b.m, {k[0]}, {A31, A32}, dt, y)) return false;
+            if (!demag(b, y, b.hd) ||
+                !eval_combine(b, y, t + 0.3 * dt, k[2], 2, b.m, {k[0], k[1]}, {A41, A42, A43}, dt, x)) return false;
+            if (!demag(b, x, b.hd) ||
+                !eval_combine(b, x, t + 0.8 * dt, k[3], 3, b.m, {k[0], k[1], k[2]}, {A51, A52, A53, A54}, dt, y)) return false;
+            if (!demag(b, y, b.hd) ||
+                !eval_combine(b, y, t + 8.0 / 9.0 * dt, k[4], 4, b.m, {k[0], k[1], k[2], k[3]}, {A61, A62, A63, A64, A65}, dt, x))
+                return false;
+            // k6 and the 5th-order solution, then k7 = RHS(y5) with the embedded error norm
+            if (!demag(b, x, b.hd) ||
+                !eval_combine(b, x, t + dt, k[5], 4, b.m, {k[0], k[2], k[3], k[4]}, {B1, B3, B4, B5, B6}, dt, y)) return false;
+            if (!demag(b, y, b.hd)) return false;
+            StageArgs<T> s = stage_args(b, y, t + dt);
             s.kout = (T *)k[6];
             s.partials = b.partials;
             s.counter = b.counter;
@@ -742,7 +789,7 @@ struct Impl {
             if (!check_launch(b, "dp45 last stage") || !read_stats(b)) return false;
             const double err = std::sqrt(b.h_out[Q_ERR2]);
             if (err <= b.max_error || dt <= b.dt_min) {
-                std::swap(b.m, b.mstage);
+                std::swap(b.m, b.mstage2);
                 b.hd_stale = false;  // the last evaluation was at the accepted state
                 std::swap(k[0], k[6]);  // FSAL: k7 is the next step's k1
                 b.time += dt;
@@ -762,10 +809,11 @@ struct Impl {
     }
 
     // Fields and RHS at the accepted state into k[0] (the next step's k1), with
-    // the step diagnostics; advances the step counter.
-    static bool finish_step(Backend &b, double dt, fullmag_fdm_step_stats *st, bool readback) {
+    // the step diagnostics where they are read back; advances the step counter.
+    static bool finish_step(Backend &b, double dt, fullmag_fdm_step_stats *st, bool readback, void *pred_out = nullptr,
+                            double pred_dt = 0.0) {
         if (!demag(b, b.m, b.hd)) return false;
-        if (!eval(b, b.m, b.time, b.k[0], true, false)) return false;
+        if (!eval(b, b.m, b.time, b.k[0], readback, false, pred_out, pred_dt)) return false;
         b.step_count += 1;
         b.k1_valid = true;
         b.obs_valid = false;
@@ -780,20 +828,24 @@ struct Impl {
     // One classical RK4 step (lib.rs:1253-1297) with the cached k1; stage
     // times t, t + dt/2, t + dt/2, t + dt.
     static bool rk4(Backend &b, double dt, fullmag_fdm_step_stats *st, bool readback) {
-        b.pred_valid = false;  // the stages below use mstage
+        const bool pred = b.pred_valid;  // mstage holds normalize(m + k1 pred_dt)
+        b.pred_valid = false;            // the stages below use mstage
         if (!ensure_k1(b)) return false;
         void **k = b.k;
         const double t = b.time;
-        if (!combine(b, 0, b.m, {k[0]}, {0.5 * dt}, dt, b.mstage)) return false;
-        if (!demag(b, b.mstage, b.hd) || !eval(b, b.mstage, t + 0.5 * dt, k[1], false, false)) return false;
-        if (!combine(b, 0, b.m, {k[1]}, {0.5 * dt}, dt, b.mstage)) return false;
-        if (!demag(b, b.mstage, b.hd) || !eval(b, b.mstage, t + 0.5 * dt, k[2], false, false)) return false;
-        if (!combine(b, 0, b.m, {k[2]}, {dt}, dt, b.mstage)) return false;
-        if (!demag(b, b.mstage, b.hd) || !eval(b, b.mstage, t + dt, k[3], false, false)) return false;
-        // m <- normalize(m0 + ((k1 + 2 k2) + (2 k3 + k4)) dt/6), in place
-        if (!combine(b, 3, b.m, {k[0], k[1], k[2], k[3]}, {1.0, 2.0, 2.0, 1.0}, dt / 6.0, b.m)) return false;
+        void *x = b.mstage, *y = b.mstage2;
+        if (!(pred && b.pred_dt == 0.5 * dt) && !combine(b, 0, b.m, {k[0]}, {0.5 * dt}, dt, x)) return false;
+        if (!demag(b, x, b.hd) || !eval_combine(b, x, t + 0.5 * dt, k[1], 0, b.m, {}, {0.5 * dt}, dt, y)) return false;
+        if (!demag(b, y, b.hd) || !eval_combine(b, y, t + 0.5 * dt, k[2], 0, b.m, {}, {dt}, dt, x)) return false;
+        // k4, then m <- normalize(m0 + ((k1 + 2 k2) + (2 k3 + k4)) dt/6), in place
+        if (!demag(b, x, b.hd) ||
+            !eval_combine(b, x, t + dt, k[3], 3, b.m, {k[0], k[1], k[2]}, {1.0, 2.0, 2.0, 1.0}, dt / 6.0, b.m)) return false;
         b.time += dt;
-        return finish_step(b, dt, st, readback);
+        // the next step's first stage state too, for the same dt
+        if (!finish_step(b, dt, st, readback, b.mstage, 0.5 * dt)) return false;
+        b.pred_valid = true;
+        b.pred_dt = 0.5 * dt;
+        return true;
     }
 
     // One accepted Bogacki-Shampine 2(3) step (lib.rs:1332-1407).  The
@@ -807,12 +859,12 @@ struct Impl {
         void **k = b.k;
         for (;;) {
             const double t = b.time;
-            if (!combine(b, 0, b.m, {k[0]}, {0.5 * dt}, dt, b.mstage)) return false;
-            if (!demag(b, b.mstage, b.hd) || !eval(b, b.mstage, t + 0.5 * dt, k[1], false, false)) return false;
-            if (!combine(b, 0, b.m, {k[1]}, {0.75 * dt}, dt, b.mstage)) return false;
-            if (!demag(b, b.mstage, b.hd) || !eval(b, b.mstage, t + 0.75 * dt, k[2], false, false)) return false;
-            if (!combine(b, 2, b.m, {k[0], k[1], k[2]}, {2.0 / 9.0, 1.0 / 3.0, 4.0 / 9.0}, dt, b.mstage)) return false;
-            if (!demag(b, b.mstage, b.hd)) return false;
+            void *x = b.mstage, *y = b.mstage2;
+            if (!combine(b, 0, b.m, {k[0]}, {0.5 * dt}, dt, x)) return false;
+            if (!demag(b, x, b.hd) || !eval_combine(b, x, t + 0.5 * dt, k[1], 0, b.m, {}, {0.75 * dt}, dt, y)) return false;
+            if (!demag(b, y, b.hd) ||
+                !eval_combine(b, y, t + 0.75 * dt, k[2], 2, b.m, {k[0], k[1]}, {2.0 / 9.0, 1.0 / 3.0, 4.0 / 9.0}, dt, x)) return false;
+            if (!demag(b, x, b.hd)) return false;
             StageArgs<T> s = stage_args(b, b.mstage, t + dt);
             s.kout = (T *)k[3];
             s.partials = b.partials;
@@ -982,18 +1034,18 @@ struct Impl {
         const double t2 = tn + dt;
         if (!demag(b, p.mp, b.hd) || !eval_fields(b, p.mp, t2, p.k2, p.hex2, p.H2)) return false;
         // corrector normalisation, then stage 2 (at m_p, t + dt)
-        k_adj_start<T><<<g, 256, 0, b.stream>>>(a, mn, p.k1, p.k2, p.lam, p.acc, p.gk);
-        k_adj_vjp<T><<<g, 256, 0, b.stream>>>(a, p.mp, p.H2, p.gk, p.lh, p.lloc);
+        pdl_launch(k_adj_start<T>, dim3(g), dim3(256), 0, b.stream, a, mn, p.k1, p.k2, p.lam, p.acc, p.gk);
+        pdl_launch(k_adj_vjp<T>, dim3(g), dim3(256), 0, b.stream, a, p.mp, p.H2, p.gk, p.lh, p.lloc);
         if (!demag(b, p.lh, p.hadj, true)) return false;
-        k_adj_apply<T><<<g, 256, 0, b.stream>>>(a, p.mp, p.lh, p.hadj, p.hex2, p.lloc, p.part, p.gms,
+        pdl_launch(k_adj_apply<T>, dim3(g), dim3(256), 0, b.stream, a, p.mp, p.lh, p.hadj, p.hex2, p.lloc, p.part, p.gms,
                                                 p.ghext, p.ghac, omega != 0.0 ? std::sin(t2 * omega) : 0.0);
         // predictor normalisation, then stage 1 (at m_n, t)
-        k_adj_pred<T><<<g, 256, 0, b.stream>>>(a, mn, p.k1, p.part, p.acc, p.gk);
-        k_adj_vjp<T><<<g, 256, 0, b.stream>>>(a, mn, p.H1, p.gk, p.lh, p.lloc);
+        pdl_launch(k_adj_pred<T>, dim3(g), dim3(256), 0, b.stream, a, mn, p.k1, p.part, p.acc, p.gk);
+        pdl_launch(k_adj_vjp<T>, dim3(g), dim3(256), 0, b.stream, a, mn, p.H1, p.gk, p.lh, p.lloc);
         if (!demag(b, p.lh, p.hadj, true)) return false;
-        k_adj_apply<T><<<g, 256, 0, b.stream>>>(a, mn, p.lh, p.hadj, p.hex1, p.lloc, p.part, p.gms,
+        pdl_launch(k_adj_apply<T>, dim3(g), dim3(256), 0, b.stream, a, mn, p.lh, p.hadj, p.hex1, p.lloc, p.part, p.gms,
                                                 p.ghext, p.ghac, omega != 0.0 ? std::sin(tn * omega) : 0.0);
-        k_adj_finish<<<g, 256, 0, b.stream>>>(3LL * b.n, p.acc, p.part, p.lam);
+        pdl_launch(k_adj_finish, dim3(g), dim3(256), 0, b.stream, 3LL * b.n, p.acc, p.part, p.lam);
         return check_launch(b, "adjoint step");
     }
 
@@ -1154,6 +1206,7 @@ bool backend_alloc(Backend &b) {
                                                                    : 2;
     items.push_back({&b.m, vec});
     items.push_back({&b.mstage, vec});
+    if (nk == 4 || nk == 7) items.push_back({&b.mstage2, vec});  // RK4, RK23, DP45
     items.push_back({&b.hd, vec});
     items.push_back({&b.hex, vec});
     items.push_back({&b.heff, vec});

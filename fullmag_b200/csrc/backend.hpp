@@ -141,6 +141,8 @@ struct Backend {
     bool info_valid = false;
     std::string last_error;
     std::string err_buf;
+    void *mstage2 = nullptr;  // the other stage state of the RK integrators
+    bool chain = false;       // RK stage kernels also form the next stage state (eval_combine)
 };
 
 }  // namespace fm

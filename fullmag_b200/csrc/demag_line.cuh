@@ -8,6 +8,7 @@
 #include "demag.cuh"
 #include "demag_line.hpp"
 #include "linefft.cuh"
+#include "pdl.cuh"
 #include "zsum.cuh"
 
 namespace fm {
@@ -15,11 +16,17 @@ namespace fm {
 // Most threads of a block: 256, or one 4-line block of 2048 points (512)
 template <typename T, int L> __host__ __device__ constexpr int line_max_threads() { return Lf<T, L>::G >= 128 ? 512 : 256; }
 // Blocks per SM the register budget is cut for: 32 warps per SM in FP32 (64
-// registers; 24 values per thread: 80, 32: 128), 16 in FP64
+// registers; 24 values per thread: 80, 32: 128), 16 in FP64 (24 with 8 to 12 values)
 template <typename T, int L> __host__ __device__ constexpr int line_min_blocks() {
     constexpr int V = L / Lf<T, L>::G;
-    constexpr int warps = sizeof(T) == 4 ? (V > 24 ? 16 : V > 16 ? 24 : 32) : (V > 16 ? 8 : 16);
+    constexpr int warps = sizeof(T) == 4 ? (V > 24 ? 16 : V > 16 ? 24 : 32) : (V > 16 ? 8 : V > 12 ? 16 : 24);
     return warps * 32 / line_max_threads<T, L>() > 0 ? warps * 32 / line_max_threads<T, L>() : 1;
+}
+
+// The twiddles on their way to L1 while the kernel before still runs, then its results.
+template <typename T, int L> __device__ __forceinline__ void line_begin(const cx<T> *tw) {
+    if constexpr (Lf<T, L>::NP > 1) warm_lines(tw, Lf<T, L>::TW * (int)sizeof(cx<T>));
+    pdl_wait();
 }
 
 // ---------------------------------------------------------------------------
@@ -98,6 +105,7 @@ __device__ __forceinline__ void lx_fwd_body(const DemagArgs<T> &a, int bx, int z
 template <typename T, int L>
 __global__ void __launch_bounds__((line_max_threads<T, L>()), (line_min_blocks<T, L>())) k_lx_fwd(DemagArgs<T> a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    line_begin<T, L>(a.twx4);
     lx_fwd_body<T, L>(a, blockIdx.x, blockIdx.y, blockIdx.z, smem_raw);
 }
 
@@ -112,6 +120,24 @@ __device__ __forceinline__ void lx_inv_body(const DemagArgs<T> &a, int bx, int z
     C *region = reinterpret_cast<C *>(smem_raw);
     const int LP = a.lines_x, TE = a.te_x, RB = 2 * LP;
     const int y0 = bx * RB, nx = a.nx, ny = a.ny, nkx = a.nkx;
+    const int q = threadIdx.x / G, t = threadIdx.x % G;
+    const int ya = y0 + 2 * q, yb = ya + 1;
+    const bool oka = ya < ny, okb = yb < ny;
+    const long long rowa = ((long long)z * ny + ya) * nx, rowb = rowa + nx;
+    // activity of the cells this thread will write, loaded before the gather so that the
+    // mask's latency is not paid after the transform
+    constexpr int NB = line_out_count<T, L, true>();
+    static_assert(NB <= 32, "activity bits");
+    unsigned acta = 0u, actb = 0u;
+    if (!UNI && (a.mask || a.ms_map)) {
+#pragma unroll
+        for (int i = 0; i < NB; ++i) {
+            const int n = line_out_index<T, L, true>(t, i);
+            double msi;
+            if (n < nx && oka && cell_active(a, rowa + n, msi)) acta |= 1u << i;
+            if (n < nx && okb && cell_active(a, rowb + n, msi)) actb |= 1u << i;
+        }
+    }
     {
         const C *s1row = a.s1 + ((long long)c * a.nz + z) * nkx * ny;
         const int qq = threadIdx.x % LP, kstep = blockDim.x / LP, k0 = threadIdx.x / LP, y = y0 + 2 * qq;
@@ -152,12 +178,8 @@ __device__ __forceinline__ void lx_inv_body(const DemagArgs<T> &a, int bx, int z
         }
     }
     __syncthreads();
-    const int q = threadIdx.x / G, t = threadIdx.x % G;
-    const int ya = y0 + 2 * q, yb = ya + 1;
-    const bool oka = ya < ny, okb = yb < ny;
     C *line = region + q * TE;
     const T nrm = (T)a.norm;
-    const long long rowa = ((long long)z * ny + ya) * nx, rowb = rowa + nx;
     T *ha = a.hd + (long long)c * a.n + rowa, *hb = ha + nx;
     auto in = [&](int k) -> C { return line[line_slot<T, L>(k)]; };
     if (UNI || (!a.mask && !a.ms_map)) {
@@ -169,11 +191,10 @@ __device__ __forceinline__ void lx_inv_body(const DemagArgs<T> &a, int bx, int z
         };
         line_inv<L, true>(t, q, a.twx4, line, in, out);
     } else {
-        auto out = [&](int n, C v) {
+        auto out = [&](int n, int i, C v) {
             if (n >= nx) return;
-            double msi;
-            if (oka) ha[n] = cell_active(a, rowa + n, msi) ? v.x * nrm : T(0);
-            if (okb) hb[n] = cell_active(a, rowb + n, msi) ? v.y * nrm : T(0);
+            if (oka) ha[n] = (acta >> i) & 1u ? v.x * nrm : T(0);
+            if (okb) hb[n] = (actb >> i) & 1u ? v.y * nrm : T(0);
         };
         line_inv<L, true>(t, q, a.twx4, line, in, out);
     }
@@ -182,6 +203,7 @@ __device__ __forceinline__ void lx_inv_body(const DemagArgs<T> &a, int bx, int z
 template <typename T, int L>
 __global__ void __launch_bounds__((line_max_threads<T, L>()), (line_min_blocks<T, L>())) k_lx_inv(DemagArgs<T> a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    line_begin<T, L>(a.twx4);
     lx_inv_body<T, L>(a, blockIdx.x, blockIdx.y, blockIdx.z, smem_raw);
 }
 
@@ -206,6 +228,7 @@ __device__ __forceinline__ void ly_fwd_body(const DemagArgs<T> &a, int bx, unsig
 template <typename T, int L>
 __global__ void __launch_bounds__((line_max_threads<T, L>()), (line_min_blocks<T, L>())) k_ly_fwd(DemagArgs<T> a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    line_begin<T, L>(a.twy4);
     ly_fwd_body<T, L>(a, blockIdx.x, smem_raw);
 }
 
@@ -226,6 +249,7 @@ __device__ __forceinline__ void ly_inv_body(const DemagArgs<T> &a, int bx, unsig
 template <typename T, int L>
 __global__ void __launch_bounds__((line_max_threads<T, L>()), (line_min_blocks<T, L>())) k_ly_inv(DemagArgs<T> a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    line_begin<T, L>(a.twy4);
     ly_inv_body<T, L>(a, blockIdx.x, smem_raw);
 }
 
@@ -254,8 +278,17 @@ __device__ __forceinline__ void ly_conv_body(const DemagArgs<T> &a, int bx, unsi
         if (kx0 + kl >= nkx) continue;
         C *lx = region + kl * TE + s, *ly = lx + KB * TE, *lz = ly + KB * TE;
         C mx = *lx, my = *ly, mz = *lz;
-        tensor_apply(a, kx0 + kl, ky, 0, mx, my, mz);
-        *lx = mx; *ly = my; *lz = mz;
+        // a film's xz and yz are zero (odd in z)
+        const bool mir = ky > L / 2;
+        const T *sp = a.spec + (long long)(kx0 + kl) * a.KY + (mir ? L - ky : ky);
+        const long long plane = (long long)nkx * a.KY;
+        const T nxx = sp[0], nyy = sp[plane], nzz = sp[2 * plane], nxy = mir ? -sp[3 * plane] : sp[3 * plane];
+        lx->x = -(nxx * mx.x + nxy * my.x);
+        lx->y = -(nxx * mx.y + nxy * my.y);
+        ly->x = -(nxy * mx.x + nyy * my.x);
+        ly->y = -(nxy * mx.y + nyy * my.y);
+        lz->x = -(nzz * mz.x);
+        lz->y = -(nzz * mz.y);
     }
     __syncthreads();
     auto in_s = [&](int k) -> C { return line[line_slot<T, L>(k)]; };
@@ -266,6 +299,11 @@ __device__ __forceinline__ void ly_conv_body(const DemagArgs<T> &a, int bx, unsi
 template <typename T, int L>
 __global__ void __launch_bounds__((line_max_threads<T, L>() * 3 / 2)) k_ly_conv(DemagArgs<T> a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    // the block's columns of the tensor (xx, yy, zz, xy)
+    const int kx0 = blockIdx.x * a.kb_y, kb = min(a.kb_y, a.nkx - kx0);
+    for (int e = 0; e < 4; ++e)
+        warm_lines(a.spec + ((long long)e * a.nkx + kx0) * a.KY, kb * a.KY * (int)sizeof(T));
+    line_begin<T, L>(a.twy4);
     ly_conv_body<T, L>(a, blockIdx.x, smem_raw);
 }
 
@@ -390,12 +428,18 @@ cudaError_t line_setup(LineCfg &c, int Lx, int Ly, bool thin, int ny, int nz, in
     return err;
 }
 
+template <typename K, typename T>
+void line_launch(const LineCfg &c, K kern, dim3 g, int threads, size_t smem, cudaStream_t st, const DemagArgs<T> &a) {
+    if (c.pdl) pdl_launch(kern, g, dim3((unsigned)threads), smem, st, a);
+    else kern<<<g, threads, smem, st>>>(a);
+}
+
 template <typename T>
 void line_x_fwd(const LineCfg &c, DemagArgs<T> a, cudaStream_t st) {
     a.lines_x = c.lines_x;
     a.te_x = c.te_x;
     const dim3 g((a.ny + 2 * c.lines_x - 1) / (2 * c.lines_x), a.nz, 3);
-    with_line(c.Lx, [&](auto l) { k_lx_fwd<T, decltype(l)::value><<<g, c.thr_x, c.smem_x, st>>>(a); });
+    with_line(c.Lx, [&](auto l) { line_launch(c, k_lx_fwd<T, decltype(l)::value>, g, c.thr_x, c.smem_x, st, a); });
 }
 
 template <typename T>
@@ -403,28 +447,28 @@ void line_x_inv(const LineCfg &c, DemagArgs<T> a, cudaStream_t st) {
     a.lines_x = c.lines_x;
     a.te_x = c.te_x;
     const dim3 g((a.ny + 2 * c.lines_x - 1) / (2 * c.lines_x), a.nz, 3);
-    with_line(c.Lx, [&](auto l) { k_lx_inv<T, decltype(l)::value><<<g, c.thr_x, c.smem_x, st>>>(a); });
+    with_line(c.Lx, [&](auto l) { line_launch(c, k_lx_inv<T, decltype(l)::value>, g, c.thr_x, c.smem_x, st, a); });
 }
 
 template <typename T>
 void line_y_fwd(const LineCfg &c, DemagArgs<T> a, cudaStream_t st) {
     a.lines_y = c.lines_y;
     const unsigned g = (unsigned)((3LL * a.nz * a.nkx + c.lines_y - 1) / c.lines_y);
-    with_line(c.Ly, [&](auto l) { k_ly_fwd<T, decltype(l)::value><<<g, c.thr_y, c.smem_y, st>>>(a); });
+    with_line(c.Ly, [&](auto l) { line_launch(c, k_ly_fwd<T, decltype(l)::value>, g, c.thr_y, c.smem_y, st, a); });
 }
 
 template <typename T>
 void line_y_inv(const LineCfg &c, DemagArgs<T> a, cudaStream_t st) {
     a.lines_y = c.lines_y;
     const unsigned g = (unsigned)((3LL * a.nz * a.nkx + c.lines_y - 1) / c.lines_y);
-    with_line(c.Ly, [&](auto l) { k_ly_inv<T, decltype(l)::value><<<g, c.thr_y, c.smem_y, st>>>(a); });
+    with_line(c.Ly, [&](auto l) { line_launch(c, k_ly_inv<T, decltype(l)::value>, g, c.thr_y, c.smem_y, st, a); });
 }
 
 template <typename T>
 void line_y_conv(const LineCfg &c, DemagArgs<T> a, cudaStream_t st) {
     a.kb_y = c.kb_y;
     const unsigned g = (unsigned)((a.nkx + c.kb_y - 1) / c.kb_y);
-    with_line(c.Ly, [&](auto l) { k_ly_conv<T, decltype(l)::value><<<g, c.thr_yc, c.smem_yc, st>>>(a); });
+    with_line(c.Ly, [&](auto l) { line_launch(c, k_ly_conv<T, decltype(l)::value>, g, c.thr_yc, c.smem_yc, st, a); });
 }
 
 #define FM_LINE_INSTANCES(T)                                                                     \

@@ -12,6 +12,7 @@ namespace fm {
 struct LineCfg {
     int Lx = 0, Ly = 0;
     bool thin = false;
+    bool pdl = true;                         // programmatic dependent launches (pdl.cuh)
     int lines_x = 0, te_x = 0, thr_x = 0;    // x passes: row pairs per block, line stride
     size_t smem_x = 0;
     int lines_y = 0, thr_y = 0;              // y passes: lines per block

@@ -1,16 +1,12 @@
-// demag_reg.cuh — register-FFT versions of the five demag passes.
-//
-// Same data flow and buffers as demag.cuh (S1 [c][z][kx][y], S2 [c][z][kx][ky],
-// real octant spectra), but every line FFT is fft4step (fftreg.cuh): one
-// shared-memory round trip per line instead of one per radix-4 stage, no
-// integer division in the butterflies, compile-time twiddles inside each
-// thread.  Used whenever all padded lengths are powers of two within the
-// register limits; other lengths use demag.cuh.
+// demag_reg.cuh — the z passes of the demag convolution in registers: direct sums
+// (k_zd) and the z FFT with the tensor product (k_zc_r), on S2 [c][z][kx][ky] of the
+// line-FFT passes (demag_line.cuh); and the line strides of the opt-in row pass.
 #pragma once
 
 #include "cpasync.cuh"
 #include "demag.cuh"
 #include "fftreg.cuh"
+#include "pdl.cuh"
 #include "zsum.cuh"
 
 namespace fm {
@@ -30,434 +26,6 @@ template <int L1, int L2> __host__ __device__ constexpr int line_region() {
 template <typename T, int L1, int L2> __host__ __device__ constexpr int pair_stride() {
     return L2 == 32 ? line_region<L1, L2>() + (sizeof(T) == 8 ? 1 : 3) : line_region<L1, L2>();
 }
-// the pipelined x forward: padded in FP32 only (measured at 1024-point lines:
-// FP32 28.9 -> 26.9 us, FP64 57.5 -> 65.6 us with the pad)
-template <typename T, int L1, int L2> __host__ __device__ constexpr int xf_stride() {
-    return sizeof(T) == 4 ? pair_stride<T, L1, L2>() : line_region<L1, L2>();
-}
-
-// ---------------------------------------------------------------------------
-// x forward: pack Ms*m (two rows per complex line), R2C, transposed store.
-// block = lines_x line groups of L2 threads; grid (ceil(ny / 2 lines_x), nz, 3)
-// ---------------------------------------------------------------------------
-// Block body (bx, z, c); also run per work item by the batched kernels
-// (batch.cuh).  PAD: the padded length may exceed 2 nx (batch), so inputs
-// j >= nx are zero; otherwise Lx = 2 nx and the half-input pruning covers them.
-template <typename T, int L1, int L2, bool PAD = false>
-__device__ __forceinline__ void xf_body(const DemagArgs<T> &a, int bx, int z, int c, unsigned char *smem_raw) {
-    using C = cx<T>;
-    constexpr int L = L1 * L2, TE = line_region<L1, L2>();
-    const C *tw = a.twxT;
-    C *region = reinterpret_cast<C *>(smem_raw);
-    const int LP = a.lines_x, RB = 2 * LP;
-    const int y0 = bx * RB;
-    const int q = threadIdx.x / L2, t = threadIdx.x - q * L2;
-    const T *mc = a.m + (long long)c * a.n;
-    const int ya = y0 + 2 * q, yb = ya + 1, nx = a.nx, ny = a.ny;
-    const long long rowa = ((long long)z * ny + ya) * nx, rowb = rowa + nx;
-    C *line = region + q * TE;
-    // M = Ms m in the storage precision (Ms of the uniform material is exact in FP32)
-    const T msT = a.unit_source ? T(1) : (T)a.ms;
-    auto in = [&](int j) -> C {
-        C v = mk<T>(0, 0);
-        if (PAD && j >= nx) return v;  // zero padding beyond the row (Lx > 2 nx)
-        if (!a.mask && !a.ms_map && !a.vf) {
-            if (ya < ny) v.x = mc[rowa + j] * msT;
-            if (yb < ny) v.y = mc[rowb + j] * msT;
-        } else {
-            if (ya < ny) v.x = demag_source(a, rowa + j, mc[rowa + j]);
-            if (yb < ny) v.y = demag_source(a, rowb + j, mc[rowb + j]);
-        }
-        return v;
-    };
-    auto out = [&](int k, C v) { line[k] = v; };
-    if (!PAD && a.mask && !a.ms_map && !a.vf && !a.unit_source && nx % 16 == 0) {
-        // masked rows: each line group first copies its two rows of m and of the
-        // mask into its own region with 16-byte loads (many in flight), then the
-        // transform reads them from there; per-element global loads under the
-        // mask test stalled on memory latency (issue active 9 % at 2048-point lines)
-        // 8-byte chunks: a line region starts on 8 bytes (its stride is odd in FP32)
-        T *rm = reinterpret_cast<T *>(line);                                 // m rows: reals [0, 2 nx)
-        unsigned char *rk = reinterpret_cast<unsigned char *>(rm + 2 * nx);  // mask rows: bytes [0, 2 nx)
-        constexpr int PT = 8 / (int)sizeof(T);
-        const int cm = 2 * nx / PT, ck = 2 * nx / 8;
-        for (int u = t; u < cm + ck; u += L2) {
-            if (u < cm) {
-                const int e = u * PT, r = e >= nx, x = e - r * nx, yy = r ? yb : ya;
-                uint2 v = make_uint2(0u, 0u);
-                if (yy < ny) v = *reinterpret_cast<const uint2 *>(mc + (r ? rowb : rowa) + x);
-                *reinterpret_cast<uint2 *>(rm + e) = v;
-            } else {
-                const int e = (u - cm) * 8, r = e >= nx, x = e - r * nx, yy = r ? yb : ya;
-                uint2 v = make_uint2(0u, 0u);
-                if (yy < ny) v = *reinterpret_cast<const uint2 *>(a.mask + (r ? rowb : rowa) + x);
-                *reinterpret_cast<uint2 *>(rk + e) = v;
-            }
-        }
-        __syncthreads();
-        // M = Ms m on active cells, the product as demag_source forms it
-        auto in_s = [&](int j) -> C {
-            C v = mk<T>(0, 0);
-            if (rk[j]) v.x = (T)((double)rm[j] * a.ms);
-            if (rk[nx + j]) v.y = (T)((double)rm[nx + j] * a.ms);
-            return v;
-        };
-        fft4step<L1, L2, false, true, true, true>(t, tw, line, in_s, out);
-    } else {
-        fft4step<L1, L2, false, false, true, true>(t, tw, line, in, out);
-    }
-    __syncthreads();
-    const int nkx = a.nkx;
-    C *s1row = a.s1 + ((long long)c * a.nz + z) * nkx * ny;
-    auto emit = [&](int k, int r) {
-        const int y = y0 + r;
-        if (y >= ny) return;
-        const C *ln = region + (r >> 1) * TE;
-        const C zk = ln[k];
-        const C zm = ln[k == 0 ? 0 : L - k];
-        C o;
-        if ((r & 1) == 0) { o.x = T(0.5) * (zk.x + zm.x); o.y = T(0.5) * (zk.y - zm.y); }
-        else { o.x = T(0.5) * (zk.y + zm.y); o.y = T(-0.5) * (zk.x - zm.x); }
-        s1row[(long long)k * ny + y] = o;
-    };
-    if (ny % 2 == 0 && blockDim.x % LP == 0) {
-        // a thread writes both rows of its line pair at one kx (adjacent in S1,
-        // one 16-byte store in FP32): Z[k] and Z[L - k] are read once
-        const int qq = threadIdx.x % LP, kstep = blockDim.x / LP, ya2 = y0 + 2 * qq;
-        if (ya2 < ny) {  // ny even: ya2 + 1 < ny as well
-            const C *ln = region + qq * TE;
-            for (int k = threadIdx.x / LP; k < nkx; k += kstep) {
-                const C zk = ln[k];
-                const C zm = ln[k == 0 ? 0 : L - k];
-                C o0, o1;
-                o0.x = T(0.5) * (zk.x + zm.x); o0.y = T(0.5) * (zk.y - zm.y);
-                o1.x = T(0.5) * (zk.y + zm.y); o1.y = T(-0.5) * (zk.x - zm.x);
-                C *d = s1row + (long long)k * ny + ya2;
-                if constexpr (sizeof(C) == 8) *reinterpret_cast<float4 *>(d) = make_float4(o0.x, o0.y, o1.x, o1.y);
-                else { d[0] = o0; d[1] = o1; }
-            }
-        }
-    } else if (blockDim.x % RB == 0) {
-        // each thread keeps its row; k advances by blockDim / RB (no division in the loop)
-        const int r = threadIdx.x % RB, kstep = blockDim.x / RB;
-        for (int k = threadIdx.x / RB; k < nkx; k += kstep) emit(k, r);
-    } else {
-        for (int u = threadIdx.x; u < nkx * RB; u += blockDim.x) emit(u / RB, u % RB);
-    }
-}
-
-template <typename T, int L1, int L2>
-__global__ void __launch_bounds__(256) k_xf_r(DemagArgs<T> a) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    xf_body<T, L1, L2>(a, blockIdx.x, blockIdx.y, blockIdx.z, smem_raw);
-}
-
-// ---------------------------------------------------------------------------
-// x forward, uniform material (no mask, Ms map or volume fraction; Lx = 2 nx,
-// rows of 16-byte multiples): persistent blocks walk the groups g = (c, z,
-// y-block) of RB = 2 lines_x rows.  The RB rows of a group are one contiguous
-// chunk of m; the next group's chunk is copied into shared memory with 16-byte
-// cp.async while the current group is transformed (double buffer, one commit
-// group per chunk), so the row loads no longer stall the FFT.  The transform
-// and the transposed store are those of xf_body.
-// Shared memory: lines_x line regions (xf_stride complex each), 2 x RB nx reals, then
-// the Lx twiddles of fft4step (2 x RB nx reals keep them 16-byte aligned).
-// ---------------------------------------------------------------------------
-
-template <int L1, int L2, typename T>
-__host__ __device__ constexpr size_t xpipe_region_bytes(int lines) {
-    return ((size_t)lines * xf_stride<T, L1, L2>() * 2 * sizeof(T) + 15) / 16 * 16;
-}
-
-template <typename T, int L1, int L2>
-__global__ void __launch_bounds__(256) k_xf_pipe(DemagArgs<T> a, int ngroups) {
-    using C = cx<T>;
-    constexpr int L = L1 * L2, TE = xf_stride<T, L1, L2>();
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int LP = a.lines_x, RB = 2 * LP, nx = a.nx, ny = a.ny, nz = a.nz, nkx = a.nkx;
-    const int nyb = (ny + RB - 1) / RB;
-    C *region = reinterpret_cast<C *>(smem_raw);
-    T *stage = reinterpret_cast<T *>(smem_raw + xpipe_region_bytes<L1, L2, T>(LP));
-    const size_t stage_elems = (size_t)RB * nx;
-    // the 4-step twiddle table, copied once per (persistent) block
-    C *tws = reinterpret_cast<C *>(stage + 2 * stage_elems);
-    for (int k = threadIdx.x; k < L; k += blockDim.x) tws[k] = a.twxT[k];
-    constexpr int PER = 16 / (int)sizeof(T);  // elements per 16-byte copy
-    auto issue = [&](int g, int buf) {
-        const int yb = g % nyb, cz = g / nyb, z = cz % nz, c = cz / nz;
-        const int y0 = yb * RB, rows = min(RB, ny - y0);
-        const T *src = a.m + (long long)c * a.n + ((long long)z * ny + y0) * nx;
-        T *dst = stage + buf * stage_elems;
-        const int chunks = rows * nx / PER;
-        for (int u = threadIdx.x; u < chunks; u += blockDim.x) cp_async16(dst + u * PER, src + u * PER);
-        cp_async_commit();
-    };
-    const int q = threadIdx.x / L2, t = threadIdx.x - q * L2;
-    C *line = region + q * TE;
-    const T msT = a.unit_source ? T(1) : (T)a.ms;
-    int buf = 0;
-    if (blockIdx.x < ngroups) issue(blockIdx.x, 0);
-    for (int g = blockIdx.x; g < ngroups; g += gridDim.x) {
-        const int gn = g + gridDim.x;
-        if (gn < ngroups) issue(gn, buf ^ 1);
-        else cp_async_commit();  // an empty group keeps "all but the newest" meaning this chunk
-        cp_async_wait_all_but_one();
-        __syncthreads();
-        const int yb = g % nyb, cz = g / nyb, z = cz % nz, c = cz / nz;
-        const int y0 = yb * RB, ya = y0 + 2 * q, yb1 = ya + 1;
-        const T *ra = stage + buf * stage_elems + (size_t)(2 * q) * nx, *rb = ra + nx;
-        auto in = [&](int j) -> C {
-            C v = mk<T>(0, 0);
-            if (ya < ny) v.x = ra[j] * msT;
-            if (yb1 < ny) v.y = rb[j] * msT;
-            return v;
-        };
-        auto out = [&](int k, C v) { line[k] = v; };
-        fft4step<L1, L2, false, false, true, true>(t, tws, line, in, out);
-        __syncthreads();
-        C *s1row = a.s1 + ((long long)c * nz + z) * nkx * ny;
-        auto emit = [&](int k, int r) {
-            const int y = y0 + r;
-            if (y >= ny) return;
-            const C *ln = region + (r >> 1) * TE;
-            const C zk = ln[k];
-            const C zm = ln[k == 0 ? 0 : L - k];
-            C o;
-            if ((r & 1) == 0) { o.x = T(0.5) * (zk.x + zm.x); o.y = T(0.5) * (zk.y - zm.y); }
-            else { o.x = T(0.5) * (zk.y + zm.y); o.y = T(-0.5) * (zk.x - zm.x); }
-            s1row[(long long)k * ny + y] = o;
-        };
-        if (ny % 2 == 0 && blockDim.x % LP == 0) {
-            // a thread writes both rows of its line pair at one kx (adjacent in S1,
-            // one 16-byte store in FP32): Z[k] and Z[L - k] are read once
-            const int qq = threadIdx.x % LP, kstep = blockDim.x / LP, ya2 = y0 + 2 * qq;
-            if (ya2 < ny) {  // ny even: ya2 + 1 < ny as well
-                const C *ln = region + qq * TE;
-                for (int k = threadIdx.x / LP; k < nkx; k += kstep) {
-                    const C zk = ln[k];
-                    const C zm = ln[k == 0 ? 0 : L - k];
-                    C o0, o1;
-                    o0.x = T(0.5) * (zk.x + zm.x); o0.y = T(0.5) * (zk.y - zm.y);
-                    o1.x = T(0.5) * (zk.y + zm.y); o1.y = T(-0.5) * (zk.x - zm.x);
-                    C *d = s1row + (long long)k * ny + ya2;
-                    if constexpr (sizeof(C) == 8) *reinterpret_cast<float4 *>(d) = make_float4(o0.x, o0.y, o1.x, o1.y);
-                    else { d[0] = o0; d[1] = o1; }
-                }
-            }
-        } else if (blockDim.x % RB == 0) {
-            const int r = threadIdx.x % RB, kstep = blockDim.x / RB;
-            for (int k = threadIdx.x / RB; k < nkx; k += kstep) emit(k, r);
-        } else {
-            for (int u = threadIdx.x; u < nkx * RB; u += blockDim.x) emit(u / RB, u % RB);
-        }
-        __syncthreads();  // the line regions and this buffer are reused
-        buf ^= 1;
-    }
-    // retire the copy groups still in flight (none land in memory still read)
-    asm volatile("cp.async.wait_all;\n" ::: "memory");
-}
-
-// ---------------------------------------------------------------------------
-// x inverse: gather A/B half spectra (transposed), form Z = A + iB on the full
-// circle, C2R, crop, 1/P, mask.  Same grid as k_xf_r.
-// ---------------------------------------------------------------------------
-// TWS: the twiddles were copied into shared memory after the line regions
-// (k_xi_r; the batched kernels read them from global memory).
-// line stride of the x inverse's shared regions (pair_stride with the pair gather)
-template <typename T, int L1, int L2, bool PAIR> __host__ __device__ constexpr int xi_stride() {
-    return PAIR ? pair_stride<T, L1, L2>() : line_region<L1, L2>();
-}
-
-// PAIR (ny even): a thread loads both rows of its line pair at one kx (adjacent
-// in S1) and writes Z[k], Z[L - k] itself, instead of the row-per-thread gather
-// whose pairs meet by shuffles; same values, no idle lanes.
-template <typename T, int L1, int L2, bool TWS = false, int U = 8, bool PAIR = false>
-__device__ __forceinline__ void xi_body(const DemagArgs<T> &a, int bx, int z, int c, unsigned char *smem_raw) {
-    using C = cx<T>;
-    constexpr int L = L1 * L2, TE = xi_stride<T, L1, L2, PAIR>();
-    C *region = reinterpret_cast<C *>(smem_raw);
-    const C *tw = TWS ? region + a.lines_x * TE : a.twxT;
-    const int LP = a.lines_x, RB = 2 * LP, nx = a.nx, ny = a.ny, nkx = a.nkx;
-    const int y0 = bx * RB;
-    // Z[k] = A[k] + i B[k] (k <= nx), Z[L-k] = conj(A[k]) + i conj(B[k]); DC and
-    // Nyquist taken as real.  Row pairs (A, B) sit in adjacent lanes.
-    const C *s1row = a.s1 + ((long long)c * a.nz + z) * nkx * ny;
-    auto place = [&](int k, int r, bool ok, C v) {
-        const T bx = __shfl_down_sync(0xffffffffu, v.x, 1);
-        const T by = __shfl_down_sync(0xffffffffu, v.y, 1);
-        if (ok && (r & 1) == 0) {
-            C A = v, B = mk<T>(bx, by);
-            C *ln = region + (r >> 1) * TE;
-            if (k == 0 || k == L / 2) {
-                ln[k] = mk<T>(A.x, B.x);
-            } else {
-                ln[k] = mk<T>(A.x - B.y, A.y + B.x);
-                ln[L - k] = mk<T>(A.x + B.y, -A.y + B.x);
-            }
-        }
-    };
-    if (PAIR && blockDim.x % LP == 0) {
-        const int qq = threadIdx.x % LP, kstep = blockDim.x / LP, k0 = threadIdx.x / LP;
-        const int ya = y0 + 2 * qq;  // ny even: ya < ny implies ya + 1 < ny
-        const bool rows = ya < ny;
-        const int iters = (nkx + kstep - 1) / kstep;
-        C *ln = region + qq * TE;
-        for (int it0 = 0; it0 < iters; it0 += U) {
-            C va[U], vb[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int k = k0 + (it0 + u) * kstep;
-                if (k < nkx && rows) {
-                    const C *p = s1row + (long long)k * ny + ya;
-                    if constexpr (sizeof(C) == 8) {
-                        const float4 v = *reinterpret_cast<const float4 *>(p);  // 16-byte aligned: ya, ny even
-                        va[u] = mk<T>(v.x, v.y);
-                        vb[u] = mk<T>(v.z, v.w);
-                    } else {
-                        va[u] = p[0];
-                        vb[u] = p[1];
-                    }
-                } else {
-                    va[u] = mk<T>(0, 0);
-                    vb[u] = mk<T>(0, 0);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int k = k0 + (it0 + u) * kstep;
-                if (k < nkx) {
-                    const C A = va[u], B = vb[u];
-                    if (k == 0 || k == L / 2) {
-                        ln[k] = mk<T>(A.x, B.x);
-                    } else {
-                        ln[k] = mk<T>(A.x - B.y, A.y + B.x);
-                        ln[L - k] = mk<T>(A.x + B.y, -A.y + B.x);
-                    }
-                }
-            }
-        }
-    } else if (blockDim.x % RB == 0) {
-        // fixed row per thread, warp-uniform trip count (the shuffle needs whole
-        // warps); U independent loads in flight per thread before they are placed
-        const int r = threadIdx.x % RB, kstep = blockDim.x / RB, k0 = threadIdx.x / RB;
-        const int y = y0 + r;
-        const int iters = (nkx + kstep - 1) / kstep;
-        for (int it0 = 0; it0 < iters; it0 += U) {
-            C vv[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int k = k0 + (it0 + u) * kstep;
-                vv[u] = (k < nkx && y < ny) ? s1row[(long long)k * ny + y] : mk<T>(0, 0);
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                if (it0 + u < iters) {
-                    const int k = k0 + (it0 + u) * kstep;
-                    place(k < nkx ? k : 0, r, k < nkx, vv[u]);
-                }
-            }
-        }
-    } else {
-        const int total = nkx * RB;
-        const int span = (total + 31) / 32 * 32;
-        for (int u = threadIdx.x; u < span; u += blockDim.x) {
-            const int k = u / RB, r = u % RB, y = y0 + r;
-            const bool ok = u < total;
-            const C v = (ok && y < ny) ? s1row[(long long)k * ny + y] : mk<T>(0, 0);
-            place(k, r, ok, v);
-        }
-    }
-    __syncthreads();
-    const int q = threadIdx.x / L2, t = threadIdx.x - q * L2;
-    const int ya = y0 + 2 * q, yb = ya + 1;
-    C *line = region + q * TE;
-    const T nrm = (T)a.norm;
-    T *hc = a.hd + (long long)c * a.n;
-    const long long rowa = ((long long)z * ny + ya) * nx, rowb = rowa + nx;
-    auto in = [&](int j) -> C { return line[j]; };
-    // no mask and no Ms map: every cell is active when Ms > 0 (cell_active's answer)
-    const bool uniform = !a.mask && !a.ms_map;
-    const bool uni_on = a.ms > 0.0;
-    auto out = [&](int k, C v) {
-        if (k >= nx) return;
-        if (uniform) {
-            if (ya < ny) hc[rowa + k] = uni_on ? v.x * nrm : T(0);
-            if (yb < ny) hc[rowb + k] = uni_on ? v.y * nrm : T(0);
-            return;
-        }
-        double msi;
-        if (ya < ny) hc[rowa + k] = cell_active(a, rowa + k, msi) ? v.x * nrm : T(0);
-        if (yb < ny) hc[rowb + k] = cell_active(a, rowb + k, msi) ? v.y * nrm : T(0);
-    };
-    fft4step<L1, L2, true, true, false>(t, tw, line, in, out);
-}
-
-// Shared memory: lines_x line regions, then the Lx twiddles.  U: gather loads
-// in flight per thread (xi_gather: measured at 512 x 512 x 8 with S1 out of
-// L2, FP32 U = 8 / 33: 57.4 / 52.3 us, FP64 U = 8 / 17: 102.7 / 94.8 us).
-template <typename T> __host__ __device__ constexpr int xi_gather() { return sizeof(T) == 4 ? 33 : 17; }
-// pair gather (two rows per load): 17 load slots, one round at 513 kx
-template <typename T> __host__ __device__ constexpr int xi_gather_pair() { return 17; }
-
-template <typename T, int L1, int L2, int U = 8, bool PAIR = false>
-__global__ void __launch_bounds__(256) k_xi_r(DemagArgs<T> a) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    cx<T> *tws = reinterpret_cast<cx<T> *>(smem_raw) + a.lines_x * xi_stride<T, L1, L2, PAIR>();
-    for (int k = threadIdx.x; k < L1 * L2; k += blockDim.x) tws[k] = a.twxT[k];
-    // the first barrier inside xi_body (after the gather) precedes every twiddle read
-    xi_body<T, L1, L2, true, U, PAIR>(a, blockIdx.x, blockIdx.y, blockIdx.z, smem_raw);
-}
-
-// ---------------------------------------------------------------------------
-// y forward (3-D): S1 -> S2, line g = (c, z, kx); block = lines_y groups of L2
-// ---------------------------------------------------------------------------
-template <typename T, int L1, int L2, bool PAD = false>
-__device__ __forceinline__ void yf_body(const DemagArgs<T> &a, int bx, unsigned char *smem_raw) {
-    using C = cx<T>;
-    constexpr int L = L1 * L2, TE = tile_elems(L1, L2);
-    const C *tw = a.twyT;
-    C *region = reinterpret_cast<C *>(smem_raw);
-    const int q = threadIdx.x / L2, t = threadIdx.x - q * L2, ny = a.ny;
-    const long long total = 3LL * a.nz * a.nkx;
-    const long long g = (long long)bx * a.lines_y + q;
-    const bool valid = g < total;
-    const C *src = a.s1 + g * ny;
-    C *dst = a.s2 + g * L;
-    auto in = [&](int j) -> C { return (valid && (!PAD || j < ny)) ? src[j] : mk<T>(0, 0); };
-    auto out = [&](int k, C v) { if (valid) dst[k] = v; };
-    fft4step<L1, L2, false, false, false, true>(t, tw, region + q * TE, in, out);
-}
-
-template <typename T, int L1, int L2>
-__global__ void __launch_bounds__(256) k_yf_r(DemagArgs<T> a) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    yf_body<T, L1, L2>(a, blockIdx.x, smem_raw);
-}
-
-// y inverse (3-D): S2 -> S1, keeps y < ny
-template <typename T, int L1, int L2>
-__device__ __forceinline__ void yi_body(const DemagArgs<T> &a, int bx, unsigned char *smem_raw) {
-    using C = cx<T>;
-    constexpr int L = L1 * L2, TE = tile_elems(L1, L2);
-    const C *tw = a.twyT;
-    C *region = reinterpret_cast<C *>(smem_raw);
-    const int q = threadIdx.x / L2, t = threadIdx.x - q * L2, ny = a.ny;
-    const long long total = 3LL * a.nz * a.nkx;
-    const long long g = (long long)bx * a.lines_y + q;
-    const bool valid = g < total;
-    const C *src = a.s2 + g * L;
-    C *dst = a.s1 + g * ny;
-    auto in = [&](int j) -> C { return valid ? src[j] : mk<T>(0, 0); };
-    auto out = [&](int k, C v) { if (valid && k < ny) dst[k] = v; };
-    fft4step<L1, L2, true, false, false>(t, tw, region + q * TE, in, out);
-}
-
-template <typename T, int L1, int L2>
-__global__ void __launch_bounds__(256) k_yi_r(DemagArgs<T> a) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    yi_body<T, L1, L2>(a, blockIdx.x, smem_raw);
-}
-
 // ---------------------------------------------------------------------------
 // z convolution (3-D): P threads per (kx, ky) column hold the three
 // components' z lines in registers: forward FFT, H = -N M per kz, inverse FFT,
@@ -575,6 +143,7 @@ template <typename T, int LZ, int P>
 __global__ void __launch_bounds__(128) k_zc_r(DemagArgs<T> a) {
     const int span = ((a.nkx * a.Ly * P + 127) / 128) * 128;  // whole pairs and warps iterate together
     const int h = (P == 2) ? (threadIdx.x & 1) : 0;
+    pdl_wait();
     for (int tid = blockIdx.x * blockDim.x + threadIdx.x; tid < span; tid += gridDim.x * blockDim.x)
         zc_task<T, LZ, P>(a, tid, h);
 }
@@ -636,6 +205,7 @@ __global__ void __launch_bounds__(zd_threads<T>()) k_zd(DemagArgs<T> a) {
                 if (c < 4 || d > 0)  // tau(0) = 0 is not read
                     cp_async_elem<sizeof(T)>(dt + (c * NZ + d) * BT * (unsigned)sizeof(T), tp + c * tstr + d * dstr);
     };
+    pdl_wait();
     const int stride = gridDim.x * BT;
     int col = blockIdx.x * BT + tid, buf = 0;
     if (col < cols) prefetch(col, 0);
@@ -667,44 +237,6 @@ __global__ void __launch_bounds__(zd_threads<T>()) k_zd(DemagArgs<T> a) {
         }
     }
     cp_async_wait_all();
-}
-
-
-// ---------------------------------------------------------------------------
-// y convolution (2-D thin film): block = kb_y kx columns x 3 components, each
-// line a group of L2 threads: forward y, multiply with N(kx, ky, 0), inverse y.
-// ---------------------------------------------------------------------------
-template <typename T, int L1, int L2>
-__global__ void __launch_bounds__(256) k_yc_r(DemagArgs<T> a) {
-    using C = cx<T>;
-    constexpr int L = L1 * L2, TE = line_region<L1, L2>();
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const C *tw = a.twyT;
-    C *region = reinterpret_cast<C *>(smem_raw);
-    const int KB = a.kb_y, ny = a.ny, nkx = a.nkx;
-    const int q = threadIdx.x / L2, t = threadIdx.x - q * L2;
-    const int comp = q / KB, kxl = q - comp * KB;
-    const int kx0 = blockIdx.x * KB, kx = kx0 + kxl;
-    const bool valid = kx < nkx;
-    C *line = region + q * TE;
-    C *g = a.s1 + ((long long)comp * nkx + kx) * ny;
-    auto in_g = [&](int j) -> C { return valid ? g[j] : mk<T>(0, 0); };
-    auto out_s = [&](int k, C v) { line[k] = v; };
-    fft4step<L1, L2, false, false, true, true>(t, tw, line, in_g, out_s);
-    __syncthreads();
-    for (int u = threadIdx.x; u < KB * L; u += blockDim.x) {
-        const int kl = u / L, ky = u - kl * L;
-        if (kx0 + kl >= nkx) continue;
-        C *lx = region + (0 * KB + kl) * TE, *lyy = region + (1 * KB + kl) * TE,
-          *lz = region + (2 * KB + kl) * TE;
-        C mx = lx[ky], my = lyy[ky], mz = lz[ky];
-        tensor_apply(a, kx0 + kl, ky, 0, mx, my, mz);
-        lx[ky] = mx; lyy[ky] = my; lz[ky] = mz;
-    }
-    __syncthreads();
-    auto in_s = [&](int j) -> C { return line[j]; };
-    auto out_g = [&](int k, C v) { if (valid && k < ny) g[k] = v; };
-    fft4step<L1, L2, true, true, false>(t, tw, line, in_s, out_g);
 }
 
 }  // namespace fm

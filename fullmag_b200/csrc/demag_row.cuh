@@ -11,7 +11,7 @@
 // y0 + RB - 1, all three components):
 //   1. gather: the slab's S1 rows (3 RB/2 complex lines, each a pair of real
 //      rows) are read into shared memory as the full-circle spectrum
-//      Z = A + i B of the line pair, as k_xi_r's pair gather does;
+//      Z = A + i B of the line pair, as the x inverse's gather does;
 //   2. x inverse: each line is C2R-transformed in place (fft4step), keeping
 //      x < nx, times 1/(Lx Ly Lz): the slab's H_d rows, in shared memory;
 //   3. stage: per group of V = 16 / sizeof(T) cells along x, the 6-point

@@ -25,11 +25,12 @@
 // table is uploaded in the same order (yzy_table), so the lanes of the z sum read
 // neighbouring slots of every row and neighbouring table values.
 //
-// Measured at 512 x 512 x 8 (FP32, P = 2, one half plane's CTA): 12.4 kcycles
-// forward, 16.8 the z sum, 8 inverse; the z sum is bound by its 576 packed
-// multiply-adds per column (2.05 cycles each per scheduler, the FP32 peak).
-// 106 us with 3-pass lines of 64 threads and named barriers, 100 us with the
-// two-pass lines of one warp each; P = 1 (384 threads) 114 us.
+// Measured at 512 x 512 x 8 (FP32, P = 2): 106 us with 3-pass lines of 64 threads and
+// named barriers, 100 us with the two-pass lines of one warp each (P = 1 with 384
+// threads 114 us); a half plane's CTA then took 12.4 kcycles for the forward lines, 16.8
+// for the z sum and 8 for the inverse, the z sum bound by its 576 packed multiply-adds
+// per column (2.05 cycles each per scheduler, the FP32 peak).  With the 288 of the sum
+// over even and odd halves: 89 us.
 // Two units per precision (demag_yzy_f32.cu, demag_yzy_f32b.cu, ..: nz <= 4 and
 // above), so that they compile in parallel.
 #pragma once
@@ -44,6 +45,7 @@
 #include "demag.cuh"
 #include "demag_reg.cuh"
 #include "linefft.cuh"
+#include "pdl.cuh"
 #include "demag_yzy.hpp"
 
 namespace cg = cooperative_groups;
@@ -117,8 +119,9 @@ __global__ void __launch_bounds__((yzy_threads<T, L, NZ, P>()), (yzy_min_blocks<
             asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
         }
     }
+    pdl_wait();
     // 1. forward y, LPP lines per pass: inputs y < ny (= L/2; the upper half is the
-    // zero padding).  Every thread takes part in every pass (fft4step has barriers).
+    // zero padding).  Every thread takes part in every pass (the lines' barriers).
 #pragma unroll 1
     for (int r0 = 0; r0 < ROWS; r0 += LPP) {
         const int lr = r0 + qg, q = h * NLH + lr;  // local row, line q = c nz + z
@@ -242,8 +245,10 @@ cudaLaunchConfig_t yzy_config(const Backend &b, cudaLaunchAttribute *attr) {
     cfg.blockDim = dim3((unsigned)yzy_threads<T, L, NZ, P>());
     cfg.dynamicSmemBytes = yzy_smem<T, L, NZ, P>();
     cfg.stream = b.stream;
-    cfg.attrs = attr;
-    cfg.numAttrs = P > 1 ? 1 : 0;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = P > 1 ? attr : attr + 1;
+    cfg.numAttrs = P > 1 ? 2 : 1;
     return cfg;
 }
 
@@ -277,7 +282,7 @@ static bool yzy_configure_t(Backend &b) {
                         return;
                     }
                     if constexpr (PP > 1) {
-                        cudaLaunchAttribute attr[1];
+                        cudaLaunchAttribute attr[2];
                         cudaLaunchConfig_t cfg = yzy_config<T, L, NZ, PP>(b, attr);
                         int nclusters = 0;
                         if (cudaOccupancyMaxActiveClusters(&nclusters, kern, &cfg) != cudaSuccess || nclusters < 1) {
@@ -301,7 +306,7 @@ static bool yzy_launch_t(Backend &b, const DemagArgs<T> &a) {
         yzy_with_p(b.yzy_P, [&](auto pc) {
             constexpr int PP = decltype(pc)::value;
             if constexpr (yzy_fits<T, L, NZ, PP>()) {
-                cudaLaunchAttribute attr[1];
+                cudaLaunchAttribute attr[2];
                 cudaLaunchConfig_t cfg = yzy_config<T, L, NZ, PP>(b, attr);
                 cudaLaunchKernelEx(&cfg, k_yzy<T, L, NZ, PP>, a);
             }

@@ -166,6 +166,7 @@ __global__ void __launch_bounds__(kZdwThreads, 2) k_zdw(DemagArgs<float> a, int 
     };
     const int warp = tid >> 5, lane = tid & 31;
     const int cl = (warp & 1) * 32 + lane, half = warp >> 1;
+    pdl_wait();
     int bt = blockIdx.x, buf = 0;
     if (bt < nbat) issue(bt, 0);
     cp_async_commit();

@@ -53,8 +53,8 @@ bool zdw_configure(Backend &b) {
 void zdw_launch(Backend &b, const DemagArgs<float> &a) {
     zdw_with_nz(b.nz, [&](auto nzc) {
         constexpr int NZ = decltype(nzc)::value;
-        if (b.zdw_win) k_zdw<NZ, true><<<b.grid_zdw, kZdwThreads, b.rsm_zdw, b.stream>>>(a, b.zdw_kyp);
-        else k_zdw<NZ, false><<<b.grid_zdw, kZdwThreads, b.rsm_zdw, b.stream>>>(a, 0);
+        if (b.zdw_win) pdl_launch(k_zdw<NZ, true>, dim3((unsigned)b.grid_zdw), dim3(kZdwThreads), b.rsm_zdw, b.stream, a, b.zdw_kyp);
+        else pdl_launch(k_zdw<NZ, false>, dim3((unsigned)b.grid_zdw), dim3(kZdwThreads), b.rsm_zdw, b.stream, a, 0);
     });
 }
 

@@ -177,10 +177,16 @@ __device__ __forceinline__ void lf_dft(C (&v)[R]) { lf_dft_at<R, 0, INV, R>(v); 
 // plans: passes R0 x R1 x R2 and threads per line.  G <= 32 divides 32 (a line
 // lies in one warp); V = L / G values per thread.
 // ---------------------------------------------------------------------------
-// FP32 at 1024 points: two passes of 32 values in one warp.  Measured at 512 x 512 x 8
-// against 16 x 8 x 8 on 64 threads: y passes 31.2 against 33.2 us, x forward 24.2 / 25.6,
-// x inverse 29.2 / 27.5, the fused plane pass 100 / 106 (its lines then need no
-// barrier at all); FP64 would need 128 registers for the values alone.
+// Longer chains of values per thread cost latency on grids that do not fill the chip,
+// fewer cost a third pass; measured per length and precision:
+// - FP32 at 1024 points: two passes of 32 values in one warp.  At 512 x 512 x 8 against
+//   16 x 8 x 8 on 64 threads: y passes 31.2 against 33.2 us, x forward 24.2 / 25.6, x
+//   inverse 29.2 / 27.5, the fused plane pass 100 / 106 (its lines then need no barrier).
+// - FP32 at 256: 16 x 16 on 16 threads; 4 x 8 x 8 on 32 the same alone, but 14.7 against
+//   10.7 us in the fused plane pass of 128 x 128 x 8.
+// - elsewhere 8 to 12 values per thread against 16 to 24: 300 x 180 x 5 masked FP32 143 ->
+//   116 us per Heun step, 256 x 256 FP32 54 -> 37, 90 x 90 x 4 FP32 56 -> 42, 384 x 384 x 8
+//   FP64 528 -> 430; 256 x 256 x 8 FP32 105 -> 101.
 template <typename T, int L> struct LfPlan;
 #define FM_LF_PLAN(L_, R0_, R1_, R2_, G_) \
     template <typename T> struct LfPlan<T, L_> { static constexpr int L = L_, R0 = R0_, R1 = R1_, R2 = R2_, G = G_; }
@@ -190,18 +196,19 @@ FM_LF_PLAN(8, 8, 1, 1, 1);
 FM_LF_PLAN(16, 4, 4, 1, 4);
 FM_LF_PLAN(32, 8, 4, 1, 4);
 FM_LF_PLAN(64, 8, 8, 1, 8);
-FM_LF_PLAN(96, 12, 8, 1, 4);
-FM_LF_PLAN(128, 16, 8, 1, 8);
-FM_LF_PLAN(192, 24, 8, 1, 8);
-FM_LF_PLAN(256, 16, 16, 1, 16);
-FM_LF_PLAN(384, 6, 8, 8, 16);
-FM_LF_PLAN(512, 8, 8, 8, 32);
-FM_LF_PLAN(768, 12, 8, 8, 32);
+FM_LF_PLAN(96, 6, 4, 4, 16);
+FM_LF_PLAN(128, 4, 4, 8, 16);
+FM_LF_PLAN(192, 6, 4, 8, 32);
+FM_LF_PLAN(256, 4, 8, 8, 32);
+FM_LF_PLAN(384, 6, 8, 8, 32);
+FM_LF_PLAN(512, 8, 8, 8, 64);
+FM_LF_PLAN(768, 12, 8, 8, 64);
 FM_LF_PLAN(1024, 16, 8, 8, 64);
 FM_LF_PLAN(1536, 24, 8, 8, 64);
 FM_LF_PLAN(2048, 16, 16, 8, 128);
 FM_LF_PLAN(4096, 16, 16, 16, 256);
 #undef FM_LF_PLAN
+template <> struct LfPlan<float, 256> { static constexpr int L = 256, R0 = 16, R1 = 16, R2 = 1, G = 16; };
 template <> struct LfPlan<float, 1024> { static constexpr int L = 1024, R0 = 32, R1 = 32, R2 = 1, G = 32; };
 
 // The lengths above; any length >= 2n - 1 gives the linear convolution of n cells.
@@ -375,6 +382,23 @@ __device__ __forceinline__ void line_fwd(int t, int q, const C *__restrict__ tw,
     }
 }
 
+// out(n, x) or, where it takes the output's index within the thread too, out(n, i, x):
+// line_out_count<T, L, HALF>() outputs per thread, output i at n = line_out_index(t, i).
+template <class Out, typename C>
+__device__ __forceinline__ void line_emit(Out &out, int n, int i, C x) {
+    if constexpr (std::is_invocable_v<Out &, int, int, C>) out(n, i, x);
+    else out(n, x);
+}
+template <typename T, int L, bool HALF> __host__ __device__ constexpr int line_out_count() {
+    using F = Lf<T, L>;
+    return (F::NP == 1 ? 1 : (F::M0 + F::G - 1) / F::G) * (HALF ? F::R0 / 2 : F::R0);
+}
+template <typename T, int L, bool HALF> __device__ __forceinline__ int line_out_index(int t, int i) {
+    using F = Lf<T, L>;
+    constexpr int NO = HALF ? F::R0 / 2 : F::R0;
+    return F::NP == 1 ? i : t + F::G * (i / NO) + F::M0 * (i % NO);
+}
+
 // Inverse (unnormalised): X[k] = in(k), out(n, x[n]) for n < L/2 with HALF, else
 // all n.  in(k) may read the tile at line_slot(k).
 template <int L, bool HALF, typename C, class In, class Out>
@@ -389,7 +413,7 @@ __device__ __forceinline__ void line_inv(int t, int q, const C *__restrict__ tw,
         for (int i = 0; i < R0; ++i) v[i] = in(i);
         lf_dft<R0, true>(v);
 #pragma unroll
-        for (int n = 0; n < NO; ++n) out(n, v[lf_perm<R0>(n)]);
+        for (int n = 0; n < NO; ++n) line_emit(out, n, n, v[lf_perm<R0>(n)]);
     } else {
         constexpr int RL = F::NP == 3 ? R2 : R1, NL = L / RL, BL = (NL + G - 1) / G;
         {
@@ -453,7 +477,7 @@ __device__ __forceinline__ void line_inv(int t, int q, const C *__restrict__ tw,
             }
             lf_dft<R0, true>(v);
 #pragma unroll
-            for (int i = 0; i < NO; ++i) out(j + M0 * i, v[lf_perm<R0>(i)]);
+            for (int i = 0; i < NO; ++i) line_emit(out, j + M0 * i, b * NO + i, v[lf_perm<R0>(i)]);
         }
     }
 }

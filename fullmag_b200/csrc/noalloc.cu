@@ -202,6 +202,8 @@ extern "C" int fullmag_fdm_demag_field_f64_noalloc(uint32_t nx, uint32_t ny, uin
         put_error(error_out, error_out_len, "cudaFuncSetAttribute failed");
         return FULLMAG_FDM_ERR_CUDA;
     }
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    line.pdl = cudaStreamIsCapturing(st, &capturing) == cudaSuccess && capturing == cudaStreamCaptureStatusNone;
     line_x_fwd<double>(line, a, st);
     if (thin) {
         line_y_conv<double>(line, a, st);

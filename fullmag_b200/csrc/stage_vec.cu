@@ -12,16 +12,18 @@ bool stage_vec_launch(Backend &b, const StageArgs<float> &s, int mode) {
     const int zb = stage_vec_zb(b, (int)sizeof(float), diag);
     if (b.stage_vec_mk) {  // mask and / or Ms map
         switch (mode) {
-            case MODE_EVAL: k_stage_vec<float, MODE_EVAL, true><<<g, blk, 0, b.stream>>>(s, zb); break;
-            case MODE_HEUN_CORR: k_stage_vec<float, MODE_HEUN_CORR, true><<<g, blk, 0, b.stream>>>(s, zb); break;
-            default: k_stage_vec<float, MODE_ERR_LAST, true><<<g, blk, 0, b.stream>>>(s, zb); break;
+            case MODE_EVAL: pdl_launch(k_stage_vec<float, MODE_EVAL, true>, g, blk, 0, b.stream, s, zb); break;
+            case MODE_HEUN_CORR: pdl_launch(k_stage_vec<float, MODE_HEUN_CORR, true>, g, blk, 0, b.stream, s, zb); break;
+            case MODE_EVAL_NEXT: pdl_launch(k_stage_vec<float, MODE_EVAL_NEXT, true>, g, blk, 0, b.stream, s, zb); break;
+            default: pdl_launch(k_stage_vec<float, MODE_ERR_LAST, true>, g, blk, 0, b.stream, s, zb); break;
         }
         return true;
     }
     switch (mode) {
-        case MODE_EVAL: k_stage_vec<float, MODE_EVAL><<<g, blk, 0, b.stream>>>(s, zb); break;
-        case MODE_HEUN_CORR: k_stage_vec<float, MODE_HEUN_CORR><<<g, blk, 0, b.stream>>>(s, zb); break;
-        default: k_stage_vec<float, MODE_ERR_LAST><<<g, blk, 0, b.stream>>>(s, zb); break;
+        case MODE_EVAL: pdl_launch(k_stage_vec<float, MODE_EVAL>, g, blk, 0, b.stream, s, zb); break;
+        case MODE_HEUN_CORR: pdl_launch(k_stage_vec<float, MODE_HEUN_CORR>, g, blk, 0, b.stream, s, zb); break;
+        case MODE_EVAL_NEXT: pdl_launch(k_stage_vec<float, MODE_EVAL_NEXT>, g, blk, 0, b.stream, s, zb); break;
+        default: pdl_launch(k_stage_vec<float, MODE_ERR_LAST>, g, blk, 0, b.stream, s, zb); break;
     }
     return true;
 }
@@ -30,7 +32,7 @@ bool combine_vec_launch(Backend &b, const CombineArgs<float> &a) {
     constexpr int V = 16 / (int)sizeof(float);
     const long long groups = b.n / V;
     const unsigned grid = (unsigned)std::max<long long>(1, std::min<long long>((groups + 255) / 256, 148LL * 16));
-    k_combine_vec<float><<<grid, 256, 0, b.stream>>>(a);
+    pdl_launch(k_combine_vec<float>, dim3(grid), dim3(256), 0, b.stream, a);
     return true;
 }
 

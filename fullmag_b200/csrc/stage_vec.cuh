@@ -64,7 +64,7 @@ __device__ __forceinline__ double sv_inv_norm(double n2) {
 constexpr int kStageVecBY = 4;  // rows (warps) per block
 
 template <typename T, int MODE> __host__ __device__ constexpr int stage_vec_min_blocks() {
-    return sizeof(T) == 4 ? 5 : 4;
+    return sizeof(T) == 4 && MODE != MODE_EVAL_NEXT ? 5 : 4;
 }
 
 // activity bits of V cells from index i (bit j: cell i + j)
@@ -97,6 +97,27 @@ template <typename R>
 struct SvConst {
     R ix2, iy2, iz2, pref, hx[3], al, gb, pr;
 };
+
+// Squared embedded error of a group's cells from NKE earlier slopes and the last one.
+template <typename T, int NKE>
+__device__ __forceinline__ void sv_error(const StageArgs<T> &a, unsigned n, unsigned i0,
+                                         const SVec<T> (&rhs)[3], double (&e2)[16 / sizeof(T)]) {
+    constexpr int V = 16 / (int)sizeof(T);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        SVec<T> kv[NKE];
+#pragma unroll
+        for (int st = 0; st < NKE; ++st) kv[st] = sv_ld<T>(a.ke[st] + c * n + i0);
+#pragma unroll
+        for (int j = 0; j < V; ++j) {
+            double e = 0.0;
+#pragma unroll
+            for (int st = 0; st < NKE; ++st) e += a.ew[st] * (double)kv[st].v[j];
+            const double ej = (e + a.ew[NKE] * (double)rhs[c].v[j]) * a.dt;
+            e2[j] += ej * ej;
+        }
+    }
+}
 
 // One group: V cells of row y, plane z, from x0 (an owning thread: x0 < nx,
 // y < ny; the others pass the last group of the row with own = false and only
@@ -275,28 +296,46 @@ __device__ __forceinline__ void sv_group(const StageArgs<T> &a, const PlainConst
 #pragma unroll
         for (int c = 0; c < 3; ++c) sv_st(dst + c * n + i0, nw[c]);
     }
+    if (MODE == MODE_EVAL_NEXT) {
+        // the next stage state, as combine_vec_group forms it
+        double v[3][V];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const SVec<T> m0 = sv_ld<T>(a.cb_m0 + c * n + i0);
+            SVec<T> kv[4];
+#pragma unroll
+            for (int s = 0; s < 4; ++s)
+                if (s < a.cb_form) kv[s] = sv_ld<T>(a.cb_k[s] + c * n + i0);
+#pragma unroll
+            for (int j = 0; j < V; ++j) {
+                const double r = (double)rhs[c].v[j];
+                double k[5];
+#pragma unroll
+                for (int s = 0; s < 5; ++s) k[s] = s < 4 && s < a.cb_form ? (double)kv[s < 4 ? s : 3].v[j] : r;
+                v[c][j] = a.cb_form == 0 ? __fma_rn(r, a.cb_c[0], (double)m0.v[j])
+                                         : (double)m0.v[j] + combine_inc(a.cb_form, k, a.cb_c, a.cb_dt);
+            }
+        }
+        SVec<T> nw[3];
+#pragma unroll
+        for (int j = 0; j < V; ++j) {
+            const double inv = sv_inv_norm<T>(v[0][j] * v[0][j] + v[1][j] * v[1][j] + v[2][j] * v[2][j]);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) nw[c].v[j] = (T)(v[c][j] * inv);
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) sv_st(a.cb_out + c * n + i0, nw[c]);
+    }
     if (MODE == MODE_ERR_LAST && diag) {
         // err = dt (sum_j ew[j] ke[j] + ew[nke] k_last) in FP64, accumulated from
         // zero in that order (max_error_norm_buf, lib.rs:1653-1674)
         double e2[V];
 #pragma unroll
         for (int j = 0; j < V; ++j) e2[j] = 0.0;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            double e[V];
-#pragma unroll
-            for (int j = 0; j < V; ++j) e[j] = 0.0;
-            for (int st = 0; st < a.nke; ++st) {
-                const SVec<T> kv = sv_ld<T>(a.ke[st] + c * n + i0);
-#pragma unroll
-                for (int j = 0; j < V; ++j) e[j] += a.ew[st] * (double)kv.v[j];
-            }
-#pragma unroll
-            for (int j = 0; j < V; ++j) {
-                const double ej = (e[j] + a.ew[a.nke] * (double)rhs[c].v[j]) * a.dt;
-                e2[j] += ej * ej;
-            }
-        }
+        // the slope count as a constant (DP45 5, RK23 3), so that a component's loads are
+        // all in flight together
+        if (a.nke == 5) sv_error<T, 5>(a, n, i0, rhs, e2);
+        else sv_error<T, 3>(a, n, i0, rhs, e2);
 #pragma unroll
         for (int j = 0; j < V; ++j)
             if ((act >> j) & 1u) acc[Q_ERR2] = fmax(acc[Q_ERR2], e2[j]);
@@ -325,6 +364,7 @@ __global__ void __launch_bounds__(32 * kStageVecBY, (stage_vec_min_blocks<T, MOD
 #pragma unroll
     for (int k = 0; k < NQ; ++k) acc[k] = 0.0;
     R mx_heff = R(0), mx_hd = R(0), mx_rhs = R(0);
+    pdl_wait();
     const int z0 = blockIdx.z * zb, z1 = min(z0 + zb, nz);
     for (int z = z0; z < z1; ++z)
         sv_group<T, MODE, MK>(a, kc, q, lane, xc, yc, z, own, acc, mx_heff, mx_hd, mx_rhs);
@@ -350,6 +390,7 @@ namespace fm {
 // component.  Requires n to be a multiple of V.
 template <typename T>
 __global__ void __launch_bounds__(256) k_combine_vec(CombineArgs<T> a) {
+    pdl_wait();
     constexpr int V = 16 / (int)sizeof(T);
     const size_t n = (size_t)a.n, groups = n / V;
     for (size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x; g < groups; g += (size_t)gridDim.x * blockDim.x) {

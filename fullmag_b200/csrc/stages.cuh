@@ -19,6 +19,7 @@
 
 #include "common.cuh"
 #include "cpasync.cuh"
+#include "pdl.cuh"
 
 namespace fm {
 
@@ -37,6 +38,7 @@ __host__ __device__ constexpr bool q_is_max(int q) { return q >= Q_HEFF2; }
 enum : int {
     MODE_EVAL = 0,        // k = RHS(m); optional observables / diagnostics
     MODE_HEUN_CORR = 1,   // k2 = RHS(m_p); m <- normalize(m0 + dt/2 (k1 + k2))
+    MODE_EVAL_NEXT = 7,   // k = RHS(m) and the integrator's next stage state
     MODE_ERR_LAST = 2,    // k_last = RHS(y); diagnostics + embedded error norm (DP45, RK23)
 };
 
@@ -87,7 +89,25 @@ struct StageArgs {
     // k, the arithmetic of k_combine form 0 (null: not written)
     T *pred_out;
     double pred_dt;
+    // MODE_EVAL_NEXT: the integrator's next stage state, normalize(cb_m0 + the weighted
+    // slopes) with the stored k as the last slope: combine_cell's form cb_form on
+    // cb_k[0 .. cb_form) and k (cb_out is not the buffer of m)
+    const T *cb_m0;
+    const T *cb_k[4];
+    double cb_c[5], cb_dt;
+    int cb_form;
+    T *cb_out;
 };
+
+// The increment of one component in combine_cell's forms (k: the slopes in order).
+__device__ __forceinline__ double combine_inc(int form, const double (&k)[5], const double *c, double dt) {
+    switch (form) {
+        case 1: return (k[0] * c[0] + k[1] * c[1]) * dt;
+        case 2: return ((k[0] * c[0] + k[1] * c[1]) + k[2] * c[2]) * dt;
+        case 3: return ((k[0] * c[0] + k[1] * c[1]) + (k[2] * c[2] + k[3] * c[3])) * dt;
+        default: return (((k[0] * c[0] + k[1] * c[1]) + k[2] * c[2]) + (k[3] * c[3] + k[4] * c[4])) * dt;
+    }
+}
 
 __device__ __forceinline__ double warp_reduce(double v, bool is_max) {
 #pragma unroll
@@ -125,6 +145,34 @@ __device__ __forceinline__ void store_predictor(const StageArgs<T> &a, size_t i,
     a.pred_out[i] = (T)(v0 * inv);
     a.pred_out[n + i] = (T)(v1 * inv);
     a.pred_out[2 * n + i] = (T)(v2 * inv);
+}
+
+// The next stage state of cell i from its slope r (as stored in T), the arithmetic
+// of combine_cell.
+template <typename T>
+__device__ __forceinline__ void store_combination(const StageArgs<T> &a, size_t i, size_t n, double r0, double r1,
+                                                  double r2) {
+    const double r[3] = {(double)(T)r0, (double)(T)r1, (double)(T)r2};
+    double v[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        const double m0 = (double)a.cb_m0[q * n + i];
+        double k[5];
+#pragma unroll
+        for (int j = 0; j < 5; ++j) k[j] = j < a.cb_form ? (double)a.cb_k[j < 4 ? j : 3][q * n + i] : r[q];
+        v[q] = a.cb_form == 0 ? __fma_rn(r[q], a.cb_c[0], m0) : m0 + combine_inc(a.cb_form, k, a.cb_c, a.cb_dt);
+    }
+    const double n2 = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
+    double inv;
+    if (sizeof(T) == 8) {
+        const double nn = sqrt(n2);
+        inv = nn > 0.0 ? 1.0 / nn : 0.0;
+    } else {
+        inv = n2 > 0.0 ? rsqrt(n2) : 0.0;
+    }
+    a.cb_out[i] = (T)(v[0] * inv);
+    a.cb_out[n + i] = (T)(v[1] * inv);
+    a.cb_out[2 * n + i] = (T)(v[2] * inv);
 }
 
 // Exchange field of the boundary tiers at an active cell i = (x, y, z) with
@@ -262,6 +310,7 @@ __device__ __forceinline__ void block_reduce_final(double (&acc)[NQ], double *pa
 // independent threads keep enough loads in flight to stream HBM.
 template <typename T, int MODE>
 __global__ void __launch_bounds__(256, 3) k_stage(StageArgs<T> a) {
+    pdl_wait();
     using R = double;
     double acc[NQ];
 #pragma unroll
@@ -287,6 +336,7 @@ __global__ void __launch_bounds__(256, 3) k_stage(StageArgs<T> a) {
                 const double c0[3] = {(double)mx[i], (double)my[i], (double)mz[i]};
                 store_predictor(a, (size_t)i, (size_t)n, c0, 0.0, 0.0, 0.0);
             }
+            if (MODE == MODE_EVAL_NEXT) store_combination(a, (size_t)i, (size_t)n, 0.0, 0.0, 0.0);
         } else {
             // neighbours: clamped at the grid edge, inactive -> centre (lib.rs:2255-2286)
             long long nb[6];
@@ -356,6 +406,7 @@ __global__ void __launch_bounds__(256, 3) k_stage(StageArgs<T> a) {
                     r2 = (pr * p2 + q2 * al) * gb;
             if (a.kout) { a.kout[i] = (T)r0; a.kout[n + i] = (T)r1; a.kout[2 * n + i] = (T)r2; }
             if (MODE == MODE_EVAL && a.pred_out) store_predictor(a, (size_t)i, (size_t)n, c3, r0, r1, r2);
+            if (MODE == MODE_EVAL_NEXT) store_combination(a, (size_t)i, (size_t)n, r0, r1, r2);
             if (a.hex_out) { a.hex_out[i] = (T)h0; a.hex_out[n + i] = (T)h1; a.hex_out[2 * n + i] = (T)h2; }
             if (a.heff_out) { a.heff_out[i] = (T)e0; a.heff_out[n + i] = (T)e1; a.heff_out[2 * n + i] = (T)e2; }
             if (MODE == MODE_HEUN_CORR) {
@@ -502,6 +553,7 @@ __device__ __forceinline__ void plain_cell(const StageArgs<T> &a, const PlainCon
     if (!inxy) return;
     if (a.kout) { a.kout[i] = (T)r0; a.kout[n + i] = (T)r1; a.kout[2 * (size_t)n + i] = (T)r2; }
     if (MODE == MODE_EVAL && a.pred_out) store_predictor(a, (size_t)i, (size_t)n, c, r0, r1, r2);
+    if (MODE == MODE_EVAL_NEXT) store_combination(a, (size_t)i, (size_t)n, r0, r1, r2);
     if (a.hex_out) { a.hex_out[i] = (T)h[0]; a.hex_out[n + i] = (T)h[1]; a.hex_out[2 * (size_t)n + i] = (T)h[2]; }
     if (a.heff_out) { a.heff_out[i] = (T)e0; a.heff_out[n + i] = (T)e1; a.heff_out[2 * (size_t)n + i] = (T)e2; }
     if (MODE == MODE_HEUN_CORR) {
@@ -694,6 +746,7 @@ __global__ void __launch_bounds__(128, ring_min_blocks<T, MODE>()) k_stage_ring(
         }
     };
     const PlainConst k = plain_const(a);
+    pdl_wait();
     unsigned i = (unsigned)z0 * sxy + ic;
     T cT[3] = {f0[i], f1[i], f2[i]};
     R c[3] = {(R)cT[0], (R)cT[1], (R)cT[2]};
@@ -745,6 +798,7 @@ __global__ void __launch_bounds__(128, ring_min_blocks<T, MODE>()) k_stage_ring(
 
 template <typename T, int MODE>
 __global__ void __launch_bounds__(128, 4) k_stage_plain(StageArgs<T> a, int zb) {
+    pdl_wait();
     double acc[NQ];
 #pragma unroll
     for (int q = 0; q < NQ; ++q) acc[q] = 0.0;
@@ -818,6 +872,7 @@ __device__ __forceinline__ void combine_cell(const CombineArgs<T> &a, long long 
 
 template <typename T>
 __global__ void __launch_bounds__(256) k_combine(CombineArgs<T> a) {
+    pdl_wait();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < a.n;
          i += (long long)gridDim.x * blockDim.x)
         combine_cell(a, i);

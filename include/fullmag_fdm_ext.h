@@ -83,9 +83,8 @@ int fullmag_fdm_adjoint_backward(fullmag_fdm_backend *handle, const double *dl_d
  * of a step is one persistent launch over all problems, and a step is one
  * CUDA graph.  Grids up to 512 x 512 x 8 cells; the demag spectra are the
  * library's FP64 Newell tensor (no mask, regions or boundary tiers), for each
- * problem's padding: x and y to the smallest power of two >= 2n, or in FP32
- * the smallest power of two or 3 * 2^k (96, 192, 384, 768) >= 2n; z to a power
- * of two >= 2 nz.  On the
+ * problem's padding: x and y to the smallest power of two or 3 * 2^k (96, 192,
+ * 384, 768) >= 2n, at least 16; z to a power of two >= 2 nz.  On the
  * first fullmag_fdm_batch_step_n call an autotuner picks each kernel's
  * persistent grid size and the tile shape of the x and y passes (128- or
  * 256-thread blocks); fullmag_fdm_batch_tuning reports the picks (7 grid sizes:
@@ -180,7 +179,7 @@ int fullmag_fdm_newell_spectra(uint32_t nx, uint32_t ny, uint32_t nz, double dx,
  * giving the bytes needed.
  *
  * The first call on a device resolves the scratch array's device address,
- * fills the twiddle constants and synchronises the device once; make that
+ * fills the twiddle tables and synchronises the device once; make that
  * first call outside any CUDA stream capture.  The constants are not refilled
  * after cudaDeviceReset (or any new primary context) on that device, so do not
  * use this entry point across a device reset.  All calls share the one scratch
