@@ -340,7 +340,12 @@ struct Impl {
         if (!upload_tw64(b)) return false;
         if (!b.force_stockham) {
             b.use_reg = true;
-            return configure_line(b) && row_configure<T>(b);
+            if (!configure_line(b) || !row_configure<T>(b)) return false;
+            // a time-dependent field enters the kernels' arguments: no graphs then.  Up to
+            // 2^18 cells a step's kernels take 3 to 8 us each, a launch 1.6 to 3 us of the host
+            // and 8 of them with their synchronisation 20 us; one graph of 8 takes 10.
+            b.use_graphs = !b.use_row && b.n <= (1LL << 18) && b.ac_freq == 0.0;
+            return true;
         }
         b.use_reg = false;
         b.zdirect = false;
@@ -698,6 +703,52 @@ struct Impl {
         return true;
     }
 
+    // The launches of `body` (no synchronisation or host copy among them), which depend on
+    // nothing but the handle and (kind, dt, stats, buffers): the first time as they are,
+    // the second captured into a graph, then that graph.  An adaptive run, whose dt
+    // changes from step to step, never pays for a capture.
+    template <class F>
+    static bool step_launches(Backend &b, int kind, double dt, bool stats, F &&body) {
+        if (!b.use_graphs || b.profiling) return body();
+        // the buffers in their present roles: accepted steps swap them
+        const void *bufs[Backend::kStepBuffers] = {b.m, b.mstage, b.mstage2};
+        for (int i = 0; i < 7; ++i) bufs[3 + i] = b.k[i];
+        Backend::StepGraph *g = nullptr;
+        for (auto &e : b.graphs)
+            if (e.kind == kind && e.dt == dt && e.stats == stats && std::equal(bufs, bufs + Backend::kStepBuffers, e.bufs)) g = &e;
+        if (!g) {
+            g = &b.graphs[b.graph_next];
+            b.graph_next = (b.graph_next + 1) % Backend::kStepGraphs;
+            if (g->exec) cudaGraphExecDestroy(g->exec);
+            *g = Backend::StepGraph{};
+            g->kind = kind; g->dt = dt; g->stats = stats;
+            std::copy(bufs, bufs + Backend::kStepBuffers, g->bufs);
+            return body();
+        }
+        if (!g->exec) {
+            cudaGraph_t graph = nullptr;
+            if (cudaStreamBeginCapture(b.stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
+                cudaGetLastError();
+                b.use_graphs = false;
+                return body();
+            }
+            const bool ok = body();
+            const cudaError_t e = cudaStreamEndCapture(b.stream, &graph);
+            cudaError_t ei = e;
+            if (ok && e == cudaSuccess) ei = cudaGraphInstantiate(&g->exec, graph, 0);
+            if (graph) cudaGraphDestroy(graph);
+            if (!ok || ei != cudaSuccess) {
+                // nothing of the captured step has run: run it as it is, here and from now on
+                cudaGetLastError();
+                g->exec = nullptr;
+                b.use_graphs = false;
+                b.last_error.clear();
+                return body();
+            }
+        }
+        return cuda_ok(b, cudaGraphLaunch(g->exec, b.stream), "step graph");
+    }
+
     // One Heun step (lib.rs:1217-1249) with the cached k1.
     static bool heun(Backend &b, double dt, fullmag_fdm_step_stats *st, bool readback) {
         if (b.use_row) return heun_rows(b, dt, st, readback);
@@ -706,22 +757,28 @@ struct Impl {
         // already wrote it when this dt equals the previous one
         if (!(b.pred_valid && b.pred_dt == dt) && !combine(b, 0, b.m, {b.k[0]}, {dt}, dt, b.mstage)) return false;
         b.pred_valid = false;
-        if (!demag(b, b.mstage, b.hd)) return false;
-        // corrector at m_p: k2 and m <- normalize(m0 + (k1 + k2) dt/2)
-        StageArgs<T> s = stage_args(b, b.mstage, b.time + dt);
-        s.kout = nullptr;  // k2 is consumed in registers
-        s.m0 = (T *)b.m;
-        s.k1 = (const T *)b.k[0];
-        s.half_dt = 0.5 * dt;
-        {
-            ProfScope p(b, "stage_heun_corr");
-            launch_stage<MODE_HEUN_CORR>(b, s);
-        }
-        if (!check_launch(b, "heun corrector")) return false;
-        // fields, RHS (next k1) and the next predictor at the new state; the diagnostics
-        // only where they are read back (512 x 512 x 8 FP32: 38 us against 47)
-        if (!demag(b, b.m, b.hd)) return false;
-        if (!eval(b, b.m, b.time + dt, b.k[0], readback, false, b.mstage, dt)) return false;
+        const bool launched = step_launches(b, FULLMAG_FDM_INTEGRATOR_HEUN, dt, readback, [&]() -> bool {
+            if (!demag(b, b.mstage, b.hd)) return false;
+            // corrector at m_p: k2 and m <- normalize(m0 + (k1 + k2) dt/2)
+            StageArgs<T> s = stage_args(b, b.mstage, b.time + dt);
+            s.kout = nullptr;  // k2 is consumed in registers
+            s.m0 = (T *)b.m;
+            s.k1 = (const T *)b.k[0];
+            s.half_dt = 0.5 * dt;
+            {
+                ProfScope p(b, "stage_heun_corr");
+                launch_stage<MODE_HEUN_CORR>(b, s);
+            }
+            if (!check_launch(b, "heun corrector")) return false;
+            // fields, RHS (next k1) and the next predictor at the new state; the diagnostics
+            // only where they are read back (512 x 512 x 8 FP32: 38 us against 47)
+            if (!demag(b, b.m, b.hd)) return false;
+            if (!eval(b, b.m, b.time + dt, b.k[0], readback, false, b.mstage, dt)) return false;
+            return true;
+        });
+        if (!launched) return false;
+        b.s1_state = 0;
+        b.hd_stale = false;  // the last field is that of the new state
         b.pred_valid = true;
         b.pred_dt = dt;
         b.time += dt;
@@ -757,36 +814,40 @@ struct Impl {
             // the stage states alternate between two buffers: a stage kernel writes the next
             // one while its stencil reads its own
             void *x = b.mstage, *y = b.mstage2;
-            if (!combine(b, 0, b.m, {k[0]}, {A21 * dt}, dt, x)) return false;
-            if (!demag(b, x, b.hd) || !eval_combine(b, x, t + 0.2 * dt, k[1], 1, b.m, {k[0]}, {A31, A32}, dt, y)) return false;
-            if (!demag(b, y, b.hd) ||
-                !eval_combine(b, y, t + 0.3 * dt, k[2], 2, b.m, {k[0], k[1]}, {A41, A42, A43}, dt, x)) return false;
-            if (!demag(b, x, b.hd) ||
-                !eval_combine(b, x, t + 0.8 * dt, k[3], 3, b.m, {k[0], k[1], k[2]}, {A51, A52, A53, A54}, dt, y)) return false;
-            if (!demag(b, y, b.hd) ||
-                !eval_combine(b, y, t + 8.0 / 9.0 * dt, k[4], 4, b.m, {k[0], k[1], k[2], k[3]}, {A61, A62, A63, A64, A65}, dt, x))
-                return false;
-            // k6 and the 5th-order solution, then k7 = RHS(y5) with the embedded error norm
-            if (!demag(b, x, b.hd) ||
-                !eval_combine(b, x, t + dt, k[5], 4, b.m, {k[0], k[2], k[3], k[4]}, {B1, B3, B4, B5, B6}, dt, y)) return false;
-            if (!demag(b, y, b.hd)) return false;
-            StageArgs<T> s = stage_args(b, y, t + dt);
-            s.kout = (T *)k[6];
-            s.partials = b.partials;
-            s.counter = b.counter;
-            s.out = b.d_out;
-            // err = dt (E1 k1 + E3 k3 + E4 k4 + E5 k5 + E6 k6 + E7 k7), lib.rs:1653-1674
-            s.ke[0] = (const T *)k[0]; s.ke[1] = (const T *)k[2]; s.ke[2] = (const T *)k[3];
-            s.ke[3] = (const T *)k[4]; s.ke[4] = (const T *)k[5];
-            s.nke = 5;
-            s.ew[0] = 71.0 / 57600.0; s.ew[1] = -71.0 / 16695.0; s.ew[2] = 71.0 / 1920.0;
-            s.ew[3] = -17253.0 / 339200.0; s.ew[4] = 22.0 / 525.0; s.ew[5] = -1.0 / 40.0;
-            s.dt = dt;
-            {
-                ProfScope p(b, "stage_dp45_last");
-                launch_stage<MODE_ERR_LAST>(b, s);
-            }
-            if (!check_launch(b, "dp45 last stage") || !read_stats(b)) return false;
+            const bool launched = step_launches(b, FULLMAG_FDM_INTEGRATOR_DP45, dt, true, [&]() -> bool {
+                if (!combine(b, 0, b.m, {k[0]}, {A21 * dt}, dt, x)) return false;
+                if (!demag(b, x, b.hd) || !eval_combine(b, x, t + 0.2 * dt, k[1], 1, b.m, {k[0]}, {A31, A32}, dt, y)) return false;
+                if (!demag(b, y, b.hd) ||
+                    !eval_combine(b, y, t + 0.3 * dt, k[2], 2, b.m, {k[0], k[1]}, {A41, A42, A43}, dt, x)) return false;
+                if (!demag(b, x, b.hd) ||
+                    !eval_combine(b, x, t + 0.8 * dt, k[3], 3, b.m, {k[0], k[1], k[2]}, {A51, A52, A53, A54}, dt, y)) return false;
+                if (!demag(b, y, b.hd) ||
+                    !eval_combine(b, y, t + 8.0 / 9.0 * dt, k[4], 4, b.m, {k[0], k[1], k[2], k[3]}, {A61, A62, A63, A64, A65}, dt, x))
+                    return false;
+                // k6 and the 5th-order solution, then k7 = RHS(y5) with the embedded error norm
+                if (!demag(b, x, b.hd) ||
+                    !eval_combine(b, x, t + dt, k[5], 4, b.m, {k[0], k[2], k[3], k[4]}, {B1, B3, B4, B5, B6}, dt, y)) return false;
+                if (!demag(b, y, b.hd)) return false;
+                StageArgs<T> s = stage_args(b, y, t + dt);
+                s.kout = (T *)k[6];
+                s.partials = b.partials;
+                s.counter = b.counter;
+                s.out = b.d_out;
+                // err = dt (E1 k1 + E3 k3 + E4 k4 + E5 k5 + E6 k6 + E7 k7), lib.rs:1653-1674
+                s.ke[0] = (const T *)k[0]; s.ke[1] = (const T *)k[2]; s.ke[2] = (const T *)k[3];
+                s.ke[3] = (const T *)k[4]; s.ke[4] = (const T *)k[5];
+                s.nke = 5;
+                s.ew[0] = 71.0 / 57600.0; s.ew[1] = -71.0 / 16695.0; s.ew[2] = 71.0 / 1920.0;
+                s.ew[3] = -17253.0 / 339200.0; s.ew[4] = 22.0 / 525.0; s.ew[5] = -1.0 / 40.0;
+                s.dt = dt;
+                {
+                    ProfScope p(b, "stage_dp45_last");
+                    launch_stage<MODE_ERR_LAST>(b, s);
+                }
+                return true;
+            });
+            b.s1_state = 0;
+            if (!launched || !check_launch(b, "dp45 last stage") || !read_stats(b)) return false;
             const double err = std::sqrt(b.h_out[Q_ERR2]);
             if (err <= b.max_error || dt <= b.dt_min) {
                 std::swap(b.m, b.mstage2);
@@ -808,12 +869,11 @@ struct Impl {
         }
     }
 
-    // Fields and RHS at the accepted state into k[0] (the next step's k1), with
-    // the step diagnostics where they are read back; advances the step counter.
-    static bool finish_step(Backend &b, double dt, fullmag_fdm_step_stats *st, bool readback, void *pred_out = nullptr,
-                            double pred_dt = 0.0) {
-        if (!demag(b, b.m, b.hd)) return false;
-        if (!eval(b, b.m, b.time, b.k[0], readback, false, pred_out, pred_dt)) return false;
+    // After the RHS at the accepted state has gone into k[0] (the next step's k1):
+    // advances the step counter and reads the statistics back where they are wanted.
+    static bool finish_step(Backend &b, double dt, fullmag_fdm_step_stats *st, bool readback) {
+        b.s1_state = 0;
+        b.hd_stale = false;
         b.step_count += 1;
         b.k1_valid = true;
         b.obs_valid = false;
@@ -835,14 +895,19 @@ struct Impl {
         const double t = b.time;
         void *x = b.mstage, *y = b.mstage2;
         if (!(pred && b.pred_dt == 0.5 * dt) && !combine(b, 0, b.m, {k[0]}, {0.5 * dt}, dt, x)) return false;
-        if (!demag(b, x, b.hd) || !eval_combine(b, x, t + 0.5 * dt, k[1], 0, b.m, {}, {0.5 * dt}, dt, y)) return false;
-        if (!demag(b, y, b.hd) || !eval_combine(b, y, t + 0.5 * dt, k[2], 0, b.m, {}, {dt}, dt, x)) return false;
-        // k4, then m <- normalize(m0 + ((k1 + 2 k2) + (2 k3 + k4)) dt/6), in place
-        if (!demag(b, x, b.hd) ||
-            !eval_combine(b, x, t + dt, k[3], 3, b.m, {k[0], k[1], k[2]}, {1.0, 2.0, 2.0, 1.0}, dt / 6.0, b.m)) return false;
+        const bool launched = step_launches(b, FULLMAG_FDM_INTEGRATOR_RK4, dt, readback, [&]() -> bool {
+            if (!demag(b, x, b.hd) || !eval_combine(b, x, t + 0.5 * dt, k[1], 0, b.m, {}, {0.5 * dt}, dt, y)) return false;
+            if (!demag(b, y, b.hd) || !eval_combine(b, y, t + 0.5 * dt, k[2], 0, b.m, {}, {dt}, dt, x)) return false;
+            // k4, then m <- normalize(m0 + ((k1 + 2 k2) + (2 k3 + k4)) dt/6), in place
+            if (!demag(b, x, b.hd) ||
+                !eval_combine(b, x, t + dt, k[3], 3, b.m, {k[0], k[1], k[2]}, {1.0, 2.0, 2.0, 1.0}, dt / 6.0, b.m)) return false;
+            // RHS at the new state (the next k1), the statistics where they are read back, and
+            // the next step's first stage state for the same dt
+            return demag(b, b.m, b.hd) && eval(b, b.m, t + dt, k[0], readback, false, b.mstage, 0.5 * dt);
+        });
+        if (!launched) return false;
         b.time += dt;
-        // the next step's first stage state too, for the same dt
-        if (!finish_step(b, dt, st, readback, b.mstage, 0.5 * dt)) return false;
+        if (!finish_step(b, dt, st, readback)) return false;
         b.pred_valid = true;
         b.pred_dt = 0.5 * dt;
         return true;
@@ -860,25 +925,29 @@ struct Impl {
         for (;;) {
             const double t = b.time;
             void *x = b.mstage, *y = b.mstage2;
-            if (!combine(b, 0, b.m, {k[0]}, {0.5 * dt}, dt, x)) return false;
-            if (!demag(b, x, b.hd) || !eval_combine(b, x, t + 0.5 * dt, k[1], 0, b.m, {}, {0.75 * dt}, dt, y)) return false;
-            if (!demag(b, y, b.hd) ||
-                !eval_combine(b, y, t + 0.75 * dt, k[2], 2, b.m, {k[0], k[1]}, {2.0 / 9.0, 1.0 / 3.0, 4.0 / 9.0}, dt, x)) return false;
-            if (!demag(b, x, b.hd)) return false;
-            StageArgs<T> s = stage_args(b, b.mstage, t + dt);
-            s.kout = (T *)k[3];
-            s.partials = b.partials;
-            s.counter = b.counter;
-            s.out = b.d_out;
-            s.ke[0] = (const T *)k[0]; s.ke[1] = (const T *)k[1]; s.ke[2] = (const T *)k[2];
-            s.nke = 3;
-            s.ew[0] = -5.0 / 72.0; s.ew[1] = 1.0 / 12.0; s.ew[2] = 1.0 / 9.0; s.ew[3] = -1.0 / 8.0;
-            s.dt = dt;
-            {
-                ProfScope p(b, "stage_rk23_last");
-                launch_stage<MODE_ERR_LAST>(b, s);
-            }
-            if (!check_launch(b, "rk23 last stage") || !read_stats(b)) return false;
+            const bool launched = step_launches(b, FULLMAG_FDM_INTEGRATOR_RK23, dt, true, [&]() -> bool {
+                if (!combine(b, 0, b.m, {k[0]}, {0.5 * dt}, dt, x)) return false;
+                if (!demag(b, x, b.hd) || !eval_combine(b, x, t + 0.5 * dt, k[1], 0, b.m, {}, {0.75 * dt}, dt, y)) return false;
+                if (!demag(b, y, b.hd) ||
+                    !eval_combine(b, y, t + 0.75 * dt, k[2], 2, b.m, {k[0], k[1]}, {2.0 / 9.0, 1.0 / 3.0, 4.0 / 9.0}, dt, x)) return false;
+                if (!demag(b, x, b.hd)) return false;
+                StageArgs<T> s = stage_args(b, b.mstage, t + dt);
+                s.kout = (T *)k[3];
+                s.partials = b.partials;
+                s.counter = b.counter;
+                s.out = b.d_out;
+                s.ke[0] = (const T *)k[0]; s.ke[1] = (const T *)k[1]; s.ke[2] = (const T *)k[2];
+                s.nke = 3;
+                s.ew[0] = -5.0 / 72.0; s.ew[1] = 1.0 / 12.0; s.ew[2] = 1.0 / 9.0; s.ew[3] = -1.0 / 8.0;
+                s.dt = dt;
+                {
+                    ProfScope p(b, "stage_rk23_last");
+                    launch_stage<MODE_ERR_LAST>(b, s);
+                }
+                return true;
+            });
+            b.s1_state = 0;
+            if (!launched || !check_launch(b, "rk23 last stage") || !read_stats(b)) return false;
             const double err = std::sqrt(b.h_out[Q_ERR2]);
             if (err <= b.max_error || dt <= b.dt_min) {
                 std::swap(b.m, b.mstage);
@@ -937,6 +1006,8 @@ struct Impl {
         if (!combine(b, 2, b.m, {k[1], k[2], k[3]}, {5.0 / 12.0, 8.0 / 12.0, -1.0 / 12.0}, dt, b.m)) return false;
         b.time += dt;
         abm_push(b, dt);
+        // fields and RHS at the accepted state, the statistics where they are read back
+        if (!demag(b, b.m, b.hd) || !eval(b, b.m, b.time, k[0], readback, false)) return false;
         return finish_step(b, dt, st, readback);
     }
 
@@ -1597,6 +1668,10 @@ void backend_free(Backend &b) {
     b.adj_mem = nullptr;
     if (b.h_out) cudaFreeHost(b.h_out);
     b.h_out = nullptr;
+    for (auto &g : b.graphs) {
+        if (g.exec) cudaGraphExecDestroy(g.exec);
+        g = Backend::StepGraph{};
+    }
     if (b.stream) cudaStreamDestroy(b.stream);
     b.stream = nullptr;
 }

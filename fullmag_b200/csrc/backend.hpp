@@ -142,6 +142,20 @@ struct Backend {
     std::string last_error;
     std::string err_buf;
     void *mstage2 = nullptr;  // the other stage state of the RK integrators
+    // a step's launches as a CUDA graph, per (kind, dt, statistics, buffers' roles): small
+    // grids, whose kernels are shorter than the time to launch them
+    static constexpr int kStepBuffers = 10;  // m, mstage, mstage2, k[0..6]
+    struct StepGraph {
+        int kind = -1;
+        double dt = 0.0;
+        bool stats = false;
+        const void *bufs[kStepBuffers] = {};
+        cudaGraphExec_t exec = nullptr;
+    };
+    static constexpr int kStepGraphs = 6;
+    StepGraph graphs[kStepGraphs];
+    int graph_next = 0;           // the entry replaced next
+    bool use_graphs = false;
     bool chain = false;       // RK stage kernels also form the next stage state (eval_combine)
 };
 

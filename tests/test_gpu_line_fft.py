@@ -1,0 +1,94 @@
+"""The line-FFT demag passes, the fused stage combinations and the step graphs.
+
+- Fields at every padded in-plane length the passes have (grids of 2n just below, at and
+  just above a length, odd row counts, both spectra sources) against the FP64 oracle, at
+  the field tolerances of the other parity tests: 1e-13 (FP64) and 2e-6 (FP32-mixed) of
+  each field's own maximum.
+- A Runge-Kutta step on either side of the cell count up to which the FP32 group kernels
+  form the next stage state themselves, FP32-mixed against FP64 at 1e-5 (the tolerance
+  of the FP32-mixed trajectories).
+- Steps replayed as CUDA graphs against the same launches issued one by one (per-kernel
+  timing on), bit for bit, through dt changes.
+- A handle with small blocks created after one with large blocks leaves its launches valid.
+"""
+import numpy as np
+import pytest
+
+from fullmag_b200 import native_fdm as nf
+from gpu_helpers import make_pair, max_abs
+
+pytestmark = pytest.mark.gpu
+
+D = (2e-9, 2.5e-9, 3e-9)
+H = (1e4, -2e4, 3e3)
+
+
+# (nx, ny, nz): 2n -> 16, 32, 64, 96, 128, 192, 256, 384, 512, 768, 1024, 1536, 2048 along x or y
+_CELLS = [(5, 7, 1), (9, 15, 3), (20, 36, 1), (48, 36, 2), (49, 64, 1), (70, 96, 2), (100, 7, 3),
+          (128, 25, 1), (135, 192, 1), (200, 245, 1), (3, 300, 2), (384, 9, 1), (10, 490, 1), (525, 4, 2),
+          (6, 625, 1), (800, 5, 1), (4, 1000, 2)]
+
+
+@pytest.mark.parametrize("prec", [nf.PRECISION_DOUBLE, nf.PRECISION_SINGLE])
+@pytest.mark.parametrize("cells", _CELLS)
+def test_padded_lengths_match_oracle(cells, prec):
+    nx, ny, nz = cells
+    rng = np.random.default_rng(nx + ny)
+    kw = dict(mask=(rng.random(nx * ny * nz) > 0.2).astype(np.uint8)) if ny % 2 else {}
+    source = "oracle" if nx % 2 else "newell"
+    be, sim, _ = make_pair(cells, D, h_ext=H, precision=prec, symmetric_kernel=True, seed=nx + 3, spectra=source, **kw)
+    be.refresh_observables()
+    obs = sim.observe()
+    tol = 1e-13 if prec == nf.PRECISION_DOUBLE else 2e-6
+    for o, key in ((nf.OBS_H_DEMAG, "h_demag"), (nf.OBS_H_EFF, "h_eff")):
+        assert max_abs(be.copy_field(o), obs[key]) <= tol * np.abs(obs[key]).max(), key
+    be.close()
+
+
+def _plan(cells, prec, integrator, seed=5, **kw):
+    n = cells[0] * cells[1] * cells[2]
+    m0 = nf.random_unit_vectors(seed, n).astype(np.float32).astype(np.float64)
+    if integrator in (nf.DP45, nf.RK23):
+        kw["adaptive"] = (1e-5, 1e-18, 2e-14, 0.8)
+    return nf.FdmPlan(cells=cells, cell_size=D, initial_magnetization=m0, damping=0.1, external_field=H,
+                      precision=prec, integrator=integrator, demag_source=nf.DEMAG_NEWELL, **kw)
+
+
+@pytest.mark.parametrize("integrator", [nf.RK4, nf.RK23, nf.DP45])
+@pytest.mark.parametrize("cells,masked", [((512, 512, 1), False), ((540, 512, 1), False), ((64, 48, 3), True), ((25, 18, 2), True)])
+def test_fused_combination_fp32_matches_fp64(cells, masked, integrator):
+    kw = {}
+    if masked:
+        kw["active_mask"] = (np.random.default_rng(3).random(cells[0] * cells[1] * cells[2]) > 0.2).astype(np.uint8)
+    out = []
+    for prec in (nf.PRECISION_SINGLE, nf.PRECISION_DOUBLE):
+        with nf.NativeFdmBackend(_plan(cells, prec, integrator, **kw)) as be:
+            for _ in range(3):
+                be.step(2e-14)
+            out.append(be.copy_m())
+    assert max_abs(out[0], out[1]) <= 1e-5
+
+
+@pytest.mark.parametrize("integrator", [nf.HEUN, nf.RK4, nf.RK23, nf.DP45, nf.ABM3])
+@pytest.mark.parametrize("cells,prec", [((40, 24, 1), nf.PRECISION_DOUBLE), ((36, 20, 3), nf.PRECISION_SINGLE)])
+def test_step_graphs_equal_single_launches(cells, prec, integrator):
+    dts = [1e-14] * 5 + [2e-14] * 4 + [1e-14] * 3
+    with nf.NativeFdmBackend(_plan(cells, prec, integrator)) as a, nf.NativeFdmBackend(_plan(cells, prec, integrator)) as b:
+        b.set_profiling(True)  # times each launch: no graphs
+        for i, dt in enumerate(dts):
+            sa, sb = a.step(dt), b.step(dt)
+            sa.pop("wall_time_ns"), sb.pop("wall_time_ns")
+            assert sa == sb, i
+        a.step_n(1e-14, 6)
+        b.step_n(1e-14, 6)
+        for o in (nf.OBS_M, nf.OBS_H_DEMAG, nf.OBS_H_EFF):
+            assert np.array_equal(a.copy_field(o), b.copy_field(o)), o
+
+
+def test_small_handle_does_not_limit_a_large_one():
+    for prec in (nf.PRECISION_DOUBLE, nf.PRECISION_SINGLE):
+        with nf.NativeFdmBackend(_plan((512, 512, 4), prec, nf.HEUN)) as big:
+            with nf.NativeFdmBackend(_plan((512, 2, 1), prec, nf.HEUN)) as small, \
+                    nf.NativeFdmBackend(_plan((2, 512, 2), prec, nf.HEUN)) as tall:
+                for be in (big, small, tall, big):
+                    assert np.isfinite(be.step(1e-14)["total_energy_joules"])
