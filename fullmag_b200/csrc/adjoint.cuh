@@ -199,4 +199,26 @@ __global__ void __launch_bounds__(256) k_adj_finish(long long n3, const double *
         lam[i] = acc[i] + part[i];
 }
 
+// Sums over the cells of the 3 components of two FP64 fields (SoA): block q < 6 sums
+// component q % 3 of a (q < 3) or b, each thread every 1024th cell in order, then a tree:
+// the same order on every run.  6 blocks: 65 536 cells are 64 loads per thread, once per
+// pull-back; on the host the sums waited for both fields' copies.
+__global__ void __launch_bounds__(1024) k_adj_sum(const double *a, const double *b, long long n, double *out) {
+    __shared__ double part[32];
+    pdl_wait();
+    const double *f = (blockIdx.x < 3 ? a : b) + (long long)(blockIdx.x % 3) * n;
+    double v = 0.0;
+    for (long long i = threadIdx.x; i < n; i += 1024) v += f[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        v = part[threadIdx.x];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        if (threadIdx.x == 0) out[blockIdx.x] = v;
+    }
+}
+
 }  // namespace fm

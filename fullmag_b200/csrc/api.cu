@@ -532,22 +532,7 @@ int fullmag_fdm_adjoint_backward(fullmag_fdm_backend *h, const double *dl_dm, ui
         b.last_error = "no recorded trajectory ends at the current state (call fullmag_fdm_adjoint_forward first)";
         return FULLMAG_FDM_ERR_INVALID;
     }
-    const size_t n = (size_t)b.n;
-    std::vector<double> lam(3 * n), gms(n), ghext(3 * n), ghac(3 * n), lam0(3 * n);
-    for (size_t i = 0; i < n; ++i)
-        for (int c = 0; c < 3; ++c) lam[c * n + i] = dl_dm[3 * i + c];
-    if (!fm::backend_adjoint_backward(b, lam.data(), gms.data(), ghext.data(), ghac.data(), lam0.data()))
-        return FULLMAG_FDM_ERR_CUDA;
-    if (dl_dms) std::copy(gms.begin(), gms.end(), dl_dms);
-    for (int c = 0; c < 3; ++c) {
-        double se = 0.0, sa = 0.0;  // fixed order: deterministic
-        for (size_t i = 0; i < n; ++i) { se += ghext[c * n + i]; sa += ghac[c * n + i]; }
-        if (dl_dh_ext) dl_dh_ext[c] = se;
-        if (dl_dh_ac) dl_dh_ac[c] = sa;
-    }
-    if (dl_dm0)
-        for (size_t i = 0; i < n; ++i)
-            for (int c = 0; c < 3; ++c) dl_dm0[3 * i + c] = lam0[c * n + i];
+    if (!fm::backend_adjoint_backward(b, dl_dm, dl_dms, dl_dh_ext, dl_dh_ac, dl_dm0)) return FULLMAG_FDM_ERR_CUDA;
     return FULLMAG_FDM_OK;
 }
 

@@ -551,15 +551,17 @@ struct BatchImpl {
         return ok;
     }
 
+    // State of a problem in the caller's layout (AoS FP64), brought there on the device in
+    // the problem's S1, which no step keeps anything in and which is longer (nkx > nx
+    // complex values per row).
     bool copy_m(fullmag_fdm_batch &B, uint32_t index, double *out) {
         const Prob &p = probs[index];
-        std::vector<T> h(3 * (size_t)p.n);
-        if (!batch_ok(B, cudaMemcpyAsync(h.data(), base() + p.off_m, h.size() * sizeof(T), cudaMemcpyDeviceToHost, B.stream), "copy m") ||
-            !batch_ok(B, cudaStreamSynchronize(B.stream), "copy m sync"))
-            return false;
-        for (long long c = 0; c < p.n; ++c)
-            for (int k = 0; k < 3; ++k) out[3 * c + k] = (double)h[k * p.n + c];
-        return true;
+        double *stage = (double *)(base() + p.off_s1);
+        k_batch_aos<T><<<(unsigned)std::min<long long>((p.n + 255) / 256, 148LL * 16), 256, 0, B.stream>>>(
+            (const T *)(base() + p.off_m), stage, p.n);
+        return batch_ok(B, cudaGetLastError(), "copy m") &&
+               batch_ok(B, cudaMemcpyAsync(out, stage, 3 * (size_t)p.n * sizeof(double), cudaMemcpyDeviceToHost, B.stream), "copy m") &&
+               batch_ok(B, cudaStreamSynchronize(B.stream), "copy m sync");
     }
 };
 
