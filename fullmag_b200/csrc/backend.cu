@@ -171,6 +171,7 @@ struct Impl {
         a.twx4 = (const C *)b.twx4; a.twy4 = (const C *)b.twy4;
         a.s1 = (C *)b.s1; a.s2 = (C *)b.s2;
         a.spec = (const T *)b.spec;
+        a.thin6 = b.thin6;
         a.m = (const T *)m;
         a.mask = b.d_mask;
         a.ms_map = b.d_msmap;
@@ -1393,6 +1394,9 @@ static bool upload_tables(Backend &b, const std::vector<double> (&spec)[6]) {
         return t.empty() || cuda_ok(b, cudaMemcpy(dst, t.data(), t.size() * sizeof(cx<T>), cudaMemcpyHostToDevice), "twiddles (line)");
     };
     if (!twl(b.Lx, b.twx4) || !twl(b.Ly, b.twy4)) return false;
+    b.thin6 = false;
+    for (int c = 4; b.thin && c < 6; ++c)
+        for (double v : spec[c]) b.thin6 = b.thin6 || v != 0.0;
     // the octant, or for the direct z convolution its z-inverse table (nz planes)
     std::vector<double> zt[6];
     if (b.zdirect) octant_to_z_direct(b.nkx, b.KY, b.nz, spec, zt);

@@ -82,6 +82,7 @@ struct Backend {
 
     // ---- demag ----
     bool thin = false;        // 2-D (nz = 1) spectra path
+    bool thin6 = false;       // thin, and the supplied tensor's xz or yz is not zero throughout
     bool projection = false;  // no spectra supplied: k k^T / k^2 tensor
     int Lx = 0, Ly = 0, Lz = 0, nkx = 0, KZ = 0, KY = 0;
     LinePlan px{}, py{}, pz{};

@@ -51,6 +51,7 @@ struct DemagArgs {
     int lines_y;            // lines per y-pass block
     int kt_z;               // ky tile of the z pass
     int kb_y;               // kx per block of the 2-D y_conv pass
+    int thin6;              // 2-D: the octant's xz and yz count too (else they are zero)
 };
 
 template <typename T>

@@ -278,17 +278,26 @@ __device__ __forceinline__ void ly_conv_body(const DemagArgs<T> &a, int bx, unsi
         if (kx0 + kl >= nkx) continue;
         C *lx = region + kl * TE + s, *ly = lx + KB * TE, *lz = ly + KB * TE;
         C mx = *lx, my = *ly, mz = *lz;
-        // a film's xz and yz are zero (odd in z)
         const bool mir = ky > L / 2;
         const T *sp = a.spec + (long long)(kx0 + kl) * a.KY + (mir ? L - ky : ky);
         const long long plane = (long long)nkx * a.KY;
         const T nxx = sp[0], nyy = sp[plane], nzz = sp[2 * plane], nxy = mir ? -sp[3 * plane] : sp[3 * plane];
-        lx->x = -(nxx * mx.x + nxy * my.x);
-        lx->y = -(nxx * mx.y + nxy * my.y);
-        ly->x = -(nxy * mx.x + nyy * my.x);
-        ly->y = -(nxy * mx.y + nyy * my.y);
-        lz->x = -(nzz * mz.x);
-        lz->y = -(nzz * mz.y);
+        if (!a.thin6) {  // a film's xz and yz are zero (odd in z): 4 of 6 tensor planes read
+            lx->x = -(nxx * mx.x + nxy * my.x);
+            lx->y = -(nxx * mx.y + nxy * my.y);
+            ly->x = -(nxy * mx.x + nyy * my.x);
+            ly->y = -(nxy * mx.y + nyy * my.y);
+            lz->x = -(nzz * mz.x);
+            lz->y = -(nzz * mz.y);
+        } else {  // an octant of the caller's that has them
+            const T nxz = sp[4 * plane], nyz = mir ? -sp[5 * plane] : sp[5 * plane];
+            lx->x = -((nxx * mx.x + nxy * my.x) + nxz * mz.x);
+            lx->y = -((nxx * mx.y + nxy * my.y) + nxz * mz.y);
+            ly->x = -((nxy * mx.x + nyy * my.x) + nyz * mz.x);
+            ly->y = -((nxy * mx.y + nyy * my.y) + nyz * mz.y);
+            lz->x = -((nxz * mx.x + nyz * my.x) + nzz * mz.x);
+            lz->y = -((nxz * mx.y + nyz * my.y) + nzz * mz.y);
+        }
     }
     __syncthreads();
     auto in_s = [&](int k) -> C { return line[line_slot<T, L>(k)]; };
@@ -299,9 +308,9 @@ __device__ __forceinline__ void ly_conv_body(const DemagArgs<T> &a, int bx, unsi
 template <typename T, int L>
 __global__ void __launch_bounds__((line_max_threads<T, L>() * 3 / 2)) k_ly_conv(DemagArgs<T> a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    // the block's columns of the tensor (xx, yy, zz, xy)
+    // the block's columns of the tensor (xx, yy, zz, xy; with thin6 also xz, yz)
     const int kx0 = blockIdx.x * a.kb_y, kb = min(a.kb_y, a.nkx - kx0);
-    for (int e = 0; e < 4; ++e)
+    for (int e = 0; e < (a.thin6 ? 6 : 4); ++e)
         warm_lines(a.spec + ((long long)e * a.nkx + kx0) * a.KY, kb * a.KY * (int)sizeof(T));
     line_begin<T, L>(a.twy4);
     ly_conv_body<T, L>(a, blockIdx.x, smem_raw);

@@ -326,7 +326,8 @@ bool octant_repad(int KZ, int nx, int ny, int Lx, int Ly, bool thin2d, double to
         for (int kz = 0; kz < KZ; ++kz)
             for (size_t kx = 0; kx < KX0; ++kx)
                 for (size_t ky = 0; ky < KY0; ++ky) {
-                    const bool edge = (oddx[c] && (kx == 0 || kx == KX0 - 1)) || (oddy[c] && (ky == 0 || ky == KY0 - 1));
+                    const bool none = thin2d && oddx[c] != oddy[c];  // a film's xz and yz are zero
+                    const bool edge = none || (oddx[c] && (kx == 0 || kx == KX0 - 1)) || (oddy[c] && (ky == 0 || ky == KY0 - 1));
                     if (edge && std::fabs(spec[c][(kz * KX0 + kx) * KY0 + ky]) > tol) return false;
                 }
     HostFft fx0((size_t)2 * nx), fy0((size_t)2 * ny), fx((size_t)Lx), fy((size_t)Ly);

@@ -39,9 +39,9 @@ void octant_to_z_direct(int nkx, int KY, int nz, const std::vector<double> (&spe
 // In-plane lengths of an octant spectrum [kz < KZ][kx <= nx][ky <= ny] of lengths
 // (2 nx, 2 ny) changed to even (Lx, Ly) with Lx >= 2 nx, Ly >= 2 ny: per axis back to
 // the offsets |d| < n (the wrapped entry d = n reaches no physical cell) and forward
-// at the new length.  thin2d: 2-D spectra (components odd in one in-plane axis are
-// zero).  False, with spec unchanged, when a component odd along an axis has more
-// than tol at frequency 0 or Nyquist there: no odd kernel has such a spectrum.
+// at the new length.  thin2d: a film's (xz and yz zero).  False, with spec unchanged,
+// when a component odd along an axis has more than tol at frequency 0 or Nyquist there,
+// or a film's xz or yz anywhere: no such kernel has that spectrum.
 bool octant_repad(int KZ, int nx, int ny, int Lx, int Ly, bool thin2d, double tol,
                   std::vector<double> (&spec)[6]);
 

@@ -190,6 +190,7 @@ extern "C" int fullmag_fdm_demag_field_f64_noalloc(uint32_t nx, uint32_t ny, uin
     a.twy4 = tw + tw_offset(Ly);
     a.s1 = ps1; a.s2 = thin ? nullptr : ps2;
     a.spec = octant;
+    a.thin6 = thin;  // the octant is the caller's: all six components
     a.m = m;
     a.mask = nullptr;
     a.ms_map = nullptr;

@@ -9,8 +9,12 @@
   of the FP32-mixed trajectories).
 - Steps replayed as CUDA graphs against the same launches issued one by one (per-kernel
   timing on), bit for bit, through dt changes.
+- A film's tensor with all six components (random octants) against numpy's FFT at the
+  FP64 field tolerance.
 - A handle with small blocks created after one with large blocks leaves its launches valid.
 """
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -92,3 +96,29 @@ def test_small_handle_does_not_limit_a_large_one():
                     nf.NativeFdmBackend(_plan((2, 512, 2), prec, nf.HEUN)) as tall:
                 for be in (big, small, tall, big):
                     assert np.isfinite(be.step(1e-14)["total_energy_joules"])
+
+
+@pytest.mark.parametrize("nx,ny", [(16, 16), (64, 32), (8, 128)])
+def test_film_octant_with_all_six_components(nx, ny):
+    """The allocation-free film call takes any real octant: xz and yz count where they are not zero."""
+    import torch
+    from test_zz_no_alloc import _entry
+
+    rng = np.random.default_rng(nx)
+    oct6, m, ms = rng.standard_normal((6, nx + 1, ny + 1)), rng.standard_normal((3, ny, nx)), 2.0
+    k = np.arange(2 * ny)
+    ky = np.where(k > ny, 2 * ny - k, k)
+    N = oct6[:, :, ky]                                     # [6][kx][ky], xy and yz odd in ky
+    N[[3, 5]] *= np.where(k > ny, -1.0, 1.0)
+    M = np.fft.fft(np.fft.rfft(ms * m, 2 * nx, axis=2), 2 * ny, axis=1).transpose(0, 2, 1)
+    xx, yy, zz, xy, xz, yz = N
+    H = -np.stack([xx * M[0] + xy * M[1] + xz * M[2], xy * M[0] + yy * M[1] + yz * M[2], xz * M[0] + yz * M[1] + zz * M[2]])
+    want = np.fft.irfft(np.fft.ifft(H, axis=2).transpose(0, 2, 1), 2 * nx, axis=2)[:, :ny, :nx]
+
+    dev = torch.device("cuda", 0)
+    o, mm = torch.from_numpy(oct6.copy()).to(dev), torch.from_numpy(np.ascontiguousarray(m)).to(dev)
+    h, err = torch.empty(3 * nx * ny, dtype=torch.float64, device=dev), C.create_string_buffer(512)
+    rc = _entry()(nx, ny, 1, 1, o.data_ptr(), mm.data_ptr(), ms, h.data_ptr(), torch.cuda.current_stream().cuda_stream, err, len(err))
+    assert rc == nf.OK, err.value.decode()
+    torch.cuda.synchronize()
+    assert np.abs(h.cpu().numpy().reshape(want.shape) - want).max() <= 1e-13 * np.abs(want).max()
