@@ -213,7 +213,10 @@ struct Impl {
         b.zreg = !b.thin && !b.zdirect && is_pow2(b.Lz) && b.Lz <= (dbl ? 16 : 32);
         if (!cuda_ok(b, line_setup<T>(b.line, b.Lx, b.Ly, b.thin, b.ny, b.nz, b.nkx), "line FFT setup")) return false;
         b.use_yz = false;
-        if (!b.thin && b.want_yz && b.zreg && is_pow2(b.Lx) && is_pow2(b.Ly) && !yz_configure<T>(b)) return false;
+        // the fused y-z pass folds a line at ny = Ly / 2 and writes all Ly / 2 outputs into
+        // S1's rows of ny: only where nothing is padded beyond 2n
+        if (!b.thin && b.want_yz && b.zreg && b.Lx == 2 * b.nx && b.Ly == 2 * b.ny && is_pow2(b.Lx) && is_pow2(b.Ly) &&
+            !yz_configure<T>(b)) return false;
         bool ok = true;
         if (b.zdirect) {
             with_nz(b.nz, [&](auto nzc) {

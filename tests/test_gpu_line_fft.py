@@ -4,6 +4,9 @@
   just above a length, odd row counts, both spectra sources) against the FP64 oracle, at
   the field tolerances of the other parity tests: 1e-13 (FP64) and 2e-6 (FP32-mixed) of
   each field's own maximum.
+- The switches of the z and fused passes on grids padded beyond 2n (the fused y-z pass,
+  which has no padding of its own, must leave them to the split kernels): fields as above,
+  m after 5 Heun steps at 1e-12 and 1e-6.
 - A Runge-Kutta step on either side of the cell count up to which the FP32 group kernels
   form the next stage state themselves, FP32-mixed against FP64 at 1e-5 (the tolerance
   of the FP32-mixed trajectories).
@@ -46,6 +49,30 @@ def test_padded_lengths_match_oracle(cells, prec):
     tol = 1e-13 if prec == nf.PRECISION_DOUBLE else 2e-6
     for o, key in ((nf.OBS_H_DEMAG, "h_demag"), (nf.OBS_H_EFF, "h_eff")):
         assert max_abs(be.copy_field(o), obs[key]) <= tol * np.abs(obs[key]).max(), key
+    be.close()
+
+
+@pytest.mark.parametrize("env", [("YZ", "fused"), ("ZCONV", "fft"), ("YZY", "off"), ("ROW", "on"), ("FFT", "stockham")])
+@pytest.mark.parametrize("cells,prec", [((64, 50, 4), nf.PRECISION_DOUBLE), ((64, 50, 8), nf.PRECISION_SINGLE),
+                                        ((50, 32, 2), nf.PRECISION_SINGLE), ((64, 96, 4), nf.PRECISION_SINGLE)])
+def test_switched_passes_on_padded_lengths(monkeypatch, env, cells, prec):
+    for k in ("YZ", "ZCONV", "YZY", "ROW", "FFT", "YZ_P"):
+        monkeypatch.delenv("FULLMAG_FDM_" + k, raising=False)
+    monkeypatch.setenv("FULLMAG_FDM_" + env[0], env[1])
+    be, sim, _ = make_pair(cells, D, alpha=0.3, h_ext=H, precision=prec, symmetric_kernel=True, seed=11, spectra="newell")
+    be.set_profiling(True)
+    be.refresh_observables()
+    names = set(be.profile())
+    be.set_profiling(False)
+    assert "demag_yz" not in names  # none of these has both lengths 2n
+    obs = sim.observe()
+    tol = 1e-13 if prec == nf.PRECISION_DOUBLE else 2e-6
+    for o, key in ((nf.OBS_H_DEMAG, "h_demag"), (nf.OBS_H_EFF, "h_eff")):
+        assert max_abs(be.copy_field(o), obs[key]) <= tol * np.abs(obs[key]).max(), key
+    for _ in range(5):
+        be.step(2e-14)
+        sim.step(2e-14)
+    assert max_abs(be.copy_m(), sim.m) <= (1e-12 if prec == nf.PRECISION_DOUBLE else 1e-6)
     be.close()
 
 
