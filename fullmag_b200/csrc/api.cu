@@ -381,7 +381,9 @@ bool create_impl(Backend &b, const fullmag_fdm_plan_desc *plan, const fullmag_fd
                 double scale = 0.0;
                 for (int c = 0; c < 3; ++c)
                     for (double v : spec[c]) scale = std::max(scale, std::fabs(v));
-                if (fm::octant_repad(b.KZ, b.nx, b.ny, PX, PY, b.thin, 1e-8 * scale, spec)) take_padded();
+                // only rounding may be left out (Newell spectra: 1.5e-14 of the largest entry,
+                // any grid tried); spectra with more there keep 2n and every entry
+                if (fm::octant_repad(b.KZ, b.nx, b.ny, PX, PY, b.thin, 1e-12 * scale, spec)) take_padded();
                 else b.force_stockham = true;
             }
         }

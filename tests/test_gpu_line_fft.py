@@ -7,6 +7,8 @@
 - The switches of the z and fused passes on grids padded beyond 2n (the fused y-z pass,
   which has no padding of its own, must leave them to the split kernels): fields as above,
   m after 5 Heun steps at 1e-12 and 1e-6.
+- Supplied spectra with more than rounding at a frequency where a Newell tensor is zero:
+  the field of numpy's FFT with every entry, at the FP64 field tolerance.
 - A Runge-Kutta step on either side of the cell count up to which the FP32 group kernels
   form the next stage state themselves, FP32-mixed against FP64 at 1e-5 (the tolerance
   of the FP32-mixed trajectories).
@@ -74,6 +76,28 @@ def test_switched_passes_on_padded_lengths(monkeypatch, env, cells, prec):
         sim.step(2e-14)
     assert max_abs(be.copy_m(), sim.m) <= (1e-12 if prec == nf.PRECISION_DOUBLE else 1e-6)
     be.close()
+
+
+@pytest.mark.parametrize("noise", [0.0, 4e-9])
+@pytest.mark.parametrize("cells", [(9, 15, 1), (18, 10, 1), (10, 9, 2)])
+def test_supplied_spectra_keep_every_entry(cells, noise):
+    """What a supplied tensor holds where a Newell tensor is zero counts (noise of single
+    precision, within what a plan may carry): xy at the Nyquist frequency along y."""
+    nx, ny, nz = cells
+    L = (1 if nz == 1 else 2 * nz, 2 * ny, 2 * nx)
+    spec = [s.copy() for s in nf.newell_spectra(nx, ny, nz, *D, thin_film_2d=nz == 1)]
+    xx, yy, zz, xy, xz, yz = (s.reshape(L + (2,))[..., 0] for s in spec)
+    xy[:, ny, :] += noise * max(np.abs(a).max() for a in (xx, yy, zz))
+    m = nf.random_unit_vectors(3, nx * ny * nz)
+    M = np.fft.fftn(8e5 * m.reshape(nz, ny, nx, 3), L, axes=(0, 1, 2))
+    H = -np.stack([(a * M).sum(-1) for a in (np.stack(r, -1) for r in ((xx, xy, xz), (xy, yy, yz), (xz, yz, zz)))], -1)
+    want = np.fft.ifftn(H, axes=(0, 1, 2)).real[:nz, :ny, :nx].reshape(-1)
+    plan = nf.FdmPlan(cells=cells, cell_size=D, initial_magnetization=m, saturation_magnetisation=8e5,
+                      precision=nf.PRECISION_DOUBLE, integrator=nf.HEUN, demag_spectra=spec)
+    with nf.NativeFdmBackend(plan) as be:
+        assert (be.memory_info()[1][:2] == (2 * nx, 2 * ny)) == (noise > 0.0)
+        be.refresh_observables()
+        assert max_abs(np.asarray(be.copy_field(nf.OBS_H_DEMAG)).reshape(-1), want) <= 1e-13 * np.abs(want).max()
 
 
 def _plan(cells, prec, integrator, seed=5, **kw):
