@@ -369,9 +369,10 @@ bool create_impl(Backend &b, const fullmag_fdm_plan_desc *plan, const fullmag_fd
             b.Lx = PX; b.Ly = PY;
             b.nkx = PX / 2 + 1; b.KY = PY / 2 + 1;
         };
+        // spec stays at the lengths 2n: the device brings it to the padded ones
         if (demag_src == FULLMAG_FDM_EXT_DEMAG_NEWELL) {
+            fm::newell_octant_spectra(b.nx, b.ny, b.nz, b.dx, b.dy, b.dz, b.thin, spec);
             if (!b.force_stockham) take_padded();
-            fm::newell_octant_spectra_padded(b.nx, b.ny, b.nz, b.dx, b.dy, b.dz, b.thin, b.Lx, b.Ly, 2 * b.nz, spec);
         } else if (b.projection) {
             projection_octant(b, spec);
         } else {
@@ -383,7 +384,7 @@ bool create_impl(Backend &b, const fullmag_fdm_plan_desc *plan, const fullmag_fd
                     for (double v : spec[c]) scale = std::max(scale, std::fabs(v));
                 // only rounding may be left out (Newell spectra: 1.5e-14 of the largest entry,
                 // any grid tried); spectra with more there keep 2n and every entry
-                if (fm::octant_repad(b.KZ, b.nx, b.ny, PX, PY, b.thin, 1e-12 * scale, spec)) take_padded();
+                if (fm::octant_can_pad(b.KZ, b.nx, b.ny, b.thin, 1e-12 * scale, spec)) take_padded();
                 else b.force_stockham = true;
             }
         }

@@ -24,6 +24,7 @@
 #include "demag.cuh"
 #include "demag_reg.cuh"
 #include "linefft.cuh"
+#include "repad.cuh"
 #include "demag_yz.hpp"
 #include "demag_row.hpp"
 #include "stage_vec.hpp"
@@ -1375,6 +1376,60 @@ bool backend_alloc(Backend &b) {
     return true;
 }
 
+// The tables src[c] ([plane][kx <= nx][ky <= ny], in-plane lengths 2n) brought to the
+// handle's lengths on the device (repad.cuh) and into b.spec in the passes' row layout.
+template <typename T>
+static bool upload_padded_table(Backend &b, const std::vector<double> *src, int planes, const std::vector<int> &map) {
+    const size_t in = (size_t)(b.nx + 1) * (b.ny + 1), mid = (size_t)(b.nx + 1) * b.KY, out = (size_t)b.nkx * b.KY;
+    const size_t W = map.size(), rows = (size_t)planes * b.nkx;
+    // up to 64 MB of planes at a time
+    const int P = (int)std::max<size_t>(1, std::min<size_t>(planes, (64u << 20) / ((in + mid + out) * 8)));
+    struct Temp {
+        void *p = nullptr;
+        ~Temp() { if (p) cudaFree(p); }
+    } temp;
+    if (!cuda_ok(b, cudaMalloc(&temp.p, P * (in + mid + out) * 8 + W * sizeof(int)), "cudaMalloc(tables)")) return false;
+    double *d0 = (double *)temp.p, *d1 = d0 + P * in, *d2 = d1 + P * mid;
+    int *dmap = (int *)(d2 + P * out);
+    if (!cuda_ok(b, cudaMemcpyAsync(dmap, map.data(), W * sizeof(int), cudaMemcpyHostToDevice, b.stream), "table map") ||
+        !cuda_ok(b, cudaFuncSetAttribute(k_repad, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost), "attr repad"))
+        return false;
+    auto axis = [&](const double *from, double *to, const LinePlan &p0, int L, bool odd, long long nrows, int inner) {
+        RepadArgs a{};
+        a.src = from; a.dst = to;
+        a.p0 = p0;
+        make_line_plan(L, a.p1);
+        a.n = p0.L / 2; a.odd = odd;
+        a.rows = nrows; a.inner = inner; a.st = inner;
+        a.so = (long long)(a.n + 1) * inner; a.dso = (long long)(L / 2 + 1) * inner;
+        a.lines = std::max(1, std::min(16, (100 * 1024 - L * 16) / (32 * (L + 1))));
+        const size_t smem = (size_t)16 * (L + 2 * (size_t)a.lines * (L + 1));
+        k_repad<<<(unsigned)((nrows + 2 * a.lines - 1) / (2 * a.lines)), 256, smem, b.stream>>>(a);
+    };
+    const bool oddx[6] = {false, false, false, true, true, false}, oddy[6] = {false, false, false, true, false, true};
+    for (int c = 0; c < 6; ++c) {
+        if (b.thin && c > 3) continue;  // a film's xz and yz: zero, as the arena is
+        for (int p0 = 0; p0 < planes; p0 += P) {
+            const int np = std::min(P, planes - p0);
+            if (!cuda_ok(b, cudaMemcpyAsync(d0, &src[c][p0 * in], np * in * 8, cudaMemcpyHostToDevice, b.stream), "table upload")) return false;
+            const double *at = d0;
+            if (b.Ly != 2 * b.ny) {
+                axis(at, d1, b.py, b.Ly, oddy[c], (long long)np * (b.nx + 1), 1);
+                at = d1;
+            }
+            if (b.Lx != 2 * b.nx) {
+                axis(at, d2, b.px, b.Lx, oddx[c], (long long)np * b.KY, b.KY);
+                at = d2;
+            }
+            const long long nrows = (long long)np * b.nkx;
+            k_table_rows<T><<<(unsigned)std::min<long long>((nrows * (long long)W + 255) / 256, 148LL * 16), 256, 0, b.stream>>>(
+                at, (T *)b.spec + (c * rows + (size_t)p0 * b.nkx) * W, dmap, b.KY, (int)W, nrows, oddy[c]);
+            if (!check_launch(b, "padded table")) return false;
+        }
+    }
+    return cuda_ok(b, cudaStreamSynchronize(b.stream), "padded table");
+}
+
 template <typename T>
 static bool upload_tables(Backend &b, const std::vector<double> (&spec)[6]) {
     auto tw = [&](int L, void *dst) {
@@ -1397,36 +1452,43 @@ static bool upload_tables(Backend &b, const std::vector<double> (&spec)[6]) {
         return t.empty() || cuda_ok(b, cudaMemcpy(dst, t.data(), t.size() * sizeof(cx<T>), cudaMemcpyHostToDevice), "twiddles (line)");
     };
     if (!twl(b.Lx, b.twx4) || !twl(b.Ly, b.twy4)) return false;
-    b.thin6 = false;
-    for (int c = 4; b.thin && c < 6; ++c)
+    b.thin6 = false;  // a padded film has neither
+    for (int c = 4; b.thin && b.Lx == 2 * b.nx && b.Ly == 2 * b.ny && c < 6; ++c)
         for (double v : spec[c]) b.thin6 = b.thin6 || v != 0.0;
-    // the octant, or for the direct z convolution its z-inverse table (nz planes)
+    // the octant, or for the direct z convolution its z-inverse table (nz planes); both at
+    // the in-plane lengths 2n
+    const int KX0 = b.nx + 1, KY0 = b.ny + 1;
     std::vector<double> zt[6];
-    if (b.zdirect) octant_to_z_direct(b.nkx, b.KY, b.nz, spec, zt);
+    if (b.zdirect) octant_to_z_direct(KX0, KY0, b.nz, spec, zt);
     const auto &src = b.zdirect ? zt : spec;
-    const size_t plane = (size_t)(b.zdirect ? b.nz : b.KZ) * b.nkx * b.KY;
-    std::vector<T> host;
+    const int planes = b.zdirect ? b.nz : b.KZ;
+    // the passes' table rows: place i holds entry |map[i]| - 1 of the ky row (map[i] < 0: the
+    // mirrored one, negated for the components odd in y), or 0 where map[i] = 0
+    std::vector<int> map;
     if (b.use_zdw && b.zdw_win) {
-        // rows of zdw_kyp values (16-byte windows of k_zdw), the padding zero
-        const size_t kyp = (size_t)b.zdw_kyp, rows = (size_t)b.nz * b.nkx;
-        host.assign(6 * rows * kyp, T(0));
-        for (int c = 0; c < 6; ++c)
-            for (size_t r = 0; r < rows; ++r)
-                for (int ky = 0; ky < b.KY; ++ky) host[(c * rows + r) * kyp + ky] = (T)src[c][r * b.KY + ky];
+        map.assign((size_t)b.zdw_kyp, 0);  // 16-byte windows of k_zdw
+        for (int i = 0; i < b.KY; ++i) map[i] = i + 1;
     } else if (b.use_yzy) {
-        const size_t row = (size_t)(sizeof(T) == 4 ? yzy_table_values_f32(b.Ly) : yzy_table_values_f64(b.Ly)), rows = (size_t)b.nz * b.nkx;
-        host.assign(6 * rows * row, T(0));
-        for (int c = 0; c < 6; ++c)
-            for (size_t r = 0; r < rows; ++r) {
-                const double *from = &src[c][r * b.KY], sign = (c == 3 || c == 5) ? -1.0 : 1.0;  // xy, yz odd in y
-                T *to = &host[(c * rows + r) * row];
-                if constexpr (sizeof(T) == 4) yzy_table_row_f32(b.Ly, from, sign, to);
-                else yzy_table_row_f64(b.Ly, from, sign, to);
-            }
+        std::vector<double> entry(b.KY);
+        for (int i = 0; i < b.KY; ++i) entry[i] = i + 1;
+        std::vector<T> row((size_t)(sizeof(T) == 4 ? yzy_table_values_f32(b.Ly) : yzy_table_values_f64(b.Ly)));
+        if constexpr (sizeof(T) == 4) yzy_table_row_f32(b.Ly, entry.data(), -1.0, row.data());
+        else yzy_table_row_f64(b.Ly, entry.data(), -1.0, row.data());
+        map.assign(row.begin(), row.end());
     } else {
-        host.resize(6 * plane);
-        for (int c = 0; c < 6; ++c)
-            for (size_t o = 0; o < plane; ++o) host[c * plane + o] = (T)src[c][o];
+        map.resize(b.KY);
+        for (int i = 0; i < b.KY; ++i) map[i] = i + 1;
+    }
+    if (b.Lx != 2 * b.nx || b.Ly != 2 * b.ny) return upload_padded_table<T>(b, src, planes, map);
+    const size_t W = map.size(), rows = (size_t)planes * b.nkx;
+    std::vector<T> host(6 * rows * W);
+    for (int c = 0; c < 6; ++c) {
+        const double mirror = (c == 3 || c == 5) ? -1.0 : 1.0;  // xy, yz odd in y
+        for (size_t r = 0; r < rows; ++r)
+            for (size_t i = 0; i < W; ++i) {
+                const int e = map[i];
+                host[(c * rows + r) * W + i] = e == 0 ? T(0) : e > 0 ? (T)src[c][r * b.KY + e - 1] : (T)(mirror * src[c][r * b.KY - e - 1]);
+            }
     }
     return cuda_ok(b, cudaMemcpy(b.spec, host.data(), host.size() * sizeof(T), cudaMemcpyHostToDevice), "spectra upload");
 }

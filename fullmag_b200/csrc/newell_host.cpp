@@ -303,50 +303,22 @@ void octant_to_z_direct(int nkx, int KY, int nz, const std::vector<double> (&spe
     }
 }
 
-// One axis of octant_repad: src (n + 1 frequencies of length 2n) -> dst (L / 2 + 1).
-static void axis_repad(const double *src, double *dst, size_t n, size_t L, bool odd, const HostFft &fft2n,
-                       const HostFft &fftL) {
-    // S(k) continued evenly or oddly to 2n frequencies
-    std::vector<std::complex<double>> F(2 * n);
-    for (size_t k = 0; k <= n; ++k) F[k] = (odd && (k == 0 || k == n)) ? 0.0 : src[k];
-    for (size_t k = 1; k < n; ++k) F[2 * n - k] = odd ? -src[k] : src[k];
-    fft2n.run(F.data());
-    // even: f(d) = Re F / 2n; odd: S = 2 sum f sin, so f(d) = (1/n) sum_k S sin = -Im F / 2n
-    std::vector<double> f(n);
-    for (size_t d = 0; d < n; ++d) f[d] = (odd ? -F[d].imag() : F[d].real()) / (double)(2 * n);
-    axis_transform(f.data(), dst, n, L, odd, fftL);
-}
-
-bool octant_repad(int KZ, int nx, int ny, int Lx, int Ly, bool thin2d, double tol,
-                  std::vector<double> (&spec)[6]) {
-    const size_t KX0 = nx + 1, KY0 = ny + 1, KX = Lx / 2 + 1, KY = Ly / 2 + 1;
+bool octant_can_pad(int KZ, int nx, int ny, bool thin2d, double tol, const std::vector<double> (&spec)[6]) {
+    const size_t KX = nx + 1, KY = ny + 1;
     const bool oddx[6] = {false, false, false, true, true, false};
     const bool oddy[6] = {false, false, false, true, false, true};
-    for (int c = 0; c < 6; ++c)
+    for (int c = 3; c < 6; ++c) {
+        const bool all = thin2d && oddx[c] != oddy[c];  // a film's xz and yz are zero
         for (int kz = 0; kz < KZ; ++kz)
-            for (size_t kx = 0; kx < KX0; ++kx)
-                for (size_t ky = 0; ky < KY0; ++ky) {
-                    const bool none = thin2d && oddx[c] != oddy[c];  // a film's xz and yz are zero
-                    const bool edge = none || (oddx[c] && (kx == 0 || kx == KX0 - 1)) || (oddy[c] && (ky == 0 || ky == KY0 - 1));
-                    if (edge && std::fabs(spec[c][(kz * KX0 + kx) * KY0 + ky]) > tol) return false;
+            for (size_t kx = 0; kx < KX; ++kx) {
+                const double *row = &spec[c][(kz * KX + kx) * KY];
+                if (all || (oddx[c] && (kx == 0 || kx == KX - 1))) {
+                    for (size_t ky = 0; ky < KY; ++ky)
+                        if (!(std::fabs(row[ky]) <= tol)) return false;
+                } else if (oddy[c] && !(std::fabs(row[0]) <= tol && std::fabs(row[KY - 1]) <= tol)) {
+                    return false;
                 }
-    HostFft fx0((size_t)2 * nx), fy0((size_t)2 * ny), fx((size_t)Lx), fy((size_t)Ly);
-    for (int c = 0; c < 6; ++c) {
-        std::vector<double> out((size_t)KZ * KX * KY, 0.0);
-        if (!(thin2d && oddx[c] != oddy[c])) {
-            std::vector<double> A((size_t)KZ * KX0 * KY);  // y axis: [kz][kx0][ky]
-            parallel_for((size_t)KZ * KX0, [&](size_t row) {
-                axis_repad(&spec[c][row * KY0], &A[row * KY], ny, Ly, oddy[c], fy0, fy);
-            });
-            parallel_for((size_t)KZ * KY, [&](size_t row) {
-                const size_t kz = row / KY, ky = row % KY;
-                std::vector<double> src(KX0), dst(KX);
-                for (size_t kx = 0; kx < KX0; ++kx) src[kx] = A[(kz * KX0 + kx) * KY + ky];
-                axis_repad(src.data(), dst.data(), nx, Lx, oddx[c], fx0, fx);
-                for (size_t kx = 0; kx < KX; ++kx) out[(kz * KX + kx) * KY + ky] = dst[kx];
-            });
-        }
-        spec[c].swap(out);
+            }
     }
     return true;
 }

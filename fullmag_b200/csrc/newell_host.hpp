@@ -36,13 +36,10 @@ void newell_octant_spectra_padded(int nx, int ny, int nz, double dx, double dy, 
 void octant_to_z_direct(int nkx, int KY, int nz, const std::vector<double> (&spec)[6],
                         std::vector<double> (&out)[6], int h = 0);
 
-// In-plane lengths of an octant spectrum [kz < KZ][kx <= nx][ky <= ny] of lengths
-// (2 nx, 2 ny) changed to even (Lx, Ly) with Lx >= 2 nx, Ly >= 2 ny: per axis back to
-// the offsets |d| < n (the wrapped entry d = n reaches no physical cell) and forward
-// at the new length.  thin2d: a film's (xz and yz zero).  False, with spec unchanged,
-// when a component odd along an axis has more than tol at frequency 0 or Nyquist there,
-// or a film's xz or yz anywhere: no such kernel has that spectrum.
-bool octant_repad(int KZ, int nx, int ny, int Lx, int Ly, bool thin2d, double tol,
-                  std::vector<double> (&spec)[6]);
+// Whether the in-plane lengths (2 nx, 2 ny) of an octant spectrum [kz < KZ][kx <= nx]
+// [ky <= ny] can be changed (repad.cuh) without losing anything: not when a component
+// odd along an axis has more than tol at frequency 0 or Nyquist there, or a film's
+// (thin2d) xz or yz anywhere, for no longer kernel has that spectrum.
+bool octant_can_pad(int KZ, int nx, int ny, bool thin2d, double tol, const std::vector<double> (&spec)[6]);
 
 }  // namespace fm
