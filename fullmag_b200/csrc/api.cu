@@ -360,8 +360,9 @@ bool create_impl(Backend &b, const fullmag_fdm_plan_desc *plan, const fullmag_fd
         // the projection fallback, which has Nyquist entries of its own, keep 2n
         const int PX = fm::line_length(b.Lx), PY = fm::line_length(b.Ly);
         const bool repad = PX != b.Lx || PY != b.Ly;
-        // Spectra and tensor in bytes at the padded lengths, up to twice those at 2n: above
-        // 64 GiB a grid keeps 2n, so that the largest grids fit as they would at 2n.
+        // Spectra and tensor in bytes at the padded lengths, which are up to 1.5 times 2n (1.9
+        // below 64), and the bytes up to 2.1 times those at 2n: above 64 GiB a grid keeps 2n,
+        // so that the largest grids fit as they would at 2n.
         const double padded_bytes = (double)(PX / 2 + 1) * b.nz * (b.precision == FULLMAG_FDM_PRECISION_DOUBLE ? 8.0 : 4.0) *
                                     (6.0 * b.ny + 6.0 * PY + 6.0 * (PY / 2 + 1));
         if (repad && (b.projection || padded_bytes > 64.0 * 1024 * 1024 * 1024)) b.force_stockham = true;

@@ -187,6 +187,9 @@ __device__ __forceinline__ void lf_dft(C (&v)[R]) { lf_dft_at<R, 0, INV, R>(v); 
 // - elsewhere 8 to 12 values per thread against 16 to 24: 300 x 180 x 5 masked FP32 143 ->
 //   116 us per Heun step, 256 x 256 FP32 54 -> 37, 90 x 90 x 4 FP32 56 -> 42, 384 x 384 x 8
 //   FP64 528 -> 430; 256 x 256 x 8 FP32 105 -> 101.
+// - 3072: without it 1025 to 1536 cells went to 4096. Heun step and handle at 4096 and here:
+//   1050 x 1050 FP32 510 -> 450 us, 272 -> 215 MB, FP64 976 -> 732 us; 1050 x 1050 x 4 FP32
+//   2329 -> 1643 us, 1994 -> 1369 MB (at 2n = 2100: 5431 us, 928 MB).
 template <typename T, int L> struct LfPlan;
 #define FM_LF_PLAN(L_, R0_, R1_, R2_, G_) \
     template <typename T> struct LfPlan<T, L_> { static constexpr int L = L_, R0 = R0_, R1 = R1_, R2 = R2_, G = G_; }
@@ -206,13 +209,14 @@ FM_LF_PLAN(768, 12, 8, 8, 64);
 FM_LF_PLAN(1024, 16, 8, 8, 64);
 FM_LF_PLAN(1536, 24, 8, 8, 64);
 FM_LF_PLAN(2048, 16, 16, 8, 128);
+FM_LF_PLAN(3072, 12, 16, 16, 256);
 FM_LF_PLAN(4096, 16, 16, 16, 256);
 #undef FM_LF_PLAN
 template <> struct LfPlan<float, 256> { static constexpr int L = 256, R0 = 16, R1 = 16, R2 = 1, G = 16; };
 template <> struct LfPlan<float, 1024> { static constexpr int L = 1024, R0 = 32, R1 = 32, R2 = 1, G = 32; };
 
 // The lengths above; any length >= 2n - 1 gives the linear convolution of n cells.
-constexpr int kLfLengths[] = {2, 4, 8, 16, 32, 64, 96, 128, 192, 256, 384, 512, 768, 1024, 1536, 2048, 4096};
+constexpr int kLfLengths[] = {2, 4, 8, 16, 32, 64, 96, 128, 192, 256, 384, 512, 768, 1024, 1536, 2048, 3072, 4096};
 // the smallest of them >= v, or 0
 inline int line_length(int v) {
     for (int L : kLfLengths)
@@ -240,6 +244,7 @@ inline bool with_line(int L, F &&f) {
         case 1024: f(LfIC<1024>{}); return true;
         case 1536: f(LfIC<1536>{}); return true;
         case 2048: f(LfIC<2048>{}); return true;
+        case 3072: f(LfIC<3072>{}); return true;
         case 4096: f(LfIC<4096>{}); return true;
         default: return false;
     }

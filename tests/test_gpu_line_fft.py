@@ -32,10 +32,10 @@ D = (2e-9, 2.5e-9, 3e-9)
 H = (1e4, -2e4, 3e3)
 
 
-# (nx, ny, nz): 2n -> 16, 32, 64, 96, 128, 192, 256, 384, 512, 768, 1024, 1536, 2048 along x or y
+# (nx, ny, nz): 2n -> 16, 32, 64, 96, 128, 192, 256, 384, 512, 768, 1024, 1536, 2048, 3072 along x or y
 _CELLS = [(5, 7, 1), (9, 15, 3), (20, 36, 1), (48, 36, 2), (49, 64, 1), (70, 96, 2), (100, 7, 3),
           (128, 25, 1), (135, 192, 1), (200, 245, 1), (3, 300, 2), (384, 9, 1), (10, 490, 1), (525, 4, 2),
-          (6, 625, 1), (800, 5, 1), (4, 1000, 2),
+          (6, 625, 1), (800, 5, 1), (4, 1000, 2), (1050, 5, 1), (3, 1280, 1), (7, 1125, 2), (1536, 2, 2),
           # the z tables' layouts: k_zdw's windows and elements, the fused plane pass's slots, the z FFT
           (20, 150, 9), (18, 36, 10), (70, 128, 3), (32, 100, 4), (49, 25, 12)]
 
