@@ -366,6 +366,14 @@ bool create_impl(Backend &b, const fullmag_fdm_plan_desc *plan, const fullmag_fd
         const double padded_bytes = (double)(PX / 2 + 1) * b.nz * (b.precision == FULLMAG_FDM_PRECISION_DOUBLE ? 8.0 : 4.0) *
                                     (6.0 * b.ny + 6.0 * PY + 6.0 * (PY / 2 + 1));
         if (repad && (b.projection || padded_bytes > 64.0 * 1024 * 1024 * 1024)) b.force_stockham = true;
+        // The shared-memory z FFT transforms every padded (kx, ky) column, which can cost more
+        // than the line FFTs of x and y gain. us per Heun step at 2n and padded, with the
+        // columns' ratio: FP64 280 x 140 x 20 1145 / 1289 (1.88), 270 x 270 x 12 1346 / 1486
+        // (2.02), 540 x 300 x 12 3014 / 3035 (1.82), 600 x 400 x 10 3381 / 3031 (1.64), 160 x 160
+        // x 16 560 / 497 (1.44); FP32 135 x 270 x 50 2067 / 2292 (2.02), 75 x 75 x 75 576 / 552
+        // (1.64). Small grids gain through their latency at any ratio (70 x 70 x 20 FP64 237 / 201).
+        const double columns = (double)(PX / 2 + 1) * PY / ((double)b.nkx * b.Ly);
+        if (repad && fm::z_fft_shared(b) && columns > 1.7 && b.n > (1LL << 17)) b.force_stockham = true;
         auto take_padded = [&] {
             b.Lx = PX; b.Ly = PY;
             b.nkx = PX / 2 + 1; b.KY = PY / 2 + 1;

@@ -63,6 +63,18 @@ static bool env_is(const char *name, const char *value) {
 // ---------------------------------------------------------------------------
 // helpers
 // ---------------------------------------------------------------------------
+// z passes of the line-FFT path: a direct sum up to nz = 8 (FULLMAG_FDM_ZCONV=fft: none),
+// the wide direct sum (zdw_wanted), the register FFT of short powers of two, else the
+// shared-memory FFT
+static bool z_direct_small(const Backend &b) {
+    return !b.thin && b.nz <= 8 && !b.want_yz && !env_is("FULLMAG_FDM_ZCONV", "fft");
+}
+bool z_fft_shared(const Backend &b) {
+    const bool dbl = b.precision == FULLMAG_FDM_PRECISION_DOUBLE;
+    if (b.thin || zdw_wanted(b, !dbl) || z_direct_small(b)) return false;
+    return !(is_pow2(b.Lz) && b.Lz <= (dbl ? 16 : 32));
+}
+
 bool cuda_ok(Backend &b, cudaError_t e, const char *what) {
     if (e == cudaSuccess) return true;
     char buf[512];
@@ -210,8 +222,8 @@ struct Impl {
         const bool dbl = sizeof(T) == 8;
         const bool zdw = zdw_wanted(b, !dbl);
         b.use_zdw = false;
-        b.zdirect = zdw || (!b.thin && b.nz <= 8 && !b.want_yz && !env_is("FULLMAG_FDM_ZCONV", "fft"));
-        b.zreg = !b.thin && !b.zdirect && is_pow2(b.Lz) && b.Lz <= (dbl ? 16 : 32);
+        b.zdirect = zdw || z_direct_small(b);
+        b.zreg = !b.thin && !b.zdirect && !z_fft_shared(b);
         if (!cuda_ok(b, line_setup<T>(b.line, b.Lx, b.Ly, b.thin, b.ny, b.nz, b.nkx), "line FFT setup")) return false;
         b.use_yz = false;
         // the fused y-z pass folds a line at ny = Ly / 2 and writes all Ly / 2 outputs into

@@ -22,6 +22,7 @@ struct Snapshot {
 
 bool cuda_ok(Backend &b, cudaError_t e, const char *what);
 bool make_line_plan(int L, LinePlan &p);
+bool z_fft_shared(const Backend &b);  // the z pass is the shared-memory z FFT
 bool backend_alloc(Backend &b);
 bool backend_configure(Backend &b);
 bool backend_upload_tables(Backend &b, const std::vector<double> (&spec)[6]);

@@ -9,6 +9,8 @@
   m after 5 Heun steps at 1e-12 and 1e-6.
 - Supplied spectra with more than rounding at a frequency where a Newell tensor is zero:
   the field of numpy's FFT with every entry, at the FP64 field tolerance.
+- Which grids are padded where the z pass is the shared-memory FFT, and their fields
+  against those at 2n (bit for bit where 2n is kept).
 - A Runge-Kutta step on either side of the cell count up to which the FP32 group kernels
   form the next stage state themselves, FP32-mixed against FP64 at 1e-5 (the tolerance
   of the FP32-mixed trajectories).
@@ -100,6 +102,22 @@ def test_supplied_spectra_keep_every_entry(cells, noise):
         assert (be.memory_info()[1][:2] == (2 * nx, 2 * ny)) == (noise > 0.0)
         be.refresh_observables()
         assert max_abs(np.asarray(be.copy_field(nf.OBS_H_DEMAG)).reshape(-1), want) <= 1e-13 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("prec", [nf.PRECISION_DOUBLE, nf.PRECISION_SINGLE])
+@pytest.mark.parametrize("cells,padded", [((70, 70, 32), False), ((70, 70, 24), True), ((135, 135, 8), True), ((63, 63, 40), True)])
+def test_padding_only_where_the_z_fft_can_bear_it(monkeypatch, cells, padded, prec):
+    """Above 2^17 cells a grid with the shared-memory z FFT and over 1.7 times the columns keeps 2n."""
+    kw = dict(cells=cells, cell_size=D, precision=prec, integrator=nf.HEUN, demag_source=nf.DEMAG_NEWELL, damping=0.1,
+              initial_magnetization=nf.random_unit_vectors(5, cells[0] * cells[1] * cells[2]))
+    fields = []
+    for fft in ("line", "stockham"):
+        monkeypatch.setenv("FULLMAG_FDM_FFT", fft)
+        with nf.NativeFdmBackend(nf.FdmPlan(**kw)) as be:
+            assert (be.memory_info()[1][0] > 2 * cells[0]) == (padded and fft == "line")
+            fields.append(np.asarray(be.copy_field(nf.OBS_H_DEMAG), dtype=np.float64))
+    tol = 1e-13 if prec == nf.PRECISION_DOUBLE else 2e-6
+    assert max_abs(*fields) <= (tol * np.abs(fields[1]).max() if padded else 0.0)
 
 
 def _plan(cells, prec, integrator, seed=5, **kw):
