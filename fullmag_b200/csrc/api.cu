@@ -362,7 +362,8 @@ bool create_impl(Backend &b, const fullmag_fdm_plan_desc *plan, const fullmag_fd
         const bool repad = PX != b.Lx || PY != b.Ly;
         // Spectra and tensor in bytes at the padded lengths, which are up to 1.5 times 2n (1.9
         // below 64), and the bytes up to 2.1 times those at 2n: above 64 GiB a grid keeps 2n,
-        // so that the largest grids fit as they would at 2n.
+        // so that the largest grids fit as they would at 2n; where the memory is short all the
+        // same, backend_retry_lean takes 2n.
         const double padded_bytes = (double)(PX / 2 + 1) * b.nz * (b.precision == FULLMAG_FDM_PRECISION_DOUBLE ? 8.0 : 4.0) *
                                     (6.0 * b.ny + 6.0 * PY + 6.0 * (PY / 2 + 1));
         if (repad && (b.projection || padded_bytes > 64.0 * 1024 * 1024 * 1024)) b.force_stockham = true;
@@ -401,9 +402,8 @@ bool create_impl(Backend &b, const fullmag_fdm_plan_desc *plan, const fullmag_fd
 
     if (!select_device(b)) return false;
     if (!fm::cuda_ok(b, cudaStreamCreateWithFlags(&b.stream, cudaStreamNonBlocking), "cudaStreamCreate")) return false;
-    if (!fm::backend_alloc(b)) return false;
-    if (!fm::backend_configure(b)) return false;
-    if (!fm::backend_upload_tables(b, spec)) return false;
+    auto place = [&] { return fm::backend_alloc(b) && fm::backend_configure(b) && fm::backend_upload_tables(b, spec); };
+    if (!place() && !(fm::backend_retry_lean(b) && place())) return false;
     if (b.has_mask && !fm::cuda_ok(b, cudaMemcpy(b.d_mask, plan->active_mask, b.n, cudaMemcpyHostToDevice), "upload mask")) return false;
     if (b.has_regions) {
         if (!fm::cuda_ok(b, cudaMemcpy(b.d_region, plan->region_mask, b.n * 4, cudaMemcpyHostToDevice), "upload regions")) return false;

@@ -80,6 +80,10 @@ bool cuda_ok(Backend &b, cudaError_t e, const char *what) {
     char buf[512];
     std::snprintf(buf, sizeof(buf), "CUDA error in %s: %s (%d)", what, cudaGetErrorString(e), (int)e);
     b.last_error = buf;
+    if (e == cudaErrorMemoryAllocation) {
+        b.out_of_memory = true;
+        cudaGetLastError();  // not sticky: nothing later may report it
+    }
     return false;
 }
 
@@ -251,7 +255,8 @@ struct Impl {
             ok &= zdw_configure(b);
             if (ok && !b.use_zdw) { b.last_error = "direct z convolution: no resident block"; return false; }
         }
-        if (ok && b.zdirect && !b.use_zdw) ok &= yzy_configure<T>(b);
+        const size_t yzy_values = (size_t)b.nz * (dbl ? yzy_table_values_f64(b.Ly) : yzy_table_values_f32(b.Ly));
+        if (ok && b.zdirect && !b.use_zdw && !(b.lean && yzy_values > (size_t)b.KZ * b.KY)) ok &= yzy_configure<T>(b);
         return ok;
     }
 
@@ -361,7 +366,7 @@ struct Impl {
         // with the group kernels, whose registers then allow 16 warps per SM instead of 20,
         // up to 2^18 cells (128 x 128 FP32 DP45 133 -> 124 us, 256 x 256 x 4 252 -> 249, but
         // 300 x 180 x 5 masked 479 -> 486 and 1024 x 512 x 16 masked 242 -> 290 us per stage)
-        b.chain = !b.stage_vec || b.n <= (1LL << 18);
+        b.chain = !b.lean && (!b.stage_vec || b.n <= (1LL << 18));
         if (!b.stage_plain) return true;
         b.stage_ring = !env_is("FULLMAG_FDM_STAGE", "plain");
         if (!b.stage_ring) return true;
@@ -390,9 +395,9 @@ struct Impl {
             return true;
         }
         b.use_reg = false;
-        b.zdirect = false;
-        b.use_yzy = false;
-        b.use_zdw = false;
+        b.zdirect = b.zreg = false;
+        b.use_yz = b.use_yzy = b.use_zdw = false;
+        b.use_row = b.use_graphs = false;
         const int budget = 100 * 1024;
         const int sz = (int)sizeof(C);
         auto lines_for = [&](int ld, int L, int per_line_mult, int maxl) {
@@ -835,6 +840,13 @@ struct Impl {
         return true;
     }
 
+    // The accepted state's buffer becomes m, m's the stage's (both stage states where the
+    // handle has one).
+    static void accept(Backend &b, void *&stage) {
+        std::swap(b.m, stage);
+        if (b.lean) b.mstage = b.mstage2 = stage;
+    }
+
     // One accepted DP45 step (lib.rs:1412-1568).
     static bool dp45(Backend &b, double dt_in, fullmag_fdm_step_stats *st) {
         b.pred_valid = false;  // the stages below use mstage
@@ -892,7 +904,7 @@ struct Impl {
             if (!launched || !check_launch(b, "dp45 last stage") || !read_stats(b)) return false;
             const double err = std::sqrt(b.h_out[Q_ERR2]);
             if (err <= b.max_error || dt <= b.dt_min) {
-                std::swap(b.m, b.mstage2);
+                accept(b, b.mstage2);
                 b.hd_stale = false;  // the last evaluation was at the accepted state
                 std::swap(k[0], k[6]);  // FSAL: k7 is the next step's k1
                 b.time += dt;
@@ -992,7 +1004,7 @@ struct Impl {
             if (!launched || !check_launch(b, "rk23 last stage") || !read_stats(b)) return false;
             const double err = std::sqrt(b.h_out[Q_ERR2]);
             if (err <= b.max_error || dt <= b.dt_min) {
-                std::swap(b.m, b.mstage);
+                accept(b, b.mstage);
                 b.hd_stale = false;  // the last evaluation was at the accepted state
                 std::swap(k[0], k[3]);
                 b.time += dt;
@@ -1314,7 +1326,8 @@ bool backend_alloc(Backend &b) {
                                                                    : 2;
     items.push_back({&b.m, vec});
     items.push_back({&b.mstage, vec});
-    if (nk == 4 || nk == 7) items.push_back({&b.mstage2, vec});  // RK4, RK23, DP45
+    const bool stages2 = nk == 4 || nk == 7;  // RK4, RK23, DP45
+    if (stages2 && !b.lean) items.push_back({&b.mstage2, vec});
     items.push_back({&b.hd, vec});
     items.push_back({&b.hex, vec});
     items.push_back({&b.heff, vec});
@@ -1330,8 +1343,11 @@ bool backend_alloc(Backend &b) {
         items.push_back({&b.s1, (size_t)3 * b.nz * b.nkx * b.ny * cs});
         if (!b.thin) items.push_back({&b.s2, (size_t)3 * b.nz * b.nkx * b.Ly * cs});
         // the octant, or a direct z table: nz planes of KY values, or of the fused pass's row
-        items.push_back({&b.spec, 6 * b.nkx * b.scalar *
-                                      std::max((size_t)b.KZ * b.KY, b.thin ? 0 : (size_t)b.nz * (dbl ? yzy_table_values_f64(b.Ly) : yzy_table_values_f32(b.Ly)))});
+        // (FP64: on request only)
+        size_t table = (size_t)b.KZ * b.KY;
+        if (!b.thin && !b.lean && (!dbl || std::getenv("FULLMAG_FDM_YZY_P")))
+            table = std::max(table, (size_t)b.nz * (dbl ? yzy_table_values_f64(b.Ly) : yzy_table_values_f32(b.Ly)));
+        items.push_back({&b.spec, 6 * b.nkx * b.scalar * table});
     }
     items.push_back({&b.staging, (size_t)3 * b.n * sizeof(double)});
     if (b.has_mask) items.push_back({(void **)&b.d_mask, (size_t)b.n});
@@ -1379,6 +1395,7 @@ bool backend_alloc(Backend &b) {
         *it.p = p;
         p += (it.bytes + 255) / 256 * 256;
     }
+    if (stages2 && b.lean) b.mstage2 = b.mstage;
     if (!cuda_ok(b, cudaMemsetAsync(b.arena, 0, total, b.stream), "arena memset")) return false;
     // step statistics: the last block of a reducing kernel writes them straight
     // into this mapped pinned buffer, so a step ends with a stream sync, no copy
@@ -1754,6 +1771,25 @@ void snapshot_free(Snapshot &s) {
     if (s.dev) cudaFree(s.dev);
     if (s.host) cudaFreeHost(s.host);
     s = Snapshot{};
+}
+
+bool backend_retry_lean(Backend &b) {
+    const bool padded = b.enable_demag && (b.Lx != 2 * b.nx || b.Ly != 2 * b.ny);
+    if (!b.out_of_memory || b.lean || !(padded || b.integrator == FULLMAG_FDM_INTEGRATOR_RK4 || adaptive(b))) return false;
+    if (b.stream) cudaStreamSynchronize(b.stream);
+    if (b.arena) cudaFree(b.arena);
+    b.arena = nullptr;
+    if (b.h_out) cudaFreeHost(b.h_out);
+    b.h_out = nullptr;
+    b.out_of_memory = false;
+    b.last_error.clear();
+    b.lean = true;
+    if (padded) {
+        b.force_stockham = true;
+        b.Lx = 2 * b.nx; b.Ly = 2 * b.ny;
+        b.nkx = b.nx + 1; b.KY = b.ny + 1;
+    }
+    return true;
 }
 
 void backend_free(Backend &b) {

@@ -69,7 +69,7 @@ struct Backend {
     double adj_t_final = 0.0;
     uint64_t adj_step_final = 0;
     bool adj_ready = false;
-    bool pred_valid = false;      // mstage holds normalize(m + k1 pred_dt) (Heun's next predictor)
+    bool pred_valid = false;      // mstage holds normalize(m + k1 pred_dt): Heun's next predictor, RK4's next first stage
     double pred_dt = 0.0;
     int abm_startup = 0;          // ABM3 start-up steps done (0..3)
     double abm_last_dt = 0.0;     // dt of the last ABM3 step
@@ -142,7 +142,9 @@ struct Backend {
     bool info_valid = false;
     std::string last_error;
     std::string err_buf;
-    void *mstage2 = nullptr;  // the other stage state of the RK integrators
+    void *mstage2 = nullptr;  // the other stage state of the RK integrators (lean: mstage)
+    bool lean = false;        // memory was short: lengths 2n, one stage state
+    bool out_of_memory = false;  // an allocation failed for want of memory
     // a step's launches as a CUDA graph, per (kind, dt, statistics, buffers' roles): small
     // grids, whose kernels are shorter than the time to launch them
     static constexpr int kStepBuffers = 10;  // m, mstage, mstage2, k[0..6]

@@ -25,6 +25,10 @@ bool make_line_plan(int L, LinePlan &p);
 bool z_fft_shared(const Backend &b);  // the z pass is the shared-memory z FFT
 bool backend_alloc(Backend &b);
 bool backend_configure(Backend &b);
+// After a handle's memory could not be had: the handle made ready for a second try with
+// the memory it would need without padding (lengths 2n, one stage state).  False when
+// the failure was another, or nothing can be saved.
+bool backend_retry_lean(Backend &b);
 bool backend_upload_tables(Backend &b, const std::vector<double> (&spec)[6]);
 bool backend_upload_m_f64(Backend &b, const double *m, uint64_t len);
 bool backend_upload_m_f32(Backend &b, const float *m, uint64_t len);

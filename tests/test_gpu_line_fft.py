@@ -18,6 +18,8 @@
   timing on), bit for bit, through dt changes.
 - A film's tensor with all six components (random octants) against numpy's FFT at the
   FP64 field tolerance.
+- Handles created where the device memory is short (the rest held by torch), against the
+  same steps with memory enough, at 1e-12.
 - A handle with small blocks created after one with large blocks leaves its launches valid.
 """
 import ctypes as C
@@ -158,6 +160,39 @@ def test_step_graphs_equal_single_launches(cells, prec, integrator):
         b.step_n(1e-14, 6)
         for o in (nf.OBS_M, nf.OBS_H_DEMAG, nf.OBS_H_EFF):
             assert np.array_equal(a.copy_field(o), b.copy_field(o)), o
+
+
+@pytest.mark.parametrize("cells,integrator", [((525, 270, 4), nf.HEUN), ((525, 270, 4), nf.RK4),
+                                              ((512, 512, 8), nf.RK4), ((512, 512, 8), nf.DP45), ((512, 512, 8), nf.RK23)])
+def test_handle_that_fits_only_without_padding(monkeypatch, cells, integrator):
+    """Where the device lacks the memory of padded lengths and a second stage state, a handle
+    is created without them and takes the same steps."""
+    import torch
+
+    def run():
+        with nf.NativeFdmBackend(_plan(cells, nf.PRECISION_DOUBLE, integrator)) as be:
+            for _ in range(2):
+                be.step(2e-14)
+            return be.copy_m(), *be.memory_info()
+
+    monkeypatch.setenv("FULLMAG_FDM_FFT", "stockham")
+    least = run()[1]
+    if integrator != nf.HEUN:
+        least -= 3 * 8 * cells[0] * cells[1] * cells[2]
+    monkeypatch.delenv("FULLMAG_FDM_FFT")
+    want, most, _ = run()
+    assert least < most
+    room, held = (least + most) // 2, []
+    torch.cuda.empty_cache()
+    while (free := torch.cuda.mem_get_info()[0] - room) > (1 << 21):
+        held.append(torch.empty(min(free, 8 << 30) >> 21 << 21, dtype=torch.uint8, device="cuda"))
+    try:
+        got, nbytes, dims = run()
+    finally:
+        held.clear()
+        torch.cuda.empty_cache()
+    assert nbytes < room and dims[:2] == (2 * cells[0], 2 * cells[1])
+    assert max_abs(got, want) <= 1e-12
 
 
 def test_small_handle_does_not_limit_a_large_one():
