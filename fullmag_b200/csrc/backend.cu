@@ -1396,7 +1396,10 @@ bool backend_alloc(Backend &b) {
         p += (it.bytes + 255) / 256 * 256;
     }
     if (stages2 && b.lean) b.mstage2 = b.mstage;
-    if (!cuda_ok(b, cudaMemsetAsync(b.arena, 0, total, b.stream), "arena memset")) return false;
+    // the tables that follow are copied on the legacy stream, which the handle's
+    // non-blocking one is not ordered with
+    if (!cuda_ok(b, cudaMemsetAsync(b.arena, 0, total, b.stream), "arena memset") ||
+        !cuda_ok(b, cudaStreamSynchronize(b.stream), "arena memset")) return false;
     // step statistics: the last block of a reducing kernel writes them straight
     // into this mapped pinned buffer, so a step ends with a stream sync, no copy
     if (!cuda_ok(b, cudaHostAlloc((void **)&b.h_out, NQ * sizeof(double) + 64, cudaHostAllocMapped), "cudaHostAlloc(stats)"))
