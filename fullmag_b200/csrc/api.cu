@@ -711,6 +711,12 @@ int fullmag_fdm_backend_memory_info(fullmag_fdm_backend *h, uint64_t *bytes, uin
     return FULLMAG_FDM_OK;
 }
 
+int fullmag_fdm_backend_graph_launches(fullmag_fdm_backend *h, uint64_t *out) {
+    if (!h || !out) return FULLMAG_FDM_ERR_INVALID;
+    *out = h->b.graph_launches;
+    return FULLMAG_FDM_OK;
+}
+
 int fullmag_fdm_backend_get_stream(fullmag_fdm_backend *h, void **out) {
     if (!h || !out) return FULLMAG_FDM_ERR_INVALID;
     *out = (void *)h->b.stream;

@@ -793,6 +793,7 @@ struct Impl {
                 return body();
             }
         }
+        ++b.graph_launches;
         return cuda_ok(b, cudaGraphLaunch(g->exec, b.stream), "step graph");
     }
 

@@ -158,6 +158,7 @@ struct Backend {
     static constexpr int kStepGraphs = 6;
     StepGraph graphs[kStepGraphs];
     int graph_next = 0;           // the entry replaced next
+    uint64_t graph_launches = 0;  // replays so far
     bool use_graphs = false;
     bool chain = false;       // RK stage kernels also form the next stage state (eval_combine)
 };

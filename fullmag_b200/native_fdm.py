@@ -122,7 +122,7 @@ EXT_FUNCTIONS = (
     "fullmag_fdm_backend_create_ext", "fullmag_fdm_backend_step_n",
     "fullmag_fdm_backend_set_profiling", "fullmag_fdm_backend_profile_count",
     "fullmag_fdm_backend_profile_entry", "fullmag_fdm_backend_profile_reset",
-    "fullmag_fdm_backend_memory_info", "fullmag_fdm_newell_spectra",
+    "fullmag_fdm_backend_memory_info", "fullmag_fdm_backend_graph_launches", "fullmag_fdm_newell_spectra",
     "fullmag_fdm_backend_get_stream", "fullmag_fdm_random_unit_vectors",
     "fullmag_fdm_adjoint_forward", "fullmag_fdm_adjoint_backward",
     "fullmag_fdm_batch_create", "fullmag_fdm_batch_step_n", "fullmag_fdm_batch_copy_m",
@@ -191,6 +191,7 @@ def load_library(build_if_missing: bool = True):
     L.fullmag_fdm_backend_profile_reset.argtypes = [vp]
     L.fullmag_fdm_backend_profile_reset.restype = None
     L.fullmag_fdm_backend_memory_info.argtypes = [vp, C.POINTER(C.c_uint64), C.POINTER(C.c_uint32)]
+    L.fullmag_fdm_backend_graph_launches.argtypes = [vp, C.POINTER(C.c_uint64)]
     L.fullmag_fdm_newell_spectra.argtypes = [C.c_uint32] * 3 + [C.c_double] * 3 + [C.c_int] + [_dp] * 6
     L.fullmag_fdm_backend_get_stream.argtypes = [vp, C.POINTER(C.c_void_p)]
     L.fullmag_fdm_random_unit_vectors.argtypes = [C.c_uint64, C.c_uint64, _dp]
@@ -558,6 +559,12 @@ class NativeFdmBackend:
         dims = (C.c_uint32 * 3)()
         self._lib.fullmag_fdm_backend_memory_info(self._h, C.byref(b), dims)
         return b.value, tuple(dims)
+
+    def graph_launches(self) -> int:
+        """Steps taken so far as the replay of a CUDA graph."""
+        c = C.c_uint64()
+        self._check(self._lib.fullmag_fdm_backend_graph_launches(self._h, C.byref(c)), "graph_launches")
+        return c.value
 
 
 class NativeFdmBatch:

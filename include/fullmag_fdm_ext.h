@@ -135,6 +135,10 @@ void fullmag_fdm_backend_profile_reset(fullmag_fdm_backend *handle);
 int fullmag_fdm_backend_memory_info(fullmag_fdm_backend *handle, uint64_t *out_device_bytes,
                                     uint32_t *out_fft_dims3);
 
+/* Step attempts the handle has made as the launch of a CUDA graph (the others issue their
+ * launches one by one). */
+int fullmag_fdm_backend_graph_launches(fullmag_fdm_backend *handle, uint64_t *out_launches);
+
 /* The CUDA stream the handle launches all its work on (a cudaStream_t), so
  * callers can order their own work or record CUDA events around steps. */
 int fullmag_fdm_backend_get_stream(fullmag_fdm_backend *handle, void **out_stream);

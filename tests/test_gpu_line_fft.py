@@ -14,8 +14,8 @@
 - A Runge-Kutta step on either side of the cell count up to which the FP32 group kernels
   form the next stage state themselves, FP32-mixed against FP64 at 1e-5 (the tolerance
   of the FP32-mixed trajectories).
-- Steps replayed as CUDA graphs against the same launches issued one by one (per-kernel
-  timing on), bit for bit, through dt changes.
+- Steps replayed as CUDA graphs (counted) against the same launches issued one by one
+  (per-kernel timing on), bit for bit, through dt changes; no replay where the rule has none.
 - A film's tensor with all six components (random octants) against numpy's FFT at the
   FP64 field tolerance.
 - Handles created where the device memory is short (the rest held by torch), against the
@@ -160,6 +160,18 @@ def test_step_graphs_equal_single_launches(cells, prec, integrator):
         b.step_n(1e-14, 6)
         for o in (nf.OBS_M, nf.OBS_H_DEMAG, nf.OBS_H_EFF):
             assert np.array_equal(a.copy_field(o), b.copy_field(o)), o
+        # 18 steps of two step sizes: of each, one issued as it is, one captured, the rest
+        # replays (the accepted states of the adaptive integrators alternate between two
+        # sets of buffers); ABM3 has graphs in its Heun start-up only
+        assert a.graph_launches() >= (1 if integrator == nf.ABM3 else 6) and b.graph_launches() == 0
+
+
+@pytest.mark.parametrize("kw", [dict(cells=(540, 512, 1)), dict(cells=(64, 16, 1), ac_field=(1e3, 0.0, 0.0), ac_frequency_hz=1e9)])
+def test_no_graphs_for_large_grids_and_time_dependent_fields(kw):
+    with nf.NativeFdmBackend(_plan(prec=nf.PRECISION_SINGLE, integrator=nf.HEUN, **kw)) as be:
+        for _ in range(6):
+            be.step(1e-14)
+        assert be.graph_launches() == 0
 
 
 @pytest.mark.parametrize("cells,integrator", [((525, 270, 4), nf.HEUN), ((525, 270, 4), nf.RK4),
