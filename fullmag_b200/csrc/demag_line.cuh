@@ -393,7 +393,6 @@ cudaError_t line_setup(LineCfg &c, int Lx, int Ly, bool thin, int ny, int nz, in
     c = LineCfg{};
     c.Lx = Lx;
     c.Ly = Ly;
-    c.thin = thin;
     cudaError_t err = cudaErrorInvalidValue;
     const bool okx = with_line(Lx, [&](auto l) {
         constexpr int L = decltype(l)::value, G = Lf<T, L>::G;

@@ -11,7 +11,6 @@ namespace fm {
 // Block shapes of the passes for one grid (line_setup).
 struct LineCfg {
     int Lx = 0, Ly = 0;
-    bool thin = false;
     bool pdl = true;                         // programmatic dependent launches (pdl.cuh)
     int lines_x = 0, te_x = 0, thr_x = 0;    // x passes: row pairs per block, line stride
     size_t smem_x = 0;

@@ -72,8 +72,6 @@ __device__ __forceinline__ float lf_mul(float a, float b) { return __fmul_rn(a, 
 __device__ __forceinline__ double lf_mul(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float lf_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double lf_fma(double a, double b, double c) { return __fma_rn(a, b, c); }
-__device__ __forceinline__ float lf_add1(float a, float b) { return __fadd_rn(a, b); }
-__device__ __forceinline__ double lf_add1(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ float2 lf_add(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 lf_sub(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
 __device__ __forceinline__ double2 lf_add(double2 a, double2 b) { return make_double2(__dadd_rn(a.x, b.x), __dadd_rn(a.y, b.y)); }

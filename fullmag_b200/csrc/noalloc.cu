@@ -20,6 +20,7 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <new>
 #include <type_traits>
 
 #include "demag_line.hpp"
@@ -68,13 +69,13 @@ void put_error(char *buf, uint64_t len, const char *msg) {
     }
 }
 
-// With the device current: resolve the array's device address (the host-side
-// symbol is only a stand-in) on every call, which is cheap, and once per
-// device (again if the address changed) fill this file's copy of the radix-64
-// twiddle table.  The upload goes through the legacy default stream from
+// With the device current: resolve the arrays' device addresses (the host-side
+// symbols are only stand-ins) on every call, which is cheap, and once per
+// device (again if an address changed) fill this file's copies of the radix-64
+// and line-FFT twiddle tables.  The upload goes through the legacy default stream from
 // pageable memory, which may return before the data reach the device, and a
 // caller's non-blocking stream is not ordered after it: the device is
-// synchronised once here, before the first kernel can read the table.
+// synchronised once here, before the first kernel can read the tables.
 bool setup_device(int dev, unsigned char **out, double2 **tw_out, char *err, uint64_t errlen) {
     std::lock_guard<std::mutex> lock(g_mu);
     DeviceSlot &s = g_slots[dev];
@@ -99,10 +100,14 @@ bool setup_device(int dev, unsigned char **out, double2 **tw_out, char *err, uin
         }
         e = cudaMemcpyToSymbol(c_tw64d, d, sizeof(d));
         if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_tw64f, f, sizeof(f));
-        for (int L : kTwLengths) {
-            const std::vector<double2> t = line_twiddles<double>(L);
-            if (e == cudaSuccess)
-                e = cudaMemcpyToSymbol(g_line_tw, t.data(), t.size() * sizeof(double2), (size_t)tw_offset(L) * sizeof(double2));
+        try {  // the tables are built in vectors; no exception leaves a C entry
+            for (int L : kTwLengths) {
+                const std::vector<double2> t = line_twiddles<double>(L);
+                if (e == cudaSuccess)
+                    e = cudaMemcpyToSymbol(g_line_tw, t.data(), t.size() * sizeof(double2), (size_t)tw_offset(L) * sizeof(double2));
+            }
+        } catch (const std::bad_alloc &) {
+            e = cudaErrorMemoryAllocation;
         }
         if (e == cudaSuccess) e = cudaDeviceSynchronize();
         if (e != cudaSuccess) {

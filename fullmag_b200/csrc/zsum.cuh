@@ -116,7 +116,7 @@ __device__ __forceinline__ void zsum_set(const C (&x)[N / 2 + 1], const C (&y)[N
             mid[0] = hx;
             mid[1] = hy;
         } else {
-            const C mz = mid[2], nmz = zs_neg(mid[2]);
+            const C nmz = zs_neg(mid[2]);
             C hz = zero;  // minus Hz, as z holds minus s_z
             zs_fma(hz, T(2) * tab(2, 0), nmz);
 #pragma unroll
@@ -128,7 +128,6 @@ __device__ __forceinline__ void zsum_set(const C (&x)[N / 2 + 1], const C (&y)[N
                 zs_fma(Z[j], czz, nmz);
             }
             mid[2] = zs_neg(hz);
-            (void)mz;
         }
     }
 }

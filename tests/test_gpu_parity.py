@@ -341,16 +341,15 @@ def test_runtime_errors_are_reported():
     assert lib.fullmag_fdm_backend_last_error(be.handle) == b"out_len mismatch"
 
 
-@pytest.mark.parametrize("fft", ["register", "fused", "stockham", "xpipe-off", "zfft"])
+@pytest.mark.parametrize("fft", ["register", "fused", "stockham", "zfft"])
 @pytest.mark.parametrize("cells,prec", [((64, 16, 1), nf.PRECISION_DOUBLE), ((32, 16, 8), nf.PRECISION_DOUBLE),
                                         ((32, 16, 8), nf.PRECISION_SINGLE), ((64, 32, 16), nf.PRECISION_SINGLE),
                                         ((256, 64, 1), nf.PRECISION_DOUBLE)])
 def test_both_fft_paths_match_oracle(monkeypatch, fft, cells, prec):
-    """The register-FFT kernels (power-of-two lengths; the y-z convolution as
-    three kernels, or fused per kx plane with FULLMAG_FDM_YZ=fused; the z
-    convolution summed directly for nz <= 8, or by z FFTs with
-    FULLMAG_FDM_ZCONV=fft) and the shared-memory Stockham kernels (any
-    2,3,5,7-smooth length; forced by FULLMAG_FDM_FFT)."""
+    """The line FFTs in x and y with the z convolution summed directly (nz <= 8,
+    FP32 nz <= 16) or, with FULLMAG_FDM_ZCONV=fft, by z FFTs; the y-z convolution
+    fused per kx plane with FULLMAG_FDM_YZ=fused; and the shared-memory Stockham
+    kernels at the lengths 2n (any 2,3,5,7-smooth length), forced by FULLMAG_FDM_FFT."""
     if fft == "stockham":
         monkeypatch.setenv("FULLMAG_FDM_FFT", "stockham")
     else:
@@ -359,12 +358,6 @@ def test_both_fft_paths_match_oracle(monkeypatch, fft, cells, prec):
         monkeypatch.setenv("FULLMAG_FDM_YZ", "fused")
     else:
         monkeypatch.delenv("FULLMAG_FDM_YZ", raising=False)
-    # the pipelined x forward serves uniform materials; "xpipe-off" keeps the
-    # one-group-per-block kernel
-    if fft == "xpipe-off":
-        monkeypatch.setenv("FULLMAG_FDM_XPIPE", "off")
-    else:
-        monkeypatch.delenv("FULLMAG_FDM_XPIPE", raising=False)
     if fft == "zfft":
         monkeypatch.setenv("FULLMAG_FDM_ZCONV", "fft")
     else:
@@ -377,7 +370,7 @@ def test_both_fft_paths_match_oracle(monkeypatch, fft, cells, prec):
     be.set_profiling(False)
     if cells[2] > 1:
         # direct z sum: nz <= 8, and in FP32 nz <= 16
-        direct = fft in ("register", "xpipe-off") and cells[2] <= (16 if prec == nf.PRECISION_SINGLE else 8)
+        direct = fft == "register" and cells[2] <= (16 if prec == nf.PRECISION_SINGLE else 8)
         assert ("demag_z_direct" in names) == direct, (fft, names)
     err = _field_errors(be, sim.observe())
     tol = 1e-13 if prec == nf.PRECISION_DOUBLE else 2e-6
@@ -396,7 +389,7 @@ def test_both_fft_paths_match_oracle(monkeypatch, fft, cells, prec):
                                         ((16, 32, 6), nf.PRECISION_DOUBLE), ((16, 8, 7), nf.PRECISION_SINGLE),
                                         ((64, 32, 7), nf.PRECISION_DOUBLE)])
 def test_direct_z_convolution_any_nz_matches_oracle(monkeypatch, cells, prec):
-    for k in ("FULLMAG_FDM_FFT", "FULLMAG_FDM_YZ", "FULLMAG_FDM_ZCONV", "FULLMAG_FDM_XPIPE"):
+    for k in ("FULLMAG_FDM_FFT", "FULLMAG_FDM_YZ", "FULLMAG_FDM_ZCONV"):
         monkeypatch.delenv(k, raising=False)
     nx, ny, nz = cells
     kw = {}

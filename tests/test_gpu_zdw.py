@@ -1,5 +1,5 @@
-"""The FP32 direct z convolution for 8 < nz <= 16 (k_zdw: each column's outputs
-split in two halves over two warps, the column's inputs and table entries
+"""The FP32 direct z convolution for 8 < nz <= 16 (k_zdw: the even and odd
+halves of each column's sum on two warps, the column's inputs and table entries
 staged in shared memory by cp.async).
 
 - Fields and 5 Heun steps against the FP64 oracle at nz = 9, 12, 14, 15, 16, at
@@ -12,9 +12,7 @@ staged in shared memory by cp.async).
 - The window form equals the element form bitwise (FULLMAG_FDM_ZDW=elem): the
   same table values in the same sums.
 - At nz = 8, forced on with FULLMAG_FDM_ZDW=on (fused plane pass off), against
-  k_zd: the same table and packed FMAs, so the lower half's z planes of H_d
-  are bitwise k_zd's; the upper half, summed in the z-reversed frame, adds each
-  +d / -d pair in the other order and agrees to FP32 rounding (1e-6 of max|H_d|).
+  k_zd: the same sums in the same order, so H_d and the state are bitwise k_zd's.
 - At nz = 16 it agrees with the z FFT pass (FULLMAG_FDM_ZCONV=fft).
 """
 import numpy as np
@@ -26,8 +24,7 @@ from gpu_helpers import make_pair, max_abs
 
 pytestmark = pytest.mark.gpu
 
-_ENV = ("FULLMAG_FDM_FFT", "FULLMAG_FDM_YZ", "FULLMAG_FDM_ZCONV", "FULLMAG_FDM_XPIPE", "FULLMAG_FDM_YZY",
-        "FULLMAG_FDM_ZDW")
+_ENV = ("FULLMAG_FDM_FFT", "FULLMAG_FDM_YZ", "FULLMAG_FDM_ZCONV", "FULLMAG_FDM_YZY", "FULLMAG_FDM_ZDW")
 
 
 def _field_errors(be, obs):
@@ -86,17 +83,11 @@ def test_wide_direct_z_against_k_zd_at_nz8(monkeypatch):
     wide, _, _ = make_pair(**kw)
     assert "demag_z_direct" in _kernels(wide)
     ref.refresh_observables()
-    nx, ny, nz = cells
-    a = wide.copy_field(nf.OBS_H_DEMAG).reshape(nz, ny, nx, 3)
-    b = ref.copy_field(nf.OBS_H_DEMAG).reshape(nz, ny, nx, 3)
-    assert np.array_equal(a[: nz // 2], b[: nz // 2])
-    rel = max_abs(a, b) / np.abs(b).max()
-    print(f"nz = 8, k_zdw vs k_zd: {rel:.2e} of max|H_d|")
-    assert rel <= 1e-6
+    assert np.array_equal(wide.copy_field(nf.OBS_H_DEMAG), ref.copy_field(nf.OBS_H_DEMAG))
     for _ in range(3):
         wide.step(2e-14)
         ref.step(2e-14)
-    assert max_abs(wide.copy_m(), ref.copy_m()) <= 1e-6
+    assert np.array_equal(wide.copy_m(), ref.copy_m())
     wide.close()
     ref.close()
 
