@@ -362,10 +362,11 @@ struct Impl {
         b.stage_vec = rows16 && simple && !keep && 3ULL * (unsigned long long)b.n < (1ULL << 32);
         b.stage_vec_mk = b.stage_vec && (b.has_mask || b.has_ms_map);
         // RK stage kernels that also form the next stage state: always with the one-value
-        // kernels (512 x 512 x 8 FP64 RK4 1566 -> 1505 us per step, 256 x 256 x 4 217 -> 208);
-        // with the group kernels, whose registers then allow 16 warps per SM instead of 20,
-        // up to 2^18 cells (128 x 128 FP32 DP45 133 -> 124 us, 256 x 256 x 4 252 -> 249, but
-        // 300 x 180 x 5 masked 479 -> 486 and 1024 x 512 x 16 masked 242 -> 290 us per stage)
+        // kernels (us per step without and with: 512 x 512 x 8 FP64 RK4 1516 / 1455, 512 x 512
+        // 186 / 179, 240 x 150 x 6 masked DP45 451 / 454); with the group kernels, whose
+        // registers then allow 16 warps per SM instead of 20, up to 2^18 cells (128 x 128 FP32
+        // DP45 113 / 107, 512 x 512 191 / 184, 256 x 256 x 4 RK4 119 / 115, but 300 x 180 x 5
+        // masked DP45 334 / 356, 540 x 512 239 / 256, 512 x 512 x 4 RK4 346 / 362)
         b.chain = !b.lean && (!b.stage_vec || b.n <= (1LL << 18));
         if (!b.stage_plain) return true;
         b.stage_ring = !env_is("FULLMAG_FDM_STAGE", "plain");
@@ -390,7 +391,10 @@ struct Impl {
             if (!configure_line(b) || !row_configure<T>(b)) return false;
             // a time-dependent field enters the kernels' arguments: no graphs then.  Up to
             // 2^18 cells a step's kernels take 3 to 8 us each, a launch 1.6 to 3 us of the host
-            // and 8 of them with their synchronisation 20 us; one graph of 8 takes 10.
+            // and 8 of them with their synchronisation 20 us; one graph of 8 takes 10.  Above,
+            // the launches are hidden (us per step without and with graphs: Heun 540 x 512 FP32
+            // 67.1 / 68.2, 512 x 256 x 4 FP64 173.5 / 175.8, 512 x 512 x 4 FP32 162 / 165; 300 x
+            // 180 x 5 masked DP45, with a read-back per step, 333 / 324)
             b.use_graphs = !b.use_row && b.n <= (1LL << 18) && b.ac_freq == 0.0;
             return true;
         }

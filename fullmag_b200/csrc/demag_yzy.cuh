@@ -28,9 +28,11 @@
 // Measured at 512 x 512 x 8 (FP32, P = 2): 106 us with 3-pass lines of 64 threads and
 // named barriers, 100 us with the two-pass lines of one warp each (P = 1 with 384
 // threads 114 us); a half plane's CTA then took 12.4 kcycles for the forward lines, 16.8
-// for the z sum and 8 for the inverse, the z sum bound by its 576 packed multiply-adds
-// per column (2.05 cycles each per scheduler, the FP32 peak).  With the 288 of the sum
-// over even and odd halves: 89 us.
+// for the z sum and 8 for the inverse.  With the z sum over even and odd halves: 88 us
+// (P = 1 90.5, P = 4 120, P = 8 128; the split kernels 31 + 54 + 31).  What bounds it now:
+// 12 warps per SM (162 registers, 107 KB per CTA) in chains of shared and cluster memory
+// and dependent arithmetic: issue 41 % active, FMA pipe 28 %, LSU 22 %, DRAM 15 %; its
+// bytes would take 24 us, its multiply-adds of the z sum 8.
 // Two units per precision (demag_yzy_f32.cu, demag_yzy_f32b.cu, ..: nz <= 4 and
 // above), so that they compile in parallel.
 #pragma once
@@ -261,8 +263,10 @@ static bool yzy_configure_t(Backend &b) {
     // cluster size: FULLMAG_FDM_YZY_P, else the smallest P whose CTA fits twice per SM
     int want = 0;
     if (const char *p = std::getenv("FULLMAG_FDM_YZY_P")) want = std::atoi(p);
-    // FP64 only on request: at 512 x 512 x 8 its 8-CTA clusters ran 320 us against
-    // 244 us for the three split kernels
+    // FP64 only on request: at 512 x 512 x 8 it takes 329, 415 and 387 us with P = 2, 4 and
+    // 8 (P = 1 does not fit) against 216 us for the three split kernels, at 256 x 256 x 8
+    // 88 us with P = 1 against 65; only 4 planes and fewer, where one CTA holds the plane,
+    // are faster fused (512 x 512 x 4: 88 against 111 us)
     if (sizeof(T) == 8 && !want) return true;
     yzy_dispatch(b.Ly, b.nz, [&](auto l, auto nzc) {
         constexpr int L = decltype(l)::value, NZ = decltype(nzc)::value;

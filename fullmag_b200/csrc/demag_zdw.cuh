@@ -12,6 +12,10 @@
 //     buffered: the next batch's copies run while this batch is summed, and
 //     both sets read one copy; the sums are exchanged in the input slots.
 // The sums and their order are k_zd's, so the outputs are bitwise its own.
+// What bounds it (1024 x 512 x 16, 250 us, 3.9 TB/s): 8 warps per SM (204 registers, 99 KiB
+// per block) whose largest stall is the fetch of the two sets' unrolled code, then
+// dependent arithmetic; issue 39 % active, FMA pipe 26 %, DRAM 46 %.  Its bytes would take
+// 155 us, its multiply-adds 67.
 // Shared memory: 2 buffers x 64 columns x (3 nz complex + 6 nz reals),
 // 96 KiB at nz = 16 (99 KiB in the window form below): two blocks per SM.
 // No TMA; plain cp.async copies.

@@ -16,10 +16,10 @@
 // line_slot(k)) and the inverse starts from there, which saves the reordering
 // round trip wherever the product with the tensor is taken in shared memory.
 //
-// 8 to 24 values per thread (32 at most) instead of 32 to 64: the transforms are bound by
-// latency (shared-memory and FP chains), not by issue slots or bandwidth, so
-// what counts is the number of warps an SM can hold; at 1024 points a thread
-// needs about 64 registers where the two-pass 32 x 32 form needed 100 to 168.
+// 4 to 16 values per thread (24 at 1536 points, 32 at FP32's 1024) instead of 32 to
+// 64: the transforms are bound by latency (shared-memory and FP chains), not by issue
+// slots or bandwidth, so what counts is the number of warps an SM can hold; at 2048 FP32
+// points a thread needs 61 to 64 registers where the two-pass 64 x 32 form needed 168 to 242.
 //
 // Zero padding: HALF inputs n >= L/2 are zero and HALF outputs n >= L/2 are not
 // wanted; both fold away at compile time (R0 is even).
