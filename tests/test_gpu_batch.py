@@ -3,7 +3,7 @@ uneven grids and materials, stepped together with one persistent launch per
 stage and one CUDA graph per step, against the FP64 oracle run alone on that
 problem.  Tolerances as for single problems: FP64 max|dm| <= 1e-10 after 10
 Heun steps (inside the predictability horizon of random m0), FP32-mixed 1e-5.
-The batch pads each in-plane axis to the smallest power of two or (FP32) 3 * 2^k
+The batch pads each in-plane axis to the smallest power of two or 3 * 2^k
 (96, 192, 384, 768) >= 2n and z to a power of two, the oracle to 2n: the fields
 agree in exact arithmetic (kernel offsets |r| <= n - 1 only).  The shapes cover
 padded lengths 16, 32, 64, 96, 128, 192, 256 and 384.  The z convolution runs
